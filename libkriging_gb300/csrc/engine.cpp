@@ -551,8 +551,7 @@ void Engine::evaluate(int batch, const double* thetas, const double* factors, bo
                             std::to_string(mixed && mw.side_stream ? mw.side_ctas : 0) + ":t=" +
                             std::to_string(oz7_tile()) + ":g=" + std::to_string(buf_gen_);
     run_phase(key, [&] {
-      cov_build_lower(kernel_, n, d, dXb, xbs, dtheta_, dfactor_, ddiag_, dA_, lda_, mstride_, batch, st_, mixed,
-                      dnv);
+      cov_build_lower(kernel_, n, d, dXb, xbs, dtheta_, dfactor_, ddiag_, dA_, lda_, mstride_, batch, st_, dnv);
       if (mixed)
         potrf_blocked_mixed(dA_, lda_, mstride_, n, dDinv_, dinfo_, batch, mw, st_);
       else
@@ -869,7 +868,7 @@ void Engine::evaluate_update(const Engine& old, const double* theta, double fact
   LKG_CUDA(cudaMemcpyAsync(ddiag_, &one, sizeof(double), cudaMemcpyHostToDevice, st_));
   // R (lower) of the whole design; its leading block is then replaced by the old factor (update_cholCov restores
   // R_old there and chol_block keeps L_oo)
-  cov_build_lower(kernel_, n, d, dX_, 0, dtheta_, dfactor_, ddiag_, dA_, lda_, mstride_, 1, st_, false, nullptr);
+  cov_build_lower(kernel_, n, d, dX_, 0, dtheta_, dfactor_, ddiag_, dA_, lda_, mstride_, 1, st_, nullptr);
   LKG_CUDA(cudaStreamSynchronize(old.stream()));
   LKG_CUDA(cudaMemcpy2DAsync(dA_, sizeof(double) * lda_, old.dL(0), sizeof(double) * old.lda(), sizeof(double) * no,
                              no, cudaMemcpyDeviceToDevice, st_));
@@ -997,7 +996,7 @@ void Engine::model_matrices(const double* theta, double factor, std::vector<doub
     LKG_CUDA(cudaMemcpyAsync(dtheta_, theta, sizeof(double) * d_, cudaMemcpyHostToDevice, st_));
     LKG_CUDA(cudaMemcpyAsync(dfactor_, &factor, sizeof(double), cudaMemcpyHostToDevice, st_));
     LKG_CUDA(cudaMemcpyAsync(ddiag_, &one, sizeof(double), cudaMemcpyHostToDevice, st_));
-    cov_build_lower(kernel_, n, d_, dX_, 0, dtheta_, dfactor_, ddiag_, dW_, lda_, mstride_, 1, st_, false, nullptr);
+    cov_build_lower(kernel_, n, d_, dX_, 0, dtheta_, dfactor_, ddiag_, dW_, lda_, mstride_, 1, st_, nullptr);
     R->assign((size_t)n * n, 0.0);
     LKG_CUDA(cudaMemcpy2DAsync(R->data(), sizeof(double) * n, dW_, sizeof(double) * lda_, sizeof(double) * n, n,
                                cudaMemcpyDeviceToHost, st_));

@@ -38,7 +38,7 @@ __device__ __forceinline__ double block_sum(double v, double* red) {
   return s;
 }
 
-template <int K, int DM, bool FAST>
+template <int K, int DM>
 __global__ void __launch_bounds__(256) k_cov_lower(int n, int d, const double* __restrict__ X, int64_t xb,
                                                    const double* __restrict__ theta, const double* __restrict__ factor,
                                                    const double* __restrict__ diag, double* __restrict__ A,
@@ -65,7 +65,7 @@ __global__ void __launch_bounds__(256) k_cov_lower(int n, int d, const double* _
 #pragma unroll
   for (int k = 0; k < DM; ++k) {
     xr[k] = xi[k][ri];
-    ck[k] = FAST ? cov_scale<K>() / th[k] : 0.0;
+    ck[k] = cov_scale<K>() / fabs(th[k]);
   }
   for (int s = 0; s < 16; ++s) {
     const int cj = (t >> 6) + 4 * s, j = c0 + cj;
@@ -75,18 +75,12 @@ __global__ void __launch_bounds__(256) k_cov_lower(int n, int d, const double* _
       v = (j == i) ? 1.0 : 0.0;
     } else if (j == i) {
       v = dv;
-    } else if (FAST) {
+    } else {
       double sum = 0.0, prod = 1.0;
 #pragma unroll
       for (int k = 0; k < DM; ++k)
         if (k < d) cov_fast_term<K>(xj[k][cj] - xr[k], ck[k], sum, prod);
       v = cov_fast_finish<K>(sum, prod) * f;
-    } else {
-      double sum = 0.0;
-#pragma unroll
-      for (int k = 0; k < DM; ++k)
-        if (k < d) sum += cov_term<K>(xj[k][cj] - xr[k], th[k]);
-      v = cov_from_sum<K>(sum) * f;
     }
     Ab[i + (int64_t)j * lda] = v;
   }
@@ -96,31 +90,31 @@ template <int K, int DM>
 __global__ void __launch_bounds__(256) k_cov_cross(int n_o, int q, int d, const double* __restrict__ Xo,
                                                    const double* __restrict__ Xn, const double* __restrict__ theta,
                                                    double factor, double* __restrict__ R, bool snap) {
-  __shared__ double xo[DM][T], xn[DM][T], th[DM];
+  __shared__ double xo[DM][T], xn[DM][T], cks[DM];
   const int r0 = blockIdx.x * T, c0 = blockIdx.y * T, t = threadIdx.x;
   for (int idx = t; idx < DM * T; idx += 256) {
     const int k = idx / T, qq = idx % T;
     xo[k][qq] = (k < d && r0 + qq < n_o) ? Xo[(r0 + qq) + (int64_t)k * n_o] : 0.0;
     xn[k][qq] = (k < d && c0 + qq < q) ? Xn[(c0 + qq) + (int64_t)k * q] : 0.0;
   }
-  if (t < DM) th[t] = (t < d) ? theta[t] : 1.0;
+  if (t < DM) cks[t] = (t < d) ? cov_scale<K>() / fabs(theta[t]) : 1.0;
   __syncthreads();
   const int ri = t & 63, i = r0 + ri;
   if (i >= n_o) return;
   for (int s = 0; s < 16; ++s) {
     const int cj = (t >> 6) + 4 * s, j = c0 + cj;
     if (j >= q) continue;
-    double sum = 0.0;
+    double sum = 0.0, prod = 1.0;
     bool coincident = true;
 #pragma unroll
     for (int k = 0; k < DM; ++k) {
       if (k < d) {
         const double dx = xo[k][ri] - xn[k][cj];
         coincident = coincident && (fabs(dx) <= 2.220446049250313e-16);
-        sum += cov_term<K>(dx, th[k]);
+        cov_fast_term<K>(dx, cks[k], sum, prod);
       }
     }
-    R[i + (int64_t)j * n_o] = (snap && coincident) ? 1.0 : cov_from_sum<K>(sum) * factor;
+    R[i + (int64_t)j * n_o] = (snap && coincident) ? 1.0 : cov_fast_finish<K>(sum, prod) * factor;
   }
 }
 
@@ -150,31 +144,34 @@ template <int K, int DM>
 __global__ void __launch_bounds__(256) k_dcov_cross(int n_o, int q, int d, const double* __restrict__ Xo,
                                                     const double* __restrict__ Xn, const double* __restrict__ theta,
                                                     double factor, double* __restrict__ DR) {
-  __shared__ double xo[DM][T], xn[DM][T], th[DM];
+  __shared__ double xo[DM][T], xn[DM][T], th[DM], cks[DM];
   const int r0 = blockIdx.x * T, c0 = blockIdx.y * T, t = threadIdx.x;
   for (int idx = t; idx < DM * T; idx += 256) {
     const int k = idx / T, qq = idx % T;
     xo[k][qq] = (k < d && r0 + qq < n_o) ? Xo[(r0 + qq) + (int64_t)k * n_o] : 0.0;
     xn[k][qq] = (k < d && c0 + qq < q) ? Xn[(c0 + qq) + (int64_t)k * q] : 0.0;
   }
-  if (t < DM) th[t] = (t < d) ? theta[t] : 1.0;
+  if (t < DM) {
+    th[t] = (t < d) ? theta[t] : 1.0;
+    cks[t] = cov_scale<K>() / fabs(th[t]);
+  }
   __syncthreads();
   const int ri = t & 63, i = r0 + ri;
   if (i >= n_o) return;
   for (int s = 0; s < 16; ++s) {
     const int cj = (t >> 6) + 4 * s, j = c0 + cj;
     if (j >= q) continue;
-    double sum = 0.0;
+    double sum = 0.0, prod = 1.0;
     bool coincident = true;
 #pragma unroll
     for (int k = 0; k < DM; ++k) {
       if (k < d) {
         const double dx = xo[k][ri] - xn[k][cj];
         coincident = coincident && (fabs(dx) <= 2.220446049250313e-16);
-        sum += cov_term<K>(dx, th[k]);
+        cov_fast_term<K>(dx, cks[k], sum, prod);
       }
     }
-    const double r = coincident ? 1.0 : cov_from_sum<K>(sum) * factor;
+    const double r = coincident ? 1.0 : cov_fast_finish<K>(sum, prod) * factor;
     double* out = DR + i + (int64_t)j * d * n_o;
 #pragma unroll
     for (int k = 0; k < DM; ++k)
@@ -470,32 +467,33 @@ template <int K, int DM>
 __global__ void __launch_bounds__(256) k_loo_gradR(int n, int d, const double* __restrict__ X,
                                                    const double* __restrict__ theta, double factor, int kdim,
                                                    double* __restrict__ G, int64_t ldg) {
-  __shared__ double xi[DM][T], xj[DM][T], th[DM];
+  __shared__ double xi[DM][T], xj[DM][T], cks[DM];
   const int r0 = blockIdx.x * T, c0 = blockIdx.y * T, t = threadIdx.x;
   for (int idx = t; idx < DM * T; idx += 256) {
     const int k = idx / T, q = idx % T;
     xi[k][q] = (k < d && r0 + q < n) ? X[(r0 + q) + (int64_t)k * n] : 0.0;
     xj[k][q] = (k < d && c0 + q < n) ? X[(c0 + q) + (int64_t)k * n] : 0.0;
   }
-  if (t < DM) th[t] = (t < d) ? theta[t] : 1.0;
+  if (t < DM) cks[t] = (t < d) ? cov_scale<K>() / fabs(theta[t]) : 1.0;
   __syncthreads();
   const int ri = t & 63, i = r0 + ri;
   if (i >= n) return;
+  const double inv = 1.0 / theta[kdim];
   for (int s = 0; s < 16; ++s) {
     const int cj = (t >> 6) + 4 * s, j = c0 + cj;
     if (j >= n) continue;
     double v = 0.0;
     if (j != i) {
-      double sum = 0.0, dk = 0.0;
+      double sum = 0.0, prod = 1.0, dk = 0.0;
 #pragma unroll
       for (int k = 0; k < DM; ++k) {
         if (k < d) {
           const double dx = xj[k][cj] - xi[k][ri];
-          sum += cov_term<K>(dx, th[k]);
-          if (k == kdim) dk = dlncov_term<K>(dx, th[k]);
+          cov_fast_term<K>(dx, cks[k], sum, prod);
+          if (k == kdim) dk = dlncov_fast<K>(dx, inv, cks[k]);
         }
       }
-      v = (cov_from_sum<K>(sum) * factor) * dk;
+      v = (cov_fast_finish<K>(sum, prod) * factor) * dk;
     }
     G[i + (int64_t)j * ldg] = v;
   }
@@ -562,17 +560,12 @@ struct LooGradRLaunch {
 template <int K, int DM>
 struct CovLowerLaunch {
   static void run(int n, int d, const double* X, int64_t xb, const double* theta, const double* factor,
-                  const double* diag, double* A, int64_t lda, int64_t mstride, int batch, bool fast, const int* nvalid,
-                  cudaStream_t st) {
+                  const double* diag, double* A, int64_t lda, int64_t mstride, int batch, const int* nvalid, cudaStream_t st) {
     const int nb = ceil_div(n, T);
     const int64_t ntiles = (int64_t)nb * (nb + 1) / 2;
     LaunchTimer lt("k_cov_lower", st, 0.5 * n * (n - 1.0) * batch, 4.0 * n * (n + 1.0) * batch);
-    if (fast)
-      k_cov_lower<K, DM, true><<<dim3((unsigned)ntiles, 1, batch), 256, 0, st>>>(n, d, X, xb, theta, factor, diag, A,
-                                                                                  lda, mstride, nvalid);
-    else
-      k_cov_lower<K, DM, false><<<dim3((unsigned)ntiles, 1, batch), 256, 0, st>>>(n, d, X, xb, theta, factor, diag,
-                                                                                   A, lda, mstride, nvalid);
+    k_cov_lower<K, DM><<<dim3((unsigned)ntiles, 1, batch), 256, 0, st>>>(n, d, X, xb, theta, factor, diag, A, lda,
+                                                                         mstride, nvalid);
     LKG_LAUNCH("k_cov_lower");
   }
 };
@@ -615,10 +608,9 @@ struct AdjointLaunch {
 
 void cov_build_lower(int kernel, int n, int d, const double* X, int64_t x_bstride, const double* theta,
                      const double* factor, const double* diag, double* A, int64_t lda, int64_t mstride, int batch,
-                     cudaStream_t st, bool fast, const int* nvalid) {
+                     cudaStream_t st, const int* nvalid) {
   if (n <= 0) return;
-  dispatch_kd<CovLowerLaunch>(kernel, d, n, d, X, x_bstride, theta, factor, diag, A, lda, mstride, batch, fast, nvalid,
-                              st);
+  dispatch_kd<CovLowerLaunch>(kernel, d, n, d, X, x_bstride, theta, factor, diag, A, lda, mstride, batch, nvalid, st);
 }
 
 void cov_cross(int kernel, int n_o, int q, int d, const double* Xo, const double* Xn, const double* theta,
