@@ -17,11 +17,12 @@
 // with one bulk copy; a 64-row tile is the first or second half of an image.
 //
 // k_oz7_gemm (one persistent CTA per SM, 18 warps):
-//   warp 0        one thread streams the digit images: per sub-chunk all S digits of B (64 rows, double-buffered),
-//                 then the S digits of A (128 rows) through a 6-7-stage ring; bulk copies complete on mbarriers
-//   warp 1        TMEM allocation (512 columns = S diagonals x 64 columns); one thread issues tcgen05.mma
-//                 (M 128, N 64 k, K 16): A digit i against up to 4 adjacent B digits at once, and releases each A
-//                 stage and B buffer with tcgen05.commit
+//   warp 0        one thread streams the digit images: per sub-chunk all S digits of B (TN rows, double-buffered),
+//                 then the S digits of A (128 rows) in groups of group_size<S, TN>() images, one ring stage and one
+//                 bulk copy each; copies complete on mbarriers
+//   warp 1        TMEM allocation (512 columns); one thread issues tcgen05.mma (M 128, N TN k, K 16): A digit i
+//                 against up to 256 / TN adjacent B digits at once, and releases each A stage and B buffer with
+//                 tcgen05.commit
 //   warps 2..17   epilogue: warp w reads TMEM lanes 32 (w % 4) .. +31 (rows) and 8 columns, 4 at a time:
 //                 folds the S diagonals exactly (int32 pairs, two exact doubles, one rounded FP64 addition) and
 //                 updates C, then releases its accumulator set to the next block (18 warps leave 96 registers a
@@ -39,8 +40,8 @@ void set_last_error(const char* msg);
 namespace {
 
 constexpr int TM = 128;
-constexpr int NA_MAX = 10;                     // A ring stages at most
-constexpr uint32_t A_BYTES = TM * 128;         // one digit of a 128-row tile, one 64-wide sub-chunk: 16 KB
+constexpr int NA_MAX = 6;                      // A ring stages at most
+constexpr uint32_t IMG_BYTES = TM * 128;       // one digit of a 128-row tile, one 64-wide sub-chunk: 16 KB
 constexpr uint64_t kWaitNs = 200000000ull;     // an mbarrier wait gives up after 200 ms
 
 // Output tiles are 128 x TN.  TN = 32: two accumulator sets of S x 32 TMEM columns, so the fold of one tile overlaps
@@ -51,12 +52,26 @@ constexpr uint32_t b_bytes() { return TN * 128; }  // one digit of a TN-row B ti
 template <int S, int TN>
 constexpr int nsets() { return 2 * S * TN <= 512 ? 2 : 1; }
 
-// A ring depth: what 227 KB of shared memory holds beside the two B buffers (10 for TN = 32, 6 for TN = 64 at
-// S = 8); a deep ring keeps enough digit images in flight to cover the L2 latency at the rate the MMAs consume them
+// A digits of one ring stage (one barrier, one copy).  The issuing thread's wait on a barrier costs about as much as
+// the products of one digit (4 MMAs of 16 x 128 x N, 70 - 130 clocks each), so a barrier for every digit left the
+// tensor pipe half idle even with no copies and no fold running (1306 TFLOP/s at S = 8).  Measured on a 12288 x 256
+// lower product, S = 8 (TFLOP/s): 1 digit per barrier and 10 stages 1180, 2 and 5 1271, 3 and 3 1433, 4 and 2 1468;
+// S = 5 on 8192 x 8192 x 256: 1 digit 770, 2 883, 3 930, 5 966.  Two stages are enough to cover the L2 latency.  What
+// bounds it now: 1640 (S = 8) and 1138 (S = 5) without the fold; an MMA takes max(N / 2, 68) clocks, so the narrow
+// ones of the last digits run below the pipe's rate (1870 and 1610 at best).
+template <int S, int TN>
+constexpr int group_size() {
+  if (TN == 64) return 2;
+  return S == 8 || S == 7 ? 4 : S == 6 ? 3 : S;
+}
+template <int S, int TN>
+constexpr int n_groups() { return (S + group_size<S, TN>() - 1) / group_size<S, TN>(); }
+
+// A ring depth: what 227 KB of shared memory holds beside the two B buffers
 template <int S, int TN>
 constexpr int ring_depth() {
-  return (int)((227u * 1024u - 1024u - 2u * S * b_bytes<TN>()) / A_BYTES) < NA_MAX
-             ? (int)((227u * 1024u - 1024u - 2u * S * b_bytes<TN>()) / A_BYTES)
+  return (int)((227u * 1024u - 1024u - 2u * S * b_bytes<TN>()) / (group_size<S, TN>() * IMG_BYTES)) < NA_MAX
+             ? (int)((227u * 1024u - 1024u - 2u * S * b_bytes<TN>()) / (group_size<S, TN>() * IMG_BYTES))
              : NA_MAX;
 }
 constexpr int NTHREADS = 576;                  // 18 warps
@@ -177,8 +192,8 @@ __device__ __forceinline__ double fold_diagonals(const uint32_t (&v)[S][4], int 
     hi = ((long long)iv[0] << 14) + (iv[1] * 128 + iv[2]);
   else if constexpr (S == 6)
     hi = iv[0] * 128 + iv[1];
-  else
-    hi = iv[0];
+  else  // S = 5: |H| < 2^49 is one exact double, no rounding addition
+    return exact_scaled(((long long)iv[0] << 28) + lo, E);
   return exact_scaled(hi, E + 28) + exact_scaled(lo, E);
 }
 
@@ -189,6 +204,8 @@ __device__ __forceinline__ uint32_t bf16_bits_of_small(int d) {
   const float f = __int_as_float(0x4B400000 + d) - 12582912.0f;
   return (uint32_t)__float_as_int(f) >> 16;
 }
+
+constexpr int kNanExp = 1 << 24;  // exponent of a block that holds an infinity or NaN
 
 // one operand of a split launch: element (r, k) of batch entry b at p[b * bstride + r * s_r + k * s_k]
 struct SplitJob {
@@ -240,7 +257,8 @@ __global__ void __launch_bounds__(256) k_oz7_split(SplitJob j0, SplitJob j1, int
   int e = 0;
   if (bm != 0) {
     const int bx = (int)(bm >> 52);
-    const int E = bx ? bx - 1022 : (64 - __clzll((long long)(bm & 0xFFFFFFFFFFFFFull))) - 1074;
+    // a block with an infinity or NaN: no digits, and an exponent that turns every product of the block into NaN
+    const int E = bx == 2047 ? kNanExp - 1 : bx ? bx - 1022 : (64 - __clzll((long long)(bm & 0xFFFFFFFFFFFFFull))) - 1074;
     e = E + 1;
   }
   const int ntile = out.rows_pad / 128, t = r >> 7, rr = r & 127;
@@ -275,14 +293,14 @@ __global__ void __launch_bounds__(256) k_oz7_split(SplitJob j0, SplitJob j1, int
     // significant first) is ((U >> 7 k) & 127) - 64 for k < S - 1 and the top digit is U >> 7 (S - 1) (|d| <= 64)
     constexpr long long C = 64ll * ((1ll << (7 * (S - 1))) - 1) / 127;
     const long long U0 = V[0] + C, U1 = V[1] + C;
-    const int64_t plane = (int64_t)out.nsub * ntile * (TM * 64);  // elements between digit images
-    uint32_t* img = reinterpret_cast<uint32_t*>(base + ((int64_t)s * ntile + t) * (TM * 64) + off);
+    // the S digit images of one (sub-chunk, tile) are adjacent, so a group of A digits is one bulk copy
+    uint32_t* img = reinterpret_cast<uint32_t*>(base + ((int64_t)s * ntile + t) * S * (TM * 64) + off);
 #pragma unroll
     for (int k = 0; k < S; ++k) {
       const int i = S - 1 - k;  // digit index, 0 = most significant
       const int d0 = (k < S - 1) ? (int)((U0 >> (7 * k)) & 127) - 64 : (int)(U0 >> (7 * k));
       const int d1 = (k < S - 1) ? (int)((U1 >> (7 * k)) & 127) - 64 : (int)(U1 >> (7 * k));
-      img[(i * plane) >> 1] = bf16_bits_of_small(d0) | (bf16_bits_of_small(d1) << 16);
+      img[i * (TM * 64 / 2)] = bf16_bits_of_small(d0) | (bf16_bits_of_small(d1) << 16);
     }
   }
   if (lane == 0) out.exps[b * out.exp_bstride + (int64_t)kb * out.rows_pad + r] = e;
@@ -330,6 +348,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_oz7_gemm(Oz7Args g, long long n
   static_assert(TN == 32 || TN == 64, "tile width");
   constexpr int NA = ring_depth<S, TN>();
   static_assert(NA >= 2 && NA <= NA_MAX, "A ring depth");
+  constexpr int GA = group_size<S, TN>(), NG = n_groups<S, TN>();
+  constexpr uint32_t A_BYTES = GA * IMG_BYTES;
   constexpr uint32_t B_BYTES = b_bytes<TN>();
   constexpr uint32_t B_BUF = S * B_BYTES;
   constexpr int NSET = nsets<S, TN>();
@@ -338,7 +358,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_oz7_gemm(Oz7Args g, long long n
   __shared__ Bars bars;
   __shared__ uint32_t tslot;
   const uint32_t raw = su32(oz7_raw);
-  const uint32_t sA = (raw + 1023u) & ~1023u;  // NA stages of one A digit
+  const uint32_t sA = (raw + 1023u) & ~1023u;  // NA stages of GA A digits
   const uint32_t sB = sA + NA * A_BYTES;        // 2 buffers of S B digits
   const int t = threadIdx.x, w = t >> 5, lane = t & 31;
   const int64_t bz = blockIdx.z;
@@ -396,27 +416,29 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_oz7_gemm(Oz7Args g, long long n
               ok = false;
               break;
             }
+            // B goes out before the wait for an A stage: its buffer is free a sub-chunk earlier
             mbar_expect_tx(bar(bars.b_full[bb]), S * B_BYTES);
             for (int j = 0; j < S; ++j) {
-              const __nv_bfloat16* src = pb + (((int64_t)j * g.SB.nsub + s) * ntB + tB) * (TM * 64) + (int64_t)hB * 64;
+              const __nv_bfloat16* src = pb + (((int64_t)s * ntB + tB) * S + j) * (TM * 64) + (int64_t)hB * 64;
               bulk_g2s(sB + bb * B_BUF + j * B_BYTES, src, B_BYTES, bar(bars.b_full[bb]));
             }
             last_fill_b[bb] = (int)(ub >> 1);
-            ++ub;
-            for (int i = 0; i < S; ++i) {
+            for (int gi = 0; gi < NG; ++gi) {
               const int st = ua % NA;
               const uint32_t us = ua / NA;
               if (!mbar_wait(bar(bars.a_empty[st]), (us & 1) ^ 1)) {
-                record_expiry(2, ti, kb, s, i, ua, ub, 0);
+                record_expiry(2, ti, kb, s, gi, ua, ub, 0);
                 ok = false;
                 break;
               }
-              mbar_expect_tx(bar(bars.a_full[st]), A_BYTES);
-              const __nv_bfloat16* src = pa + (((int64_t)i * g.SA.nsub + s) * ntA + tA) * (TM * 64);
-              bulk_g2s(sA + st * A_BYTES, src, A_BYTES, bar(bars.a_full[st]));
+              const uint32_t abytes = (uint32_t)min(GA, S - gi * GA) * IMG_BYTES;
+              mbar_expect_tx(bar(bars.a_full[st]), abytes);
+              bulk_g2s(sA + st * A_BYTES, pa + (((int64_t)s * ntA + tA) * S + gi * GA) * (TM * 64), abytes,
+                       bar(bars.a_full[st]));
               last_fill_a[st] = (int)us;
               ++ua;
             }
+            ++ub;
           }
         }
       }
@@ -456,15 +478,14 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_oz7_gemm(Oz7Args g, long long n
               ok = false;
               break;
             }
-            asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
             // descriptors advance with the address: +2 per 32-byte (16-element) step along k, so each MMA costs one
             // add and one issue
             const uint64_t bdesc0 = sdesc(sB + bb * B_BUF);
 #pragma unroll
-            for (int i = 1; i <= S; ++i) {
+            for (int gi = 0; gi < NG; ++gi) {
               const int st = ua % NA;
               if (!mbar_wait(bar(bars.a_full[st]), (ua / NA) & 1)) {
-                record_expiry(5, ti, kb, s, i, ua, ub, uacc);
+                record_expiry(5, ti, kb, s, gi, ua, ub, uacc);
                 ok = false;
                 break;
               }
@@ -472,17 +493,21 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_oz7_gemm(Oz7Args g, long long n
               const uint64_t adesc0 = sdesc(sA + st * A_BYTES);
               // A digit i meets B digits 1 .. S + 1 - i: adjacent TN-row blocks of one K-major operand, whose
               // diagonals i + 1 .. S + 1 are adjacent TN-column blocks of TMEM -- MMAs of up to N = 256 (256 / TN
-              // digits each: one MMA for TN = 32)
+              // digits each: one MMA for TN = 32).  The k steps are outermost: the group's digits read the same 16
+              // columns of B one after the other (10 % over a digit's four k steps in a row)
 #pragma unroll
-              for (int j0 = 1; j0 <= S + 1 - i; j0 += 256 / TN) {
-                const int k = (S + 2 - i - j0) < 256 / TN ? (S + 2 - i - j0) : 256 / TN;
-                const uint32_t d = tset + (uint32_t)((i + j0 - 2) * TN);
-                const uint64_t bdesc = bdesc0 + (uint64_t)((j0 - 1) * (B_BYTES >> 4));
-                const uint32_t idesc = idesc_n(TN * k);
+              for (int kk = 0; kk < 4; ++kk) {
 #pragma unroll
-                for (int kk = 0; kk < 4; ++kk)
-                  mma_issue(d, adesc0 + (uint64_t)(2 * kk), bdesc + (uint64_t)(2 * kk), idesc,
-                            (!first_sub || i > 1 || kk > 0) ? 1u : 0u);
+                for (int i = gi * GA + 1; i <= (gi + 1) * GA && i <= S; ++i) {
+#pragma unroll
+                  for (int j0 = 1; j0 <= S + 1 - i; j0 += 256 / TN) {
+                    const int k = (S + 2 - i - j0) < 256 / TN ? (S + 2 - i - j0) : 256 / TN;
+                    mma_issue(tset + (uint32_t)((i + j0 - 2) * TN),
+                              adesc0 + (uint64_t)((i - 1 - gi * GA) * (IMG_BYTES >> 4) + 2 * kk),
+                              bdesc0 + (uint64_t)((j0 - 1) * (B_BYTES >> 4) + 2 * kk), idesc_n(TN * k),
+                              (!first_sub || i > 1 || kk > 0) ? 1u : 0u);
+                  }
+                }
               }
               mma_commit(bar(bars.a_empty[st]));
               issued = true;
@@ -575,7 +600,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_oz7_gemm(Oz7Args g, long long n
             const int col = col0 + q0 + q;
             if (row < g.M && col < g.N && (!tri || row >= col)) {
               // the block's exact product, in units 2^(er + ec - 7 (S + 1)), rounded once
-              const double val = fold_diagonals<S>(v, q, er + ec[q] - 7 * (S + 1));
+              const int E = er + ec[q] - 7 * (S + 1);
+              const double val = E > kNanExp / 2 ? __longlong_as_double(0x7FF8000000000000ll) : fold_diagonals<S>(v, q, E);
               double out;
               switch (upd) {
                 case 0: out = val; break;
@@ -604,7 +630,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_oz7_gemm(Oz7Args g, long long n
 
 template <int S, int TN>
 void launch_oz7(const Oz7Args& a, long long ntiles, int batch, int max_ctas, cudaStream_t st) {
-  const size_t smem = (size_t)ring_depth<S, TN>() * A_BYTES + 2 * S * b_bytes<TN>() + 1024;
+  const size_t smem = (size_t)ring_depth<S, TN>() * group_size<S, TN>() * IMG_BYTES + 2 * S * b_bytes<TN>() + 1024;
   static bool attr = false;
   if (!attr) {
     LKG_CUDA(cudaFuncSetAttribute(k_oz7_gemm<S, TN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));

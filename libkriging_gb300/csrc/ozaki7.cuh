@@ -11,7 +11,7 @@ constexpr int OZ7_SUB = 64;      // k sub-chunk of one staged digit image (128 b
 constexpr int OZ7_MAX_SPB = 4;   // sub-chunks per exponent block: at most 256 columns (exact FP32 sums)
 constexpr int OZ7_KB = 256;      // the k block of the trailing updates and of W^T W
 
-// planes [batch][S][nsub][rows_pad / 128][128 x 64 bf16 swizzled image]; exps [batch][nblk][rows_pad]
+// planes [batch][nsub][rows_pad / 128][S][128 x 64 bf16 swizzled image]; exps [batch][nblk][rows_pad]
 struct Split7 {
   __nv_bfloat16* planes = nullptr;
   int* exps = nullptr;
@@ -58,7 +58,7 @@ void oz7_set_tile(int tn);
 int oz7_tile();
 // 1 if a CTA gave up waiting since the last call (then reset); synchronous.  where (8 ints, optional): the first
 // expired wait -- role (1, 2 producer B / A; 3, 4, 5 MMA TMEM / B / A; 6 + 16 warp epilogue), tile, k block,
-// sub-chunk, digit and the role's counters
+// sub-chunk, digit group and the role's counters
 int oz7_error_and_reset(int* where = nullptr);
 
 }  // namespace lkg
