@@ -46,17 +46,21 @@ void wtw_lower(const double* W, int64_t ldw, int64_t wstride, int n, double* C, 
 void copy_dinv_block(const double* Dinv, int64_t dinv_bstride, int blk, double* W, int64_t ldw, int64_t wstride,
                      int k0, int nb, int batch, cudaStream_t st);
 
-// Mixed-precision variants (trailing updates, trtri updates and W^T W on the bf16 tensor cores by error-free
-// splitting into 7-bit digit planes, see ozaki7.cuh); the diagonal blocks stay FP64.
+// Digit-product variants: the O(n^3) products on the bf16 tensor cores by error-free splitting into 7-bit digits
+// (ozaki7.cuh); the diagonal blocks stay FP64.  With 8 digits (56-bit operands, one rounding per 256 columns) they
+// serve the FP64 path too: see digits_pay().
+constexpr int FP64_DIGITS = 8;
 struct MixedWorkspace {
-  int slices = 7;      // digit slices of the Cholesky's trailing updates
-  int slices_inv = 6;  // digit slices of the triangular inverse and W^T W (gradient only)
+  int digits = FP64_DIGITS;      // digits of the Cholesky's products (6 .. 8)
+  int digits_inv = FP64_DIGITS;  // digits of the triangular inverse and W^T W, which feed only the gradient (5 .. 8)
+  bool wide = true;              // 8-bit leading digits (ozaki7.cu)
   void* panel = nullptr;  // bf16 planes, oz7_plane_elems(n, 256, 8) per batch entry
   int* panel_exp = nullptr;
   void* rowblk = nullptr;  // bf16 planes, same size
   int* rowblk_exp = nullptr;
-  void* wfull = nullptr;  // bf16 planes, oz7_plane_elems(n, n, digits) per batch entry
-  int* wfull_exp = nullptr;
+  void* wchunk = nullptr;  // bf16 planes, oz7_plane_elems(n, wk, 8) per batch entry
+  int* wchunk_exp = nullptr;
+  int wk = 0;  // columns of a chunk of the long products (W^T W, square products): a multiple of 256, at least 512
   int n = 0;
   // look-ahead of the blocked Cholesky (single matrix): the next panel is factored on side_stream, on side_ctas SMs
   // kept free by the trailing update, with its splits in side / side_exp (the size of panel); off when null
@@ -72,6 +76,16 @@ void trtri_blocked_mixed(const double* L, int64_t lda, int64_t mstride, int n, c
                          int64_t ldw, int64_t wstride, int batch, const MixedWorkspace& ws, cudaStream_t st);
 void wtw_lower_mixed(const double* W, int64_t ldw, int64_t wstride, int n, double* C, int64_t ldc, int64_t cstride,
                      int batch, const MixedWorkspace& ws, cudaStream_t st);
+
+// C (n x n, ldc) = A B with A, B n x n column-major (lda, ldb), FP64_DIGITS digits, in chunks of ws.wk / 2 columns of A
+void gemm_square_digits(int n, const double* A, int64_t lda, const double* B, int64_t ldb, double* C, int64_t ldc,
+                        const MixedWorkspace& ws, cudaStream_t st);
+// Bytes of scratch for trsm_lower_left_digits, and L X = B in place (B n x r column-major, ldb; one matrix)
+size_t trsm_digits_bytes(int n, int r);
+void trsm_lower_left_digits(const double* L, int64_t lda, int n, const double* Dinv, double* B, int64_t ldb, int r,
+                            void* scratch, cudaStream_t st);
+// Whether the FP64 path runs its products over n x n factors as 8-digit products (else as DFMA tiles).
+bool digits_pay(int n);
 
 // Dinv blocks (nblk * NB * NB per matrix) of an existing lower factor L: the inverses of its NB x NB diagonal
 // blocks, computed exactly as potrf_diag computes them.

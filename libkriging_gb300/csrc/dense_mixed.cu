@@ -3,16 +3,11 @@
 #include "dense_fp64.cuh"
 #include "ozaki7.cuh"
 
+#include <algorithm>
+
 namespace lkg {
 
 namespace {
-
-// digits of the 7-bit split of the factorisation for a given count of 8-bit slices: the same operand precision, one
-// digit more (6 .. 8)
-int oz7_digits(int slices) { return std::min(8, std::max(6, slices + 1)); }
-// digits of the triangular inverse and of W^T W, which feed only the gradient: as many 7-bit digits as the inverse
-// has 8-bit slices (5 .. 8)
-int oz7_inv_digits(int slices_inv) { return std::min(8, std::max(5, slices_inv)); }
 
 // Two-level blocked Cholesky: 256-wide panels factored in 64-wide steps (FP64 diagonal block; panel solve and the update
 // of the panel's remaining columns as 64-deep digit products), then one rank-256 trailing update per panel.  Every
@@ -49,10 +44,10 @@ void factor_panel7(double* A, int64_t lda, int64_t mstride, int n, int K0, doubl
 void potrf_blocked_mixed7(double* A, int64_t lda, int64_t mstride, int n, double* Dinv, int* info, int batch,
                           const MixedWorkspace& ws, cudaStream_t st) {
   LKG_CUDA(cudaMemsetAsync(info, 0, sizeof(int) * batch, st));
-  const int S = oz7_digits(ws.slices);
-  Split7 P = oz7_buffer(ws.panel, ws.panel_exp, S, ws.n, OZ7_KB, OZ7_KB);
-  Split7 SA = oz7_buffer(ws.panel, ws.panel_exp, S, ws.n, NB, NB);
-  Split7 SD = oz7_buffer(ws.rowblk, ws.rowblk_exp, S, ws.n, NB, NB);
+  const int S = ws.digits;
+  Split7 P = oz7_buffer(ws.panel, ws.panel_exp, S, ws.n, OZ7_KB, OZ7_KB, ws.wide);
+  Split7 SA = oz7_buffer(ws.panel, ws.panel_exp, S, ws.n, NB, NB, ws.wide);
+  Split7 SD = oz7_buffer(ws.rowblk, ws.rowblk_exp, S, ws.n, NB, NB, ws.wide);
   const bool ahead = ws.side_stream && batch == 1;
   if (!ahead) {
     for (int K0 = 0; K0 < n; K0 += OZ7_KB) {
@@ -69,7 +64,7 @@ void potrf_blocked_mixed7(double* A, int64_t lda, int64_t mstride, int n, double
   }
   // the side stream's panel splits have their own buffer: the main stream's trailing update still reads P (the
   // Dinv splits in rowblk are used by one stream at a time)
-  Split7 SAs = oz7_buffer(ws.side, ws.side_exp, S, ws.n, NB, NB);
+  Split7 SAs = oz7_buffer(ws.side, ws.side_exp, S, ws.n, NB, NB, ws.wide);
   const int rest_ctas = std::max(1, oz7_sm_count() - ws.side_ctas);
   factor_panel7(A, lda, mstride, n, 0, Dinv, info, batch, SA, SD, 0, st);
   for (int K0 = 0; K0 < n; K0 += OZ7_KB) {
@@ -130,11 +125,11 @@ void trtri_blocked_mixed7(const double* L, int64_t lda, int64_t mstride, int n, 
   const int64_t dstride = (int64_t)nblk * NB * NB;
   for (int b = 0; b < batch; ++b)
     LKG_CUDA(cudaMemset2DAsync(W + b * wstride, ldw * sizeof(double), 0, n * sizeof(double), n, st));
-  const int S = oz7_inv_digits(ws.slices_inv);
-  Split7 SL = oz7_buffer(ws.panel, ws.panel_exp, S, ws.n, OZ7_KB, OZ7_KB);
-  Split7 SR = oz7_buffer(ws.rowblk, ws.rowblk_exp, S, ws.n, OZ7_KB, OZ7_KB);
-  Split7 SA = oz7_buffer(ws.panel, ws.panel_exp, S, ws.n, NB, NB);
-  Split7 SB = oz7_buffer(ws.rowblk, ws.rowblk_exp, S, ws.n, NB, NB);
+  const int S = ws.digits_inv;
+  Split7 SL = oz7_buffer(ws.panel, ws.panel_exp, S, ws.n, OZ7_KB, OZ7_KB, ws.wide);
+  Split7 SR = oz7_buffer(ws.rowblk, ws.rowblk_exp, S, ws.n, OZ7_KB, OZ7_KB, ws.wide);
+  Split7 SA = oz7_buffer(ws.panel, ws.panel_exp, S, ws.n, NB, NB, ws.wide);
+  Split7 SB = oz7_buffer(ws.rowblk, ws.rowblk_exp, S, ws.n, NB, NB, ws.wide);
   for (int K0 = 0; K0 < n; K0 += OZ7_KB) {
     const int Wd = std::min(OZ7_KB, n - K0);
     trtri_block7(L, lda, mstride, n, K0, Wd, Dinv, dstride, W, ldw, wstride, batch, SA, SB, st);
@@ -148,11 +143,17 @@ void trtri_blocked_mixed7(const double* L, int64_t lda, int64_t mstride, int n, 
   }
 }
 
+// R^-1 = W^T W in chunks of ws.wk rows of W: rows past the chunk's last hold no entry of it (W is lower triangular), so
+// chunk c0 updates the leading c0 + kc block.  Every tile adds its 256-row blocks in ascending order, one rounding
+// each, whatever the chunk, so the result does not depend on ws.wk.
 void wtw_lower_mixed7(const double* W, int64_t ldw, int64_t wstride, int n, double* C, int64_t ldc, int64_t cstride,
                       int batch, const MixedWorkspace& ws, cudaStream_t st) {
-  Split7 SW = oz7_buffer(ws.wfull, ws.wfull_exp, oz7_inv_digits(ws.slices_inv), ws.n, ws.n, OZ7_KB);
-  oz7_split(n, n, W, ldw, 1, wstride, batch, SW, st);  // rows of the split = columns of W, k = rows of W
-  oz7_wtw(n, SW, C, ldc, cstride, batch, st);
+  Split7 SW = oz7_buffer(ws.wchunk, ws.wchunk_exp, ws.digits_inv, ws.n, ws.wk, OZ7_KB, ws.wide);
+  for (int c0 = 0; c0 < n; c0 += ws.wk) {
+    const int kc = std::min(ws.wk, n - c0);
+    oz7_split(c0 + kc, kc, W + c0, ldw, 1, wstride, batch, SW, st);  // rows of the split = columns of W
+    oz7_wtw(c0 + kc, c0, SW, C, ldc, cstride, batch, st);
+  }
 }
 
 }  // namespace
@@ -171,5 +172,74 @@ void wtw_lower_mixed(const double* W, int64_t ldw, int64_t wstride, int n, doubl
                      int batch, const MixedWorkspace& ws, cudaStream_t st) {
   wtw_lower_mixed7(W, ldw, wstride, n, C, ldc, cstride, batch, ws, st);
 }
+
+void gemm_square_digits(int n, const double* A, int64_t lda, const double* B, int64_t ldb, double* C, int64_t ldc,
+                        const MixedWorkspace& ws, cudaStream_t st) {
+  const int S = FP64_DIGITS, kh = ws.wk / 2 / OZ7_KB * OZ7_KB;  // half of the chunk buffer for each operand
+  __nv_bfloat16* planes = static_cast<__nv_bfloat16*>(ws.wchunk);
+  Split7 SA = oz7_buffer(planes, ws.wchunk_exp, S, ws.n, kh, OZ7_KB, true);
+  Split7 SB = oz7_buffer(planes + oz7_plane_elems(ws.n, kh, S), ws.wchunk_exp + oz7_exp_elems(ws.n, kh, OZ7_KB), S, ws.n,
+                         kh, OZ7_KB, true);
+  for (int c0 = 0; c0 < n; c0 += kh) {
+    const int kc = std::min(kh, n - c0);
+    oz7_split2(n, kc, A + (int64_t)c0 * lda, 1, lda, 0, SA, n, kc, B + c0, ldb, 1, 0, SB, 1, st);
+    oz7_gemm(n, n, 0, SA.nblk, 1.0, SA, SB, c0 == 0 ? 0.0 : 1.0, C, ldc, 0, 1, false, st);
+  }
+}
+
+size_t trsm_digits_bytes(int n, int r) {
+  auto bytes = [](int rows) {
+    return oz7_plane_elems(rows, OZ7_KB, FP64_DIGITS) * sizeof(__nv_bfloat16) +
+           (oz7_exp_elems(rows, OZ7_KB, NB) * sizeof(int) + 255) / 256 * 256;
+  };
+  return bytes(n) + bytes(r);
+}
+
+// Two-level forward substitution with many right-hand sides, the structure of the digit Cholesky: inside a 256-row panel
+// the 64-row steps X_k = Dinv_k B_k and the update of the panel's remaining rows, then one rank-256 update of the rows
+// below.  A column's result depends on that column alone (its own exponents), so predictions do not depend on how the
+// points are grouped.
+void trsm_lower_left_digits(const double* L, int64_t lda, int n, const double* Dinv, double* B, int64_t ldb, int r,
+                            void* scratch, cudaStream_t st) {
+  const int S = FP64_DIGITS;
+  char* at = static_cast<char*>(scratch);
+  void* lp = at;
+  at += oz7_plane_elems(n, OZ7_KB, S) * sizeof(__nv_bfloat16);
+  void* xp = at;
+  at += oz7_plane_elems(r, OZ7_KB, S) * sizeof(__nv_bfloat16);
+  int* le = reinterpret_cast<int*>(at);
+  int* xe = le + (oz7_exp_elems(n, OZ7_KB, NB) * sizeof(int) + 255) / 256 * 64;
+  Split7 SL = oz7_buffer(lp, le, S, n, OZ7_KB, OZ7_KB, true);
+  Split7 SX = oz7_buffer(xp, xe, S, r, OZ7_KB, OZ7_KB, true);
+  Split7 sl = oz7_buffer(lp, le, S, n, NB, NB, true), sx = oz7_buffer(xp, xe, S, r, NB, NB, true);
+  for (int K0 = 0; K0 < n; K0 += OZ7_KB) {
+    const int Wd = std::min(OZ7_KB, n - K0);
+    for (int k0 = K0; k0 < K0 + Wd; k0 += NB) {
+      const int nb = std::min(NB, n - k0), k = k0 / NB;
+      oz7_split2(nb, nb, Dinv + (int64_t)k * NB * NB, 1, NB, 0, sl, r, nb, B + k0, ldb, 1, 0, sx, 1, st);
+      oz7_gemm(nb, r, 0, 1, 1.0, sl, sx, 0.0, B + k0, ldb, 0, 1, false, st);
+      const int mr = K0 + Wd - (k0 + nb);
+      if (mr > 0) {
+        oz7_split2(mr, nb, L + (k0 + nb) + (int64_t)k0 * lda, 1, lda, 0, sl, r, nb, B + k0, ldb, 1, 0, sx, 1, st);
+        oz7_gemm(mr, r, 0, 1, -1.0, sl, sx, 1.0, B + k0 + nb, ldb, 0, 1, false, st);
+      }
+    }
+    const int M2 = n - K0 - Wd;
+    if (M2 <= 0) continue;
+    oz7_split2(M2, Wd, L + (K0 + Wd) + (int64_t)K0 * lda, 1, lda, 0, SL, r, Wd, B + K0, ldb, 1, 0, SX, 1, st);
+    oz7_gemm(M2, r, 0, 1, -1.0, SL, SX, 1.0, B + K0 + Wd, ldb, 0, 1, false, st);
+  }
+}
+
+// The FP64 path's products as digit products: GB300 issues one FP64 warp instruction per 19 clocks and SM (1.25 TFLOP/s
+// over the chip), so 36 exact bf16 products of 7-bit digits are 10 to 30 times faster than one DFMA, and from the first
+// few blocks on also shorter: a 64 x 64 x 64 DFMA tile takes its SM 70 us, a digit launch 10.  Their error is no larger:
+// one rounding per 256 columns instead of one per column, on operands of 57 bits (relative errors of LL, gradient and
+// leave-one-out against extended precision, 12 designs x 6 seeds, n = 300 and 520, geometric mean: 2.4e-13 here, 4.5e-13
+// with DFMA tiles; n = 2048 at cond(R) near 1e10: gradient 2.8e-11 here, 1.2e-10 with DFMA tiles).  Measured, LL + gradient, d = 4, matern5_2 with nugget, one
+// matrix (us, DFMA / digits): n = 192 1518 / 854, 256 2015 / 1047, 512 4058 / 1825, 1024 8313 / 3394, 2048 22087 / 7343;
+// 32 matrices at once, gauss: n = 192 2247 / 1415, 512 9569 / 3860.  The rule looks at n alone, so that a matrix gives
+// the same bits alone and in a batch.
+bool digits_pay(int n) { return n >= 192; }
 
 }  // namespace lkg

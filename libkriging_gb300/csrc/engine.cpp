@@ -156,9 +156,9 @@ Engine::~Engine() {
   if (dgls_info_) cudaFree(dgls_info_);
   if (dXe_) cudaFree(dXe_);
   if (dnv_) cudaFree(dnv_);
-  for (void* p : {dpanel_, drowblk_, dwfull_, dside_})
+  for (void* p : {dpanel_, drowblk_, dwchunk_, dside_})
     if (p) cudaFree(p);
-  for (int* p : {dpanel_exp_, drowblk_exp_, dwfull_exp_, dside_exp_})
+  for (int* p : {dpanel_exp_, drowblk_exp_, dwchunk_exp_, dside_exp_})
     if (p) cudaFree(p);
   if (ev_strip_) cudaEventDestroy(ev_strip_);
   if (ev_panel_) cudaEventDestroy(ev_panel_);
@@ -280,24 +280,12 @@ bool Engine::lookahead_enabled() const { return n_ >= 4 * OZ7_KB && lookahead_ct
 
 int Engine::lookahead_ctas() const { return lookahead_ctas_for(n_); }
 
-void Engine::ensure_mixed_buffers(bool with_grad) {
-  if (mixed_alloc_slices_ != slices_) {
-    buffers_changed();
-    for (void** p : {&dpanel_, &drowblk_, &dwfull_, &dside_})
-      if (*p) {
-        cudaFree(*p);
-        *p = nullptr;
-      }
-    for (int** p : {&dpanel_exp_, &drowblk_exp_, &dwfull_exp_, &dside_exp_})
-      if (*p) {
-        cudaFree(*p);
-        *p = nullptr;
-      }
-    mixed_alloc_slices_ = slices_;
-  }
+bool Engine::digit_path() const { return slices_ > 0 || digits_pay(n_); }
+
+MixedWorkspace Engine::digit_workspace(int batch, bool long_products) {
   // up to 8 7-bit digits of a 256-wide panel per batch entry (ozaki7.cuh)
-  const size_t pe = oz7_plane_elems(n_, OZ7_KB, 8) * cap_;
-  const size_t ee = oz7_exp_elems(n_, OZ7_KB, OZ7_KB) * cap_;
+  const size_t pe = oz7_plane_elems(n_, OZ7_KB, FP64_DIGITS) * cap_;
+  const size_t ee = oz7_exp_elems(n_, OZ7_KB, NB) * cap_;
   if (!dpanel_) {
     buffers_changed();
     LKG_CUDA(cudaMalloc(&dpanel_, pe * 2));
@@ -308,7 +296,7 @@ void Engine::ensure_mixed_buffers(bool with_grad) {
   // the look-ahead's own panel splits (single-matrix evaluations of a size where it pays)
   if (lookahead_enabled() && !dside_) {
     buffers_changed();
-    const size_t pe1 = oz7_plane_elems(n_, OZ7_KB, 8), ee1 = oz7_exp_elems(n_, OZ7_KB, OZ7_KB);
+    const size_t pe1 = oz7_plane_elems(n_, OZ7_KB, FP64_DIGITS), ee1 = oz7_exp_elems(n_, OZ7_KB, NB);
     LKG_CUDA(cudaMalloc(&dside_, pe1 * 2));
     dalloc(&dside_exp_, ee1);
     if (!side_st_) {
@@ -317,11 +305,40 @@ void Engine::ensure_mixed_buffers(bool with_grad) {
       LKG_CUDA(cudaEventCreateWithFlags(&ev_panel_, cudaEventDisableTiming));
     }
   }
-  if (with_grad && !dwfull_) {
+  // the long products' operand in chunks of at most 512 MiB (a whole n x n split would take twice the matrix)
+  if (long_products && !dwchunk_) {
     buffers_changed();
-    LKG_CUDA(cudaMalloc(&dwfull_, oz7_plane_elems(n_, n_, std::min(8, slices_ + 1)) * cap_ * 2));
-    dalloc(&dwfull_exp_, oz7_exp_elems(n_, n_, OZ7_KB) * cap_);
+    const size_t per_k = oz7_plane_elems(n_, OZ7_KB, FP64_DIGITS) / OZ7_KB * 2 * cap_;  // bytes per column
+    const int64_t fit = (int64_t)(((size_t)512 << 20) / per_k) / OZ7_KB * OZ7_KB;
+    wchunk_k_ = (int)std::max<int64_t>(2 * OZ7_KB, std::min<int64_t>(fit, ceil_div(n_, OZ7_KB) * (int64_t)OZ7_KB));
+    LKG_CUDA(cudaMalloc(&dwchunk_, oz7_plane_elems(n_, wchunk_k_, FP64_DIGITS) * cap_ * 2));
+    dalloc(&dwchunk_exp_, oz7_exp_elems(n_, wchunk_k_, OZ7_KB) * cap_);
   }
+  MixedWorkspace mw;
+  if (slices_ > 0) {
+    // one 7-bit digit more than 8-bit slices holds the same operand; L^-1 and R^-1 feed only the gradient (tolerance
+    // 1e-6): two slices fewer, each slice dropped costing about two decimal digits of the gradient
+    mw.digits = std::min(8, std::max(6, slices_ + 1));
+    mw.digits_inv = std::min(8, std::max(5, std::max(4, slices_ - 2)));
+    mw.wide = false;
+  }
+  mw.n = n_;
+  mw.panel = dpanel_;
+  mw.panel_exp = dpanel_exp_;
+  mw.rowblk = drowblk_;
+  mw.rowblk_exp = drowblk_exp_;
+  mw.wchunk = dwchunk_;
+  mw.wchunk_exp = dwchunk_exp_;
+  mw.wk = wchunk_k_;
+  if (batch == 1 && dside_ && lookahead_enabled()) {
+    mw.side_stream = side_st_;
+    mw.ev_strip = ev_strip_;
+    mw.ev_panel = ev_panel_;
+    mw.side = dside_;
+    mw.side_exp = dside_exp_;
+    mw.side_ctas = lookahead_ctas();
+  }
+  return mw;
 }
 
 void Engine::ensure_grad_buffers() {
@@ -339,15 +356,22 @@ const double* Engine::factor_inverse() {
     dalloc(&dWp_, (size_t)mstride_);
   }
   if (!wp_valid_) {
+    // DFMA tiles: products with a whole L^-1 need its small entries to their own precision, which digit products
+    // (exponents per 256-wide block) do not keep; on ill-conditioned factors the predictions would lose a digit
     trtri_blocked(dA_, lda_, mstride_, n_, dDinv_, dWp_, lda_, mstride_, 1, st_);
     wp_valid_ = true;
   }
   return dWp_;
 }
 
-void Engine::solve_lower_inplace(int b, double* dB, int64_t ldb, int r) const {
-  trsm_lower_left(dA_ + (size_t)b * mstride_, lda_, mstride_, n_, dDinv_ + (size_t)b * dstride_, dB, ldb, 0, r, 1,
-                  st_);
+size_t Engine::solve_scratch_bytes(int r) const { return r > 16 && digits_pay(n_) ? trsm_digits_bytes(n_, r) : 0; }
+
+void Engine::solve_lower_inplace(int b, double* dB, int64_t ldb, int r, void* scratch) const {
+  if (r > 16 && digits_pay(n_))
+    trsm_lower_left_digits(dA_ + (size_t)b * mstride_, lda_, n_, dDinv_ + (size_t)b * dstride_, dB, ldb, r, scratch, st_);
+  else
+    trsm_lower_left(dA_ + (size_t)b * mstride_, lda_, mstride_, n_, dDinv_ + (size_t)b * dstride_, dB, ldb, 0, r, 1,
+                    st_);
 }
 
 // dtrcon('1', 'L', 'N') style estimate (LAPACK dlacn2 iteration of Hager / Higham) of rcond(L)^2 for every entry,
@@ -517,36 +541,16 @@ void Engine::evaluate(int batch, const double* thetas, const double* factors, bo
   std::vector<char> dead(batch, 0);
   std::vector<int> info(batch, 0);
   std::vector<double> rc2(batch, -1.0);
+  bool digit = digit_path();  // digit products, else DFMA tiles
   MixedWorkspace mw;
-  if (slices_ > 0) {
-    ensure_mixed_buffers(with_grad);
-    mw.slices = slices_;
-    // L^-1 and R^-1 feed only the gradient (tolerance 1e-6): two slices fewer than the factorisation, each slice
-    // dropped costing about two decimal digits of the gradient
-    mw.slices_inv = std::max(4, slices_ - 2);
-    mw.n = n;
-    mw.panel = dpanel_;
-    mw.panel_exp = dpanel_exp_;
-    mw.rowblk = drowblk_;
-    mw.rowblk_exp = drowblk_exp_;
-    mw.wfull = dwfull_;
-    mw.wfull_exp = dwfull_exp_;
-    if (batch == 1 && dside_ && lookahead_enabled()) {
-      mw.side_stream = side_st_;
-      mw.ev_strip = ev_strip_;
-      mw.ev_panel = ev_panel_;
-      mw.side = dside_;
-      mw.side_exp = dside_exp_;
-      mw.side_ctas = lookahead_ctas();
-    }
-  }
+  if (digit) mw = digit_workspace(batch, with_grad);
   bool retreated = false;
   bool w_valid = false;  // W = L^-1 of the accepted factor is already in dW_
   // the covariance build and the factorisation as one launch sequence (a CUDA graph after its first run): its
   // inputs -- theta, factor, diagonal -- are read from device memory
   const bool graphs_ok = (bench == nullptr);
   auto factor_phase = [&](bool mixed) {
-    const std::string key = "factor:b=" + std::to_string(batch) + ":m=" + std::to_string(mixed ? slices_ : 0) +
+    const std::string key = "factor:b=" + std::to_string(batch) + ":m=" + std::to_string(mixed ? mw.digits + 100 * mw.wide : 0) +
                             ":xe=" + std::to_string(dXb == dXe_) + ":la=" +
                             std::to_string(mixed && mw.side_stream ? mw.side_ctas : 0) + ":t=" +
                             std::to_string(oz7_tile()) + ":g=" + std::to_string(buf_gen_);
@@ -560,18 +564,19 @@ void Engine::evaluate(int batch, const double* thetas, const double* factors, bo
   };
   for (int attempt = 0;; ++attempt) {
     LKG_CUDA(cudaMemcpyAsync(ddiag_, diag.data(), sizeof(double) * batch, cudaMemcpyHostToDevice, st_));
+    factor_phase(digit);
     if (slices_ > 0 && !retreated) {
-      factor_phase(true);
       LKG_CUDA(cudaMemcpyAsync(info.data(), dinfo_, sizeof(int) * batch, cudaMemcpyDeviceToHost, st_));
       LKG_CUDA(cudaStreamSynchronize(st_));
       bool any_fail = false;
       for (int b = 0; b < batch; ++b) any_fail = any_fail || (info[b] != 0 && !dead[b]);
       if (any_fail) {  // retreat: redo this factorisation on the FP64 path before the nugget-retry rules apply
         retreated = true;
-        factor_phase(false);
+        digit = digits_pay(n);
+        mw.digits = mw.digits_inv = FP64_DIGITS;
+        mw.wide = true;
+        factor_phase(digit);
       }
-    } else {
-      factor_phase(false);
     }
     LKG_CUDA(cudaMemcpyAsync(info.data(), dinfo_, sizeof(int) * batch, cudaMemcpyDeviceToHost, st_));
     LKG_CUDA(cudaStreamSynchronize(st_));
@@ -581,7 +586,7 @@ void Engine::evaluate(int batch, const double* thetas, const double* factors, bo
         // The gradient needs W = L^-1 anyway: rcond_exact = 1 / (|L|_1 |L^-1|_1) <= the dlacn2 estimate, so
         // rcond_exact^2 >= min_rcond already decides "no retry"; only entries below it run the estimator.
         ensure_grad_buffers();
-        if (slices_ > 0 && !retreated)
+        if (digit)
           trtri_blocked_mixed(dA_, lda_, mstride_, n, dDinv_, dW_, lda_, mstride_, batch, mw, st_);
         else
           trtri_blocked(dA_, lda_, mstride_, n, dDinv_, dW_, lda_, mstride_, batch, st_);
@@ -646,15 +651,14 @@ void Engine::evaluate(int batch, const double* thetas, const double* factors, bo
     out[b].nugget_increments = inc[b];
     out[b].rcond = rc2[b];
     out[b].slices = retreated ? 0 : slices_;
-    out[b].retreated = retreated;
+    out[b].retreated = retreated && slices_ > 0;
   }
   tm.lap("R = _Cov(dX) & L = Chol(R)");
 
   // ---- [F* y*] = L \ [F y], GLS, E*, SSE, and the gradient's R^-1 and adjoint sums: one launch sequence (a CUDA
   // graph after its first run) ----
   if (with_grad) ensure_grad_buffers();
-  const bool mixed_post = slices_ > 0 && !retreated;
-  const std::string post_key = "post:b=" + std::to_string(batch) + ":m=" + std::to_string(mixed_post ? slices_ : 0) +
+  const std::string post_key = "post:b=" + std::to_string(batch) + ":m=" + std::to_string(digit ? mw.digits_inv + 100 * mw.wide : 0) +
                                ":gr=" + std::to_string(with_grad) + ":w=" + std::to_string(w_valid) + ":sa=" +
                                std::to_string(skip_adjoint_) + ":xe=" + std::to_string(dXb == dXe_) + ":t=" +
                                std::to_string(oz7_tile()) + ":g=" + std::to_string(buf_gen_);
@@ -683,7 +687,7 @@ void Engine::evaluate(int batch, const double* thetas, const double* factors, bo
       LKG_CUDA(cudaMemcpyAsync(dxv_, dEstar_, sizeof(double) * n * batch, cudaMemcpyDeviceToDevice, st_));
       trsm_lower_left_t(dA_, lda_, mstride_, n, dDinv_, dxv_, n, n, 1, batch, st_);
       tm.lap("x = tL \\ z");
-      if (slices_ > 0 && !retreated) {
+      if (digit) {
         if (!w_valid) trtri_blocked_mixed(dA_, lda_, mstride_, n, dDinv_, dW_, lda_, mstride_, batch, mw, st_);
         wtw_lower_mixed(dW_, lda_, mstride_, n, dRinv_, lda_, mstride_, batch, mw, st_);
       } else {
@@ -722,8 +726,8 @@ void Engine::evaluate(int batch, const double* thetas, const double* factors, bo
     LKG_CUDA(cudaMemcpyAsync(adj.data(), dadj_, sizeof(double) * adj.size(), cudaMemcpyDeviceToHost, st_));
   }
   LKG_CUDA(cudaStreamSynchronize(st_));
-  if (slices_ > 0 && oz7_error_and_reset())
-    throw std::runtime_error("mixed path: a tensor-core digit product did not complete (timed out)");
+  if ((digit || slices_ > 0) && oz7_error_and_reset())
+    throw std::runtime_error("a tensor-core digit product did not complete (timed out)");
   for (int b = 0; b < batch; ++b) {
     EvalOut& o = out[b];
     if (o.status == 0 && gls[b] != 0) {
@@ -797,6 +801,9 @@ void Engine::leave_one_out(int batch, const double* thetas, const double* factor
   skip_adjoint_ = false;
   ensure_loo_buffers(true);
   if (p > 0) build_At(batch);
+  const bool digit = want_grad && digits_pay(n);
+  MixedWorkspace mw;
+  if (digit) mw = digit_workspace(1, true);
   out.assign(batch, LooOut());
   for (int b = 0; b < batch; ++b) {
     LooOut& o = out[b];
@@ -815,8 +822,11 @@ void Engine::leave_one_out(int batch, const double* thetas, const double* factor
       const double* th = dtheta_ + (size_t)b * d;
       for (int k = 0; k < d; ++k) {
         loo_gradR(kernel_, n, d, dX_, th, factors[b], k, G, lda_, st_);
-        gemm_tiles(n, n, n, 1.0, MatView{G, 1, lda_, 0}, MatView{Bm, 1, lda_, 0}, 0.0, dloo_m_, lda_, 0, 1, false,
-                   st_);
+        if (digit)
+          gemm_square_digits(n, G, lda_, Bm, lda_, dloo_m_, lda_, mw, st_);
+        else
+          gemm_tiles(n, n, n, 1.0, MatView{G, 1, lda_, 0}, MatView{Bm, 1, lda_, 0}, 0.0, dloo_m_, lda_, 0, 1, false,
+                     st_);
         col_dot(n, Bm, lda_, dloo_m_, lda_, dloo_vec_ + (size_t)(2 + 2 * k) * n, st_);  // diag(B G_k B)
         col_dot(n, By, 0, dloo_m_, lda_, dloo_vec_ + (size_t)(3 + 2 * k) * n, st_);     // (G_k B)' By
       }
@@ -825,6 +835,8 @@ void Engine::leave_one_out(int batch, const double* thetas, const double* factor
     std::vector<double> hv((size_t)n * nvec);
     LKG_CUDA(cudaMemcpyAsync(hv.data(), dloo_vec_, sizeof(double) * hv.size(), cudaMemcpyDeviceToHost, st_));
     LKG_CUDA(cudaStreamSynchronize(st_));
+    if (digit && oz7_error_and_reset())
+      throw std::runtime_error("leave-one-out: a tensor-core digit product did not complete (timed out)");
     // host assembly (Kriging.cpp:411-465), n-vectors only
     const double* dg = hv.data();
     const double* by = hv.data() + n;
@@ -1004,8 +1016,16 @@ void Engine::model_matrices(const double* theta, double factor, std::vector<doub
     mirror(*R);
   }
   if (Rinv) {
-    trtri_blocked(dA_, lda_, mstride_, n, dDinv_, dW_, lda_, mstride_, 1, st_);
-    wtw_lower(dW_, lda_, mstride_, n, dRinv_, lda_, mstride_, 1, st_);
+    if (digits_pay(n)) {
+      MixedWorkspace mw = digit_workspace(1, true);
+      mw.digits_inv = FP64_DIGITS;
+      mw.wide = true;
+      trtri_blocked_mixed(dA_, lda_, mstride_, n, dDinv_, dW_, lda_, mstride_, 1, mw, st_);
+      wtw_lower_mixed(dW_, lda_, mstride_, n, dRinv_, lda_, mstride_, 1, mw, st_);
+    } else {
+      trtri_blocked(dA_, lda_, mstride_, n, dDinv_, dW_, lda_, mstride_, 1, st_);
+      wtw_lower(dW_, lda_, mstride_, n, dRinv_, lda_, mstride_, 1, st_);
+    }
     Rinv->assign((size_t)n * n, 0.0);
     LKG_CUDA(cudaMemcpy2DAsync(Rinv->data(), sizeof(double) * n, dRinv_, sizeof(double) * lda_, sizeof(double) * n,
                                n, cudaMemcpyDeviceToHost, st_));

@@ -13,6 +13,7 @@
 #include <vector>
 
 #include "config.hpp"
+#include "dense_fp64.cuh"
 
 namespace lkg {
 
@@ -133,8 +134,9 @@ class Engine {
   int64_t mstride() const { return mstride_; }
   const double* dFY(int b = 0) const { return dFY_ + (size_t)b * fystride_; }
   const double* dEstar(int b = 0) const { return dEstar_ + (size_t)b * n_; }
-  // solve L Z = B in place for entry b (B device, n x r, ldb)
-  void solve_lower_inplace(int b, double* dB, int64_t ldb, int r) const;
+  // solve L Z = B in place for entry b (B device, n x r, ldb); scratch: solve_scratch_bytes(r) bytes
+  void solve_lower_inplace(int b, double* dB, int64_t ldb, int r, void* scratch) const;
+  size_t solve_scratch_bytes(int r) const;
   // W = L^-1 of the (single-matrix) factor, formed once per factor on the FP64 path and kept for predictions whose
   // solves run as digit products (W R_on)
   const double* factor_inverse();
@@ -144,7 +146,11 @@ class Engine {
   void ensure_loo_buffers(bool with_product);
   // A' = L^-T F* Rstar^-1 (n x p per entry, stride n p) into dloo_at_ for entries [0, batch)
   void build_At(int batch);
-  void ensure_mixed_buffers(bool with_grad);
+  // digit products run this engine's factorisations: the mixed path, or the FP64 path at a size where they pay
+  bool digit_path() const;
+  // (re)allocates the digit buffers and describes them; long_products: also those of the inverse's W^T W and of
+  // leave-one-out's square products
+  MixedWorkspace digit_workspace(int batch, bool long_products);
   // rcond(L)^2 per entry, dtrcon('1') style estimate on each entry's first nvb[b] rows / columns
   void rcond_batch(int batch, std::vector<double>& rc2, const std::vector<int>& nvb);
   // the same estimate for the n x n lower factors at A (lda, mstride) with diagonal-block inverses Dinv
@@ -177,11 +183,11 @@ class Engine {
   double* dXe_ = nullptr;                 // per-entry copy of its design's X (several designs only)
   int* dnv_ = nullptr;                    // per-entry valid sizes on the device (several designs only)
   int slices_ = 0;
-  void *dpanel_ = nullptr, *drowblk_ = nullptr, *dwfull_ = nullptr, *dside_ = nullptr;
-  int *dpanel_exp_ = nullptr, *drowblk_exp_ = nullptr, *dwfull_exp_ = nullptr, *dside_exp_ = nullptr;
+  void *dpanel_ = nullptr, *drowblk_ = nullptr, *dwchunk_ = nullptr, *dside_ = nullptr;
+  int *dpanel_exp_ = nullptr, *drowblk_exp_ = nullptr, *dwchunk_exp_ = nullptr, *dside_exp_ = nullptr;
+  int wchunk_k_ = 0;  // columns that dwchunk_ holds
   cudaStream_t side_st_ = nullptr;  // look-ahead stream of the mixed Cholesky (single-matrix evaluations)
   cudaEvent_t ev_strip_ = nullptr, ev_panel_ = nullptr;
-  int mixed_alloc_slices_ = 0;
   int64_t lda_, mstride_, dstride_, fystride_;
   cudaStream_t st_ = nullptr;
   double *dX_ = nullptr, *dY_ = nullptr, *dF_ = nullptr;

@@ -121,9 +121,12 @@ class NestedService : public DenseService {
     // batch capacity per class: every design x starts entries, scaled down to ~70% of the free device memory
     size_t free_b = 0, total_b = 0;
     LKG_CUDA(cudaMemGetInfo(&free_b, &total_b));
-    const double per_n2 = slices > 0 ? 38.0 : 25.0;  // bytes per n^2 per entry (A, W, R^-1, digit planes)
+    // bytes per entry: A, W, R^-1, and the digit images of two 256-column panels and a 512-column chunk
     double need = 0.0;
-    for (auto& c : classes_) need += per_n2 * (double)c.n_pad * c.n_pad * c.designs.size() * starts;
+    for (auto& c : classes_) {
+      const double n = c.n_pad, digits = slices > 0 || digits_pay(c.n_pad) ? 16384.0 * ceil_div(c.n_pad, 128) * 128 : 0.0;
+      need += (25.0 * n * n + digits) * c.designs.size() * starts;
+    }
     const double scale = std::min(1.0, 0.7 * (double)free_b / std::max(need, 1.0));
     for (auto& c : classes_) {
       c.cap = std::max(1, (int)std::floor(scale * c.designs.size() * starts));

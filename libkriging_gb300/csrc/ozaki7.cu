@@ -10,7 +10,18 @@
 // diagonals are folded into FP64 once per block: adjacent diagonals paired in int32, the exact sum split into two
 // integers below 2^46 that are exact doubles, one correctly rounded FP64 addition.  S = 8 gives 56-bit operands
 // (FP64-level products); S = 5
-// (35 bits) serves the triangular inverse and W^T W, which feed only the gradient.
+// (35 bits) serves the mixed path's triangular inverse and W^T W, which feed only the gradient.
+//
+// Wide leading digits (Split7::wide): the block exponent is one smaller (max |x| 2^-e < 1), so the first digit runs over
+// [-128, 128], still exact in bf16, and every operand keeps one bit more.  The sum over i + j = g grows to
+// (2 (2) + g - 3) 2^12 per column at most (two products with a first digit, 2^13 each; 2^14 for g = 2), below
+// 10 * 256 * 2^12 < 2^24 for S = 8: still exact in FP32, a pair of diagonals below 10 * 2^27 < 2^31 in int32, and four of
+// them below 2^46.  The FP64 path uses them: the truncation and the dropped digit pairs, at 56 bits, would make its
+// results 2.5 times less accurate than DFMA products, at 57 they make them no less accurate.  What the dropped pairs
+// i + j = S + 2 hold is random from entry to entry except on the diagonal of a product of an operand with itself, where
+// the squares d_5^2 add up: left out, every diagonal entry of the Cholesky's trailing updates stays about 1e-16 of
+// its row's square too large, and log-likelihoods at n = 2048 were 20 times less accurate than with DFMA products.  So
+// the split also sums d_5^2 per (row, block), and the fold adds it to the diagonal entries before their rounding.
 //
 // Data layout: the split writes each (digit, 64-wide k sub-chunk, 128-row tile) as the 16 KB shared-memory image of
 // a K-major tile with the 128-byte swizzle (16-byte chunk c of row r at chunk c ^ (r & 7)), so the kernel moves it
@@ -176,11 +187,12 @@ __device__ __forceinline__ double exact_scaled(long long x, int e) {
 }
 
 // The block's exact product H = sum_g v_g 128^(S + 1 - g) (v_g the FP32 diagonal sums, g = 2 .. S + 1, exact
-// integers with |v_g| <= (g - 1) 2^20) times 2^E, correctly rounded: adjacent diagonals first combine in int32
+// integers with |v_g| <= (g + 1) 2^20) times 2^E, correctly rounded: adjacent diagonals first combine in int32
 // (v_g 128 + v_(g+1) < 2^31), then H = hi 2^28 + lo with lo the last four diagonals and hi the first S - 4, both
 // below 2^46 and so exact as doubles; one FP64 addition rounds their sum once (ties to even).
+// extra 128^-1 (|extra| < 2^21) joins the sum before the rounding (S > 5).
 template <int S>
-__device__ __forceinline__ double fold_diagonals(const uint32_t (&v)[S][4], int q, int E) {
+__device__ __forceinline__ double fold_diagonals(const uint32_t (&v)[S][4], int q, int E, int extra) {
   int iv[S];
 #pragma unroll
   for (int j = 0; j < S; ++j) iv[j] = __float2int_rn(__uint_as_float(v[j][q]));
@@ -192,14 +204,14 @@ __device__ __forceinline__ double fold_diagonals(const uint32_t (&v)[S][4], int 
     hi = ((long long)iv[0] << 14) + (iv[1] * 128 + iv[2]);
   else if constexpr (S == 6)
     hi = iv[0] * 128 + iv[1];
-  else  // S = 5: |H| < 2^49 is one exact double, no rounding addition
+  else  // S = 5: |H| < 2^52 is one exact double, no rounding addition
     return exact_scaled(((long long)iv[0] << 28) + lo, E);
-  return exact_scaled(hi, E + 28) + exact_scaled(lo, E);
+  return exact_scaled(hi, E + 28) + exact_scaled(lo * 128 + extra, E - 7);
 }
 
 // ---------------------------------------------------------------------------------------------------------------
-// bf16 bit pattern of a small integer d (|d| <= 64): 1.5 2^23 + d is exact in FP32, so subtracting 1.5 2^23 gives d
-// as a float whose low 16 bits are zero (at most 7 significant bits), and its high half is the bf16 value
+// bf16 bit pattern of a small integer d (|d| <= 128): 1.5 2^23 + d is exact in FP32, so subtracting 1.5 2^23 gives d
+// as a float whose low 16 bits are zero (at most 8 significant bits), and its high half is the bf16 value
 __device__ __forceinline__ uint32_t bf16_bits_of_small(int d) {
   const float f = __int_as_float(0x4B400000 + d) - 12582912.0f;
   return (uint32_t)__float_as_int(f) >> 16;
@@ -259,8 +271,9 @@ __global__ void __launch_bounds__(256) k_oz7_split(SplitJob j0, SplitJob j1, int
     const int bx = (int)(bm >> 52);
     // a block with an infinity or NaN: no digits, and an exponent that turns every product of the block into NaN
     const int E = bx == 2047 ? kNanExp - 1 : bx ? bx - 1022 : (64 - __clzll((long long)(bm & 0xFFFFFFFFFFFFFull))) - 1074;
-    e = E + 1;
+    e = E + 1 - out.wide;
   }
+  int sq = 0;
   const int ntile = out.rows_pad / 128, t = r >> 7, rr = r & 127;
   __nv_bfloat16* base = out.planes + b * out.plane_bstride;
 #pragma unroll
@@ -270,7 +283,7 @@ __global__ void __launch_bounds__(256) k_oz7_split(SplitJob j0, SplitJob j1, int
     if (s >= out.nsub) break;
     long long V[2];
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {  // V = round(x 2^(7 S - e)), |V| < 2^(7 S - 1)
+    for (int h = 0; h < 2; ++h) {  // V = round(x 2^(7 S - e)), |V| <= 2^(7 S - 1), 2^(7 S) if wide
       const unsigned long long bits = (unsigned long long)__double_as_longlong(x[2 * q + h]);
       const unsigned long long ab = bits & 0x7FFFFFFFFFFFFFFFull;
       long long v = 0;
@@ -290,9 +303,11 @@ __global__ void __launch_bounds__(256) k_oz7_split(SplitJob j0, SplitJob j1, int
     const int kk = 2 * lane, c = kk >> 3, e8 = kk & 7;
     const int64_t off = (int64_t)rr * 64 + ((c ^ (rr & 7)) << 3) + e8;
     // balanced base-128 digits in closed form: with U = V + 64 (1 + 128 + ... + 128^(S-2)), digit k (least
-    // significant first) is ((U >> 7 k) & 127) - 64 for k < S - 1 and the top digit is U >> 7 (S - 1) (|d| <= 64)
+    // significant first) is ((U >> 7 k) & 127) - 64 for k < S - 1 and the top digit is U >> 7 (S - 1) (|d| <= 64,
+    // 128 for wide leading digits)
     constexpr long long C = 64ll * ((1ll << (7 * (S - 1))) - 1) / 127;
     const long long U0 = V[0] + C, U1 = V[1] + C;
+    constexpr int MID = S / 2;  // digit (S + 2) / 2: its square heads the dropped pairs i + j = S + 2 (S even)
     // the S digit images of one (sub-chunk, tile) are adjacent, so a group of A digits is one bulk copy
     uint32_t* img = reinterpret_cast<uint32_t*>(base + ((int64_t)s * ntile + t) * S * (TM * 64) + off);
 #pragma unroll
@@ -300,10 +315,16 @@ __global__ void __launch_bounds__(256) k_oz7_split(SplitJob j0, SplitJob j1, int
       const int i = S - 1 - k;  // digit index, 0 = most significant
       const int d0 = (k < S - 1) ? (int)((U0 >> (7 * k)) & 127) - 64 : (int)(U0 >> (7 * k));
       const int d1 = (k < S - 1) ? (int)((U1 >> (7 * k)) & 127) - 64 : (int)(U1 >> (7 * k));
+      if (i == MID) sq += d0 * d0 + d1 * d1;
       img[i * (TM * 64 / 2)] = bf16_bits_of_small(d0) | (bf16_bits_of_small(d1) << 16);
     }
   }
-  if (lane == 0) out.exps[b * out.exp_bstride + (int64_t)kb * out.rows_pad + r] = e;
+  int* ex = out.exps + b * out.exp_bstride + (int64_t)kb * out.rows_pad + r;
+  if (lane == 0) ex[0] = e;
+  if (out.wide) {
+    for (int o = 16; o > 0; o >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, o);
+    if (lane == 0) ex[out.exp_bstride / 2] = sq;
+  }
 }
 
 // ---------------------------------------------------------------------------------------------------------------
@@ -327,7 +348,7 @@ __device__ __forceinline__ bool tile_of(const Oz7Args& g, long long t, Tile& T) 
     T.n0 = (int)(t / tx) * TN;
   }
   if (g.wtw) {
-    T.kb0 = T.m0 / (OZ7_SUB * g.SA.sub_per_blk);  // W is lower triangular: rows above m0 contribute zeros
+    T.kb0 = max(0, T.m0 / (OZ7_SUB * g.SA.sub_per_blk) - g.wkb);  // W is lower triangular: rows above m0 are zero
     T.kb1 = g.SA.nblk;
   } else {
     T.kb0 = g.kb0;
@@ -537,6 +558,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_oz7_gemm(Oz7Args g, long long n
     const uint32_t tl0 = tmem + ((uint32_t)(32 * quarter) << 16) + (uint32_t)(cg * CPW);
     double* Cb = g.C + bz * g.c_batch;
     const bool tri = g.lower || g.wtw;
+    const bool self = g.SA.wide && g.SA.planes == g.SB.planes;
+    const int* sqa = ea + g.SA.exp_bstride / 2;
     uint32_t uacc = 0;
     for (long long ti = blockIdx.x; ti < ntiles && ok; ti += gridDim.x) {
       Tile T;
@@ -546,12 +569,17 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_oz7_gemm(Oz7Args g, long long n
         const int set = NSET == 2 ? (int)(uacc & 1) : 0;
         const uint32_t use = NSET == 2 ? (uacc >> 1) : uacc;
         const uint32_t tl = tl0 + (uint32_t)set * TMEM_SET;
-        const bool first = (kb == T.kb0);
+        // the tile's first block over the whole product (wtw: an earlier chunk may have held it)
+        const bool first = (kb == T.kb0) && (!g.wtw || T.m0 / (OZ7_SUB * g.SA.sub_per_blk) >= g.wkb);
         const bool need_c = !(first && g.beta == 0.0);
         // operands of the update, loaded while the block's products run: the column exponents and the first four
         // C values (each group then prefetches the next group's C)
         const int er = ea[(int64_t)kb * g.SA.rows_pad + g.a_row0 + row];
         const int* ebk = eb + (int64_t)kb * g.SB.rows_pad + g.b_row0;
+        // a diagonal entry of a product of an operand with itself gets back the squares that the dropped pairs hold
+        int sq = 0;
+        const int dcol = row + g.a_row0 - g.b_row0;  // the column of this row's own operand row
+        if (self && dcol >= T.n0 && dcol < T.n0 + TN) sq = sqa[(int64_t)kb * g.SA.rows_pad + g.a_row0 + row];
         double cnext[4];
         int enext[4];
 #pragma unroll
@@ -601,7 +629,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_oz7_gemm(Oz7Args g, long long n
             if (row < g.M && col < g.N && (!tri || row >= col)) {
               // the block's exact product, in units 2^(er + ec - 7 (S + 1)), rounded once
               const int E = er + ec[q] - 7 * (S + 1);
-              const double val = E > kNanExp / 2 ? __longlong_as_double(0x7FF8000000000000ll) : fold_diagonals<S>(v, q, E);
+              const double val = E > kNanExp / 2 ? __longlong_as_double(0x7FF8000000000000ll) : fold_diagonals<S>(v, q, E, col == dcol ? sq : 0);
               double out;
               switch (upd) {
                 case 0: out = val; break;
@@ -682,15 +710,16 @@ size_t oz7_plane_elems(int rows, int K, int S) {
 }
 
 size_t oz7_exp_elems(int rows, int K, int kb) {
-  return (size_t)ceil_div(K, kb) * (ceil_div(rows, TM) * TM);
+  return (size_t)2 * ceil_div(K, kb) * (ceil_div(rows, TM) * TM);
 }
 
-Split7 oz7_buffer(void* planes, int* exps, int S, int rows_cap, int K_cap, int kb) {
+Split7 oz7_buffer(void* planes, int* exps, int S, int rows_cap, int K_cap, int kb, bool wide) {
   Split7 s;
   s.planes = static_cast<__nv_bfloat16*>(planes);
   s.exps = exps;
   s.S = S;
   s.sub_per_blk = kb / OZ7_SUB;
+  s.wide = wide ? 1 : 0;
   s.plane_bstride = (int64_t)oz7_plane_elems(rows_cap, K_cap, S);
   s.exp_bstride = (int64_t)oz7_exp_elems(rows_cap, K_cap, kb);
   return s;
@@ -706,7 +735,7 @@ void split_prepare(int rows, int K, Split7& out) {
   out.nsub = ceil_div(K, OZ7_SUB);
   out.nblk = ceil_div(out.nsub, out.sub_per_blk);
   if ((size_t)out.S * out.nsub * out.rows_pad * OZ7_SUB > (size_t)out.plane_bstride ||
-      (size_t)out.nblk * out.rows_pad > (size_t)out.exp_bstride)
+      (size_t)2 * out.nblk * out.rows_pad > (size_t)out.exp_bstride)
     throw std::logic_error("oz7_split: operand larger than its buffer");
 }
 
@@ -776,7 +805,7 @@ void oz7_gemm_ex(int M, int N, int kb0, int kb1, double alpha, const Split7& SA,
   if (SA.rows_pad < a_row0 + ceil_div(M, TM) * TM || SB.rows_pad < b_row0 + ceil_div(N, TM) * TM)
     throw std::logic_error("oz7_gemm: operand rows do not cover C");
   if (lower && M != N) throw std::invalid_argument("oz7_gemm: lower products are square");
-  Oz7Args a{M, N, kb0, kb1, alpha, beta, SA, SB, C, ldc, c_batch, lower ? 1 : 0, 0, a_row0, b_row0};
+  Oz7Args a{M, N, kb0, kb1, alpha, beta, SA, SB, C, ldc, c_batch, lower ? 1 : 0, 0, 0, a_row0, b_row0};
   const double K = std::min<double>((double)(kb1 - kb0) * SA.sub_per_blk * OZ7_SUB,
                                     (double)(SA.nsub - kb0 * SA.sub_per_blk) * OZ7_SUB);
   const double fl = lower ? K * M * (M + 1.0) : 2.0 * M * N * K;
@@ -785,11 +814,13 @@ void oz7_gemm_ex(int M, int N, int kb0, int kb1, double alpha, const Split7& SA,
   dispatch(SA.S, a, batch, st, max_ctas);
 }
 
-void oz7_wtw(int n, const Split7& SW, double* C, int64_t ldc, int64_t cstride, int batch, cudaStream_t st) {
-  Oz7Args a{n, n, 0, SW.nblk, 1.0, 0.0, SW, SW, C, ldc, cstride, 0, 1, 0, 0};
-  // executed work: tile (I, J) sums the k blocks from the one holding row 128 I
-  LaunchTimer lt("k_oz7_wtw", st, (double)n * (n + 1.0) * (n + 2.0) / 3.0 * batch * SW.S * (SW.S + 1) / 2.0,
-                 8.0 * n * (n + 1.0) * batch);
+void oz7_wtw(int n, int c0, const Split7& SW, double* C, int64_t ldc, int64_t cstride, int batch, cudaStream_t st) {
+  const int kb = OZ7_SUB * SW.sub_per_blk;
+  if (c0 < 0 || c0 % kb) throw std::invalid_argument("oz7_wtw: the first row must be a multiple of the k block");
+  Oz7Args a{n, n, 0, SW.nblk, 1.0, 0.0, SW, SW, C, ldc, cstride, 0, 1, c0 / kb, 0, 0};
+  // executed work: tile (I, J) sums the k blocks of the chunk from the one holding row 128 I
+  const double nn = n, nc = c0, below = nn * (nn + 1.0) * (nn + 2.0) - nc * (nc + 1.0) * (nc + 2.0);
+  LaunchTimer lt("k_oz7_wtw", st, below / 3.0 * batch * SW.S * (SW.S + 1) / 2.0, 8.0 * n * (n + 1.0) * batch);
   dispatch(SW.S, a, batch, st);
 }
 
@@ -833,7 +864,7 @@ extern "C" int lkg_oz7_mode_check(int mode, int M, int N, int K, const double* A
     Split7 sa = oz7_buffer(pa, ea, S, M, ka, OZ7_KB);
     if (mode == 2) {
       oz7_split(M, M, dA, M, 1, 0, 1, sa, 0);  // rows of the split = columns of W
-      oz7_wtw(M, sa, dC, M, 0, 1, 0);
+      oz7_wtw(M, 0, sa, dC, M, 0, 1, 0);
     } else {
       oz7_split(M, K, dA, 1, M, 0, 1, sa, 0);
       Split7 sb = sa;

@@ -11,11 +11,13 @@ constexpr int OZ7_SUB = 64;      // k sub-chunk of one staged digit image (128 b
 constexpr int OZ7_MAX_SPB = 4;   // sub-chunks per exponent block: at most 256 columns (exact FP32 sums)
 constexpr int OZ7_KB = 256;      // the k block of the trailing updates and of W^T W
 
-// planes [batch][nsub][rows_pad / 128][S][128 x 64 bf16 swizzled image]; exps [batch][nblk][rows_pad]
+// planes [batch][nsub][rows_pad / 128][S][128 x 64 bf16 swizzled image]; exps [batch][2][nblk][rows_pad]: the
+// block exponents, then (wide) the sums of the middle digits' squares
 struct Split7 {
   __nv_bfloat16* planes = nullptr;
   int* exps = nullptr;
   int S = 0, sub_per_blk = 0, nsub = 0, nblk = 0, rows_pad = 0;
+  int wide = 0;  // 1: 8-bit leading digits (one bit more per operand, see ozaki7.cu)
   int64_t plane_bstride = 0, exp_bstride = 0;
 };
 
@@ -27,13 +29,15 @@ struct Oz7Args {
   int64_t ldc, c_batch;
   int lower;  // square lower product: tiles on or below the diagonal, entries r >= c
   int wtw;    // R^-1 = W^T W (lower): tile (I, J) sums the k blocks from the one holding row 128 I
+  int wkb;    // wtw: the split's first k block is block wkb of W's rows
   int a_row0, b_row0;  // first operand rows of A and B in their splits (multiples of 128)
 };
 
 size_t oz7_plane_elems(int rows, int K, int S);     // bf16 elements per batch entry
-size_t oz7_exp_elems(int rows, int K, int kb);      // ints per batch entry
+size_t oz7_exp_elems(int rows, int K, int kb);      // ints per batch entry (exponents and squares)
 // a split descriptor over caller-owned buffers sized for rows_cap x K_cap, exponent block kb (64 .. 256)
-Split7 oz7_buffer(void* planes, int* exps, int S, int rows_cap, int K_cap, int kb);
+// (wide: see Split7)
+Split7 oz7_buffer(void* planes, int* exps, int S, int rows_cap, int K_cap, int kb, bool wide = false);
 
 // rows x K operand, element (r, k) at p[b*bstride + r*s_r + k*s_k], into out.S digit planes
 void oz7_split(int rows, int K, const double* p, int64_t s_r, int64_t s_k, int64_t bstride, int batch, Split7& out,
@@ -51,8 +55,9 @@ void oz7_gemm_ex(int M, int N, int kb0, int kb1, double alpha, const Split7& SA,
                  int b_row0, double beta, double* C, int64_t ldc, int64_t c_batch, int batch, bool lower, int max_ctas,
                  cudaStream_t st);
 int oz7_sm_count();
-// C = W^T W (lower) with W split by columns (rows of SW = columns of W, k = rows of W)
-void oz7_wtw(int n, const Split7& SW, double* C, int64_t ldc, int64_t cstride, int batch, cudaStream_t st);
+// C (+)= W^T W (lower, n x n) over the rows c0 .. of W in the split (rows of SW = columns of W, k = rows of W from c0, a
+// multiple of the k block): a tile whose first rows lie before c0 is added to, the others are written
+void oz7_wtw(int n, int c0, const Split7& SW, double* C, int64_t ldc, int64_t cstride, int batch, cudaStream_t st);
 // output tile width of the digit products: 32 (two TMEM accumulator sets, the default) or 64 (one set)
 void oz7_set_tile(int tn);
 int oz7_tile();

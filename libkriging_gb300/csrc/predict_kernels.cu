@@ -109,7 +109,10 @@ PredictOut predict_gpu(Engine& model, const double* Xn, int q, const double* the
   LKG_CUDA(cudaMemcpyAsync(dz.p, z, sizeof(double) * n, cudaMemcpyHostToDevice, st));
   if (whole) {
     cov_cross(model.kernel(), n, q, d, model.dX(), dXn.p, dth.p, factor, dRs.p, st);
-    model.solve_lower_inplace(0, dRs.p, n, q);
+    {
+      DevBuf dsc(model.solve_scratch_bytes(q) / sizeof(double) + 1, st);
+      model.solve_lower_inplace(0, dRs.p, n, q, dsc.p);
+    }
     predict_reduce(n, q, p, dRs.p, dz.p, dRs.p, 1, model.dFY(0), drz.p, drr.p, drm.p, st);
   } else {
     // the chunk's points as their own q x d column-major block
@@ -121,6 +124,7 @@ PredictOut predict_gpu(Engine& model, const double* Xn, int q, const double* the
     DevBuf dWs(digits ? oz7_plane_elems(n, n, S) / 4 + 1 : 1, st), dRsp(digits ? oz7_plane_elems(qc, n, S) / 4 + 1 : 1, st);
     DevBuf dWe(digits ? oz7_exp_elems(n, n, OZ7_KB) / 2 + 1 : 1, st), dRse(digits ? oz7_exp_elems(qc, n, OZ7_KB) / 2 + 1 : 1, st);
     Split7 SW, SR;
+    DevBuf dsc(digits ? 1 : model.solve_scratch_bytes(qc) / sizeof(double) + 1, st);
     if (digits) {
       SW = oz7_buffer(dWs.p, reinterpret_cast<int*>(dWe.p), S, n, n, OZ7_KB);
       SR = oz7_buffer(dRsp.p, reinterpret_cast<int*>(dRse.p), S, qc, n, OZ7_KB);
@@ -136,13 +140,11 @@ PredictOut predict_gpu(Engine& model, const double* Xn, int q, const double* the
         oz7_split(nc, n, dRs.p, n, 1, 0, 1, SR, st);
         oz7_gemm(n, nc, 0, SW.nblk, 1.0, SW, SR, 0.0, dRs.p, n, 0, 1, false, st);
       } else {
-        model.solve_lower_inplace(0, dRs.p, n, nc);
+        model.solve_lower_inplace(0, dRs.p, n, nc, dsc.p);
       }
       predict_reduce(n, nc, p, dRs.p, dz.p, dRs.p, 1, model.dFY(0), drz.p + c0, drr.p + c0,
                      drm.p + (size_t)c0 * p, st);
     }
-    if (digits && oz7_error_and_reset())
-      throw std::runtime_error("predict: a tensor-core digit product did not complete (timed out)");
   }
   o.rz.resize(q);
   o.rr.resize(q);
@@ -171,7 +173,7 @@ PredictOut predict_gpu(Engine& model, const double* Xn, int q, const double* the
     // Rstar_on(:, c) and M (KrigingImpl.cpp:254-281)
     const int qd = (int)std::max<int64_t>(1, std::min<int64_t>(q, ((int64_t)1 << 26) / ((int64_t)n * d)));
     DevBuf dW((size_t)n * qd * d, st), dwz((size_t)qd * d, st), dwr((size_t)qd * d, st),
-        dwm((size_t)qd * d * std::max(p, 1), st);
+        dwm((size_t)qd * d * std::max(p, 1), st), dsc(model.solve_scratch_bytes(qd * d) / sizeof(double) + 1, st);
     o.wz.resize((size_t)q * d);
     o.wr.resize((size_t)q * d);
     o.wm.resize((size_t)q * d * p);
@@ -184,7 +186,7 @@ PredictOut predict_gpu(Engine& model, const double* Xn, int q, const double* the
       DevBuf dxc((size_t)nc * d, st);
       LKG_CUDA(cudaMemcpyAsync(dxc.p, xc.data(), sizeof(double) * nc * d, cudaMemcpyHostToDevice, st));
       dcov_cross(model.kernel(), n, nc, d, model.dX(), dxc.p, dth.p, factor, dW.p, st);
-      model.solve_lower_inplace(0, dW.p, n, ncol);
+      model.solve_lower_inplace(0, dW.p, n, ncol, dsc.p);
       predict_reduce(n, ncol, p, dW.p, dz.p, dRs.p + (size_t)c0 * n, d, model.dFY(0), dwz.p, dwr.p, dwm.p, st);
       LKG_CUDA(cudaMemcpyAsync(o.wz.data() + (size_t)c0 * d, dwz.p, sizeof(double) * ncol, cudaMemcpyDeviceToHost,
                                st));
@@ -197,6 +199,8 @@ PredictOut predict_gpu(Engine& model, const double* Xn, int q, const double* the
     }
   }
   LKG_CUDA(cudaStreamSynchronize(st));
+  if ((digits || digits_pay(n)) && oz7_error_and_reset())
+    throw std::runtime_error("predict: a tensor-core digit product did not complete (timed out)");
   return o;
 }
 
