@@ -106,25 +106,26 @@ constexpr int DPAD = NB + 1;
 
 constexpr int PB = 16;  // panel width inside a diagonal block
 
-// Inverse of the 16 x 16 lower block of s at (jb, jb) into the same block of w, one warp, row by row: row i is scaled
-// by 1 / L_ii, then subtracted from the rows below it, w(r, c) -= L(r, i) w(i, c) for c <= i < r, with the (r, c)
-// pairs spread over the lanes.  Each entry accumulates its terms in ascending i from the identity and is scaled
-// last: the same operations, in the same order, as forward substitution column by column.
+// Inverse of the 16 x 16 lower block of s (pitch DPAD) at (jb, jb) into rows jb .. of w (pitch PB + 1, columns 0 .. 15),
+// one warp, row by row: row i is scaled by 1 / L_ii, then subtracted from the rows below it, w(r, c) -= L(r, i) w(i, c)
+// for c <= i < r, with the (r, c) pairs spread over the lanes.  Each entry accumulates its terms in ascending i from
+// the identity and is scaled last: the same operations, in the same order, as forward substitution column by column.
 __device__ __forceinline__ void diag16_inverse(const double* s, double* w, int jb, int lane) {
+  constexpr int WP = PB + 1;
   const double rdl = (lane < PB) ? __drcp_rn(s[(jb + lane) * DPAD + jb + lane]) : 0.0;
   for (int e = lane; e < PB * PB; e += 32) {
     const int r = e / PB, c = e % PB;
-    if (c <= r) w[(jb + r) * DPAD + jb + c] = (r == c) ? 1.0 : 0.0;
+    w[(jb + r) * WP + c] = (r == c) ? 1.0 : 0.0;
   }
   __syncwarp();
   for (int i = 0; i < PB; ++i) {
     const double rd = __shfl_sync(0xffffffffu, rdl, i);
-    if (lane <= i) w[(jb + i) * DPAD + jb + lane] *= rd;
+    if (lane <= i) w[(jb + i) * WP + lane] *= rd;
     __syncwarp();
     const int ncol = i + 1, nel = (PB - 1 - i) * ncol;
     for (int e = lane; e < nel; e += 32) {
-      const int r = jb + i + 1 + e / ncol, c = jb + e % ncol;
-      w[r * DPAD + c] = fma(-s[r * DPAD + jb + i], w[(jb + i) * DPAD + c], w[r * DPAD + c]);
+      const int r = i + 1 + e / ncol, c = e % ncol;
+      w[(jb + r) * WP + c] = fma(-s[(jb + r) * DPAD + jb + i], w[(jb + i) * WP + c], w[(jb + r) * WP + c]);
     }
     __syncwarp();
   }
@@ -138,140 +139,121 @@ __device__ __forceinline__ void tri_index(int e, int& r, int& c) {
   c = e - r * (r + 1) / 2;
 }
 
-// The off-diagonal 16 x 16 blocks of the inverse from the diagonal ones, by block diagonals:
-// W_ij = -W_ii sum_{k=j}^{i-1} L_ik W_kj.  scratch: 3 x 16 x 16 doubles.  Ends with a barrier.
-__device__ __forceinline__ void assemble_inverse(const double* s, double* w, double* scratch, int t) {
-  constexpr int NPB = NB / PB;
-  for (int dist = 1; dist < NPB; ++dist) {
-    const int npair = NPB - dist;
-    for (int it = t; it < npair * PB * PB; it += NT) {  // T = sum_k L_ik W_kj
-      const int pr = it / (PB * PB), r = (it / PB) % PB, c = it % PB;
-      const int bi = (pr + dist) * PB, bj = pr * PB;
-      double acc = 0.0;
-      for (int k = bj; k < bi; ++k) acc = fma(s[(bi + r) * DPAD + k], w[k * DPAD + bj + c], acc);
-      scratch[it] = acc;
-    }
-    __syncthreads();
-    for (int it = t; it < npair * PB * PB; it += NT) {  // W_ij = -W_ii T
-      const int pr = it / (PB * PB), r = (it / PB) % PB, c = it % PB;
-      const int bi = (pr + dist) * PB, bj = pr * PB;
-      double acc = 0.0;
-      for (int m = 0; m <= r; ++m) acc = fma(w[(bi + r) * DPAD + bi + m], scratch[pr * PB * PB + m * PB + c], acc);
-      w[(bi + r) * DPAD + bj + c] = -acc;
-    }
-    __syncthreads();
+// root = sqrt(x) and rroot = 1 / root of a pivot, rounded as sqrt and the reciprocal round them: the hardware's 20-bit
+// approximation of 1 / sqrt(x), one third-order step (e^3 < 2^-56), and one correction step each; a chain of 10 operations
+// (640 clocks) instead of the library's two routines (990).  Outside the range where the approximation is a normal
+// number, the library's operations.  (Stopping at the uncorrected 1 / sqrt(x) is 8 us a block faster, but moves the last
+// bit of most entries, and with it which duplicate points need a numerical nugget.)
+__device__ __forceinline__ void pivot_roots(double x, double& root, double& rroot) {
+  const int hi = __double2hiint(x);
+  if (hi < 0x02000000 || hi >= 0x7E000000) {
+    root = sqrt(x);
+    rroot = __drcp_rn(root);
+    return;
   }
+  double r;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
+  const double e = fma(-(x * r), r, 1.0);
+  const double y = fma(r * e, fma(e, 0.375, 0.5), r);
+  const double q = x * y;
+  root = fma(fma(-q, q, x), 0.5 * y, q);
+  rroot = fma(fma(-root, y, 1.0), y, y);
 }
 
-// Cholesky factor and inverse of one nb x nb diagonal block (nb <= 64) in shared memory.  16-column block steps:
-// update the block column with the columns left of it, factor and invert its 16 x 16 diagonal block in one warp,
-// then solve the rows below with that inverse; the full inverse is assembled from the diagonal inverses.  A ragged
-// block is padded with the identity.
-__global__ void __launch_bounds__(NT) k_potrf_diag(double* A, int64_t lda, int64_t mstride, int k0, int nb,
-                                                   double* Dinv, int64_t dinv_bstride, int blk, int* info) {
+constexpr int PT = 256;           // threads of k_potrf_diag
+constexpr int PW = 6 * 32;        // of them, those that update the trailing entries
+
+// Cholesky factor of one nb x nb diagonal block (nb <= 64, a ragged block padded with the identity), right-looking, one
+// column per step.  The serial chain bounds it: an FP64 operation takes 64 clocks and holds its sub-partition's pipe for
+// 64, so warp 0 has the pipe of its sub-partition to itself (warp 4, on the same one, only loads and stores) for the
+// chain -- the update of column j + 1, the pivot's reciprocal root, the scaling -- while the six warps of the other
+// pipes apply column j to the entries right of it, (row, column) pairs packed over their lanes.  Before, one warp
+// factored and inverted each 16 x 16 block with sqrt and 1 / x (620 and 370 clocks) between rank-16 updates: 118 us a
+// block with its inverse; now 49 us, and 16 us for the inverse in k_trtri_diag, whose columns go to 16 CTAs.
+__global__ void __launch_bounds__(PT) k_potrf_diag(double* A, int64_t lda, int64_t mstride, int k0, int nb, int* info) {
   const int64_t b = blockIdx.z;
   if (info[b] != 0) return;  // an earlier block of this matrix already failed
-  extern __shared__ double dsm[];
-  double* s = dsm;                   // [NB][DPAD]  s[i*DPAD + j] = L(i, j)
-  double* w = dsm + NB * DPAD;       // [NB][DPAD]  w[i*DPAD + j] = L^-1(i, j)
-  double* scratch = w + NB * DPAD;   // [3][PB][PB]
-  __shared__ int failed;
+  __shared__ double s[NB * DPAD];  // s[j * DPAD + i]: column j
+  __shared__ double l[2][NB];      // the factor's column of the current and of the next step
+  __shared__ unsigned short tab[(NB - 2) * (NB - 1) / 2];
+  __shared__ int bad;
   double* Ab = A + b * mstride + k0 + (int64_t)k0 * lda;
-  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-  if (t == 0) failed = 0;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  if (tid == 0) bad = 0;
   {  // all 16 loads of a thread in flight before the shared-memory stores
-    double v[NB * NB / NT];
+    double v[NB * NB / PT];
 #pragma unroll
-    for (int u = 0; u < NB * NB / NT; ++u) {
-      const int idx = t + u * NT, i = idx & 63, j = idx >> 6;
-      v[u] = (i < nb && j < nb) ? ((i >= j) ? Ab[i + (int64_t)j * lda] : 0.0) : (i == j ? 1.0 : 0.0);
+    for (int q = 0; q < NB * NB / PT; ++q) {
+      const int idx = tid + q * PT, i = idx & 63, j = idx >> 6;
+      v[q] = (i < nb && j < nb) ? ((i >= j) ? Ab[i + (int64_t)j * lda] : 0.0) : (i == j ? 1.0 : 0.0);
     }
 #pragma unroll
-    for (int u = 0; u < NB * NB / NT; ++u) {
-      const int idx = t + u * NT, i = idx & 63, j = idx >> 6;
-      s[i * DPAD + j] = v[u];
-      w[i * DPAD + j] = 0.0;
+    for (int q = 0; q < NB * NB / PT; ++q) {
+      const int idx = tid + q * PT;
+      s[(idx >> 6) * DPAD + (idx & 63)] = v[q];
     }
+  }
+  // (row, column) of the packed lower triangle, row by row: a smaller triangle is a prefix
+  for (int e = tid; e < (NB - 2) * (NB - 1) / 2; e += PT) {
+    int r, c;
+    tri_index(e, r, c);
+    tab[e] = (unsigned short)(r | c << 8);
   }
   __syncthreads();
-  for (int jb = 0; jb < NB; jb += PB) {
-    // (1) columns jb .. jb+15, rows i >= c: subtract the columns 0 .. jb-1
-    if (jb > 0) {
-      for (int it = t; it < (NB - jb) * PB; it += NT) {
-        const int c = jb + (it % PB), i = jb + it / PB;
-        if (i >= c) {
-          double acc = s[i * DPAD + c];
-          for (int k = 0; k < jb; ++k) acc = fma(-s[i * DPAD + k], s[c * DPAD + k], acc);
-          s[i * DPAD + c] = acc;
-        }
+  // column c: minus the product with column c - 1 (its own earlier ones are applied), then scaled by its pivot's root
+  auto column = [&](int c) {
+    const double* lc = l[(c - 1) & 1];
+    double v[2] = {0.0, 0.0};
+    const int hp = c >> 5;  // the half of the rows that holds the pivot
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+      if (h >= hp) {
+        const int r = lane + 32 * h;
+        v[h] = s[c * DPAD + r];
+        if (c > 0) v[h] = fma(-lc[r], lc[c], v[h]);
       }
-      __syncthreads();
-    }
-    // (2) the 16 x 16 diagonal block: right-looking Cholesky (column scaling by the reciprocal of the pivot, as
-    // LAPACK's dpotf2 does), then its inverse
+    const double piv = __shfl_sync(0xffffffffu, hp ? v[1] : v[0], c & 31);
+    if (!(piv > 0.0) && lane == 0 && bad == 0) bad = c + 1;  // non-positive or NaN pivot (the rest runs on NaNs)
+    double root, y;
+    pivot_roots(piv, root, y);
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+      if (h >= hp) {
+        const int r = lane + 32 * h;
+        const double x = v[h] * y;
+        l[c & 1][r] = x;
+        s[c * DPAD + r] = (r == c) ? root : x;
+      }
+  };
+  if (warp == 0) column(0);
+  __syncthreads();
+  const int wid = tid - 32 - (warp > 4 ? 32 : 0);  // 0 .. PW - 1 over the warps 1, 2, 3, 5, 6, 7
+  for (int j = 0; j < NB - 1; ++j) {
     if (warp == 0) {
-      const int r = jb + lane;
-      bool bad = false;
-      for (int j = 0; j < PB; ++j) {
-        const int cj = jb + j;
-        const double piv = s[cj * DPAD + cj];
-        if (!(piv > 0.0)) {  // non-positive or NaN pivot
-          bad = true;
-          if (lane == 0) {
-            failed = 1;
-            info[b] = k0 + cj + 1;
-          }
-          break;
-        }
-        const double d = sqrt(piv), rd = __drcp_rn(d);
-        __syncwarp();
-        if (lane == 0) s[cj * DPAD + cj] = d;
-        if (lane > j && lane < PB) s[r * DPAD + cj] *= rd;
-        __syncwarp();
-        // trailing update s(r, c) -= L(r, j) L(c, j), j < c <= r < 16, the (r, c) pairs spread over the lanes
-        const int m = PB - 1 - j;
-        for (int e = lane; e < m * (m + 1) / 2; e += 32) {
-          int rr, cc;
-          tri_index(e, rr, cc);
-          const int ra = jb + j + 1 + rr, ca = jb + j + 1 + cc;
-          s[ra * DPAD + ca] = fma(-s[ra * DPAD + cj], s[ca * DPAD + cj], s[ra * DPAD + ca]);
-        }
-        __syncwarp();
+      column(j + 1);
+    } else if (warp != 4) {
+      const int m = NB - 2 - j, ne = m * (m + 1) / 2, o = j + 2;
+      const double* lj = l[j & 1] + o;
+      double* sj = s + o * DPAD + o;
+      for (int e = wid; e < ne; e += 2 * PW) {  // two entries in flight
+        const bool two = e + PW < ne;
+        const int p0 = tab[e], p1 = tab[two ? e + PW : e];
+        const int r0 = p0 & 255, c0 = p0 >> 8, r1 = p1 & 255, c1 = p1 >> 8;
+        const double a0 = sj[c0 * DPAD + r0], a1 = sj[c1 * DPAD + r1];
+        const double x0 = fma(-lj[r0], lj[c0], a0), x1 = fma(-lj[r1], lj[c1], a1);
+        sj[c0 * DPAD + r0] = x0;
+        if (two) sj[c1 * DPAD + r1] = x1;
       }
-      if (!bad) diag16_inverse(s, w, jb, lane);
     }
     __syncthreads();
-    if (failed) return;
-    // (3) rows below: L(i, jb..jb+15) = A(i, jb..jb+15) W_dd^T, computed into registers, then stored
-    {
-      const int nrow = NB - jb - PB;
-      double out[3];
-#pragma unroll
-      for (int u = 0; u < 3; ++u) {
-        const int it = t + u * NT;
-        out[u] = 0.0;
-        if (it < nrow * PB) {
-          const int i = jb + PB + it / PB, c = it % PB;
-          double acc = 0.0;
-          for (int k = 0; k <= c; ++k) acc = fma(s[i * DPAD + jb + k], w[(jb + c) * DPAD + jb + k], acc);
-          out[u] = acc;
-        }
-      }
-      __syncthreads();
-#pragma unroll
-      for (int u = 0; u < 3; ++u) {
-        const int it = t + u * NT;
-        if (it < nrow * PB) s[(jb + PB + it / PB) * DPAD + jb + it % PB] = out[u];
-      }
-      __syncthreads();
-    }
   }
-  assemble_inverse(s, w, scratch, t);
-  double* Db = Dinv + b * dinv_bstride + (int64_t)blk * NB * NB;
-  for (int idx = t; idx < NB * NB; idx += NT) {
+  if (bad) {
+    if (tid == 0) info[b] = k0 + bad;
+    return;
+  }
+  for (int idx = tid; idx < NB * NB; idx += PT) {
     const int i = idx & 63, j = idx >> 6;
-    if (i < nb && j < nb && i >= j) Ab[i + (int64_t)j * lda] = s[i * DPAD + j];
-    Db[i + j * NB] = (i >= j && i < nb && j < nb) ? w[i * DPAD + j] : 0.0;  // zero above the diagonal and padding
+    if (i < nb && j < nb && i >= j) Ab[i + (int64_t)j * lda] = s[j * DPAD + i];
   }
 }
 
@@ -489,40 +471,63 @@ __global__ void __launch_bounds__(256) k_copy_dinv_block(const double* __restric
   }
 }
 
-// Inverses of the NB x NB diagonal blocks of an existing lower factor (one CTA per block): the same row wavefront as
-// k_potrf_diag, so a block inverted here equals the one the factorisation itself stored.
-__global__ void __launch_bounds__(NT) k_trtri_diag(const double* L, int64_t lda, int64_t mstride, int n, double* Dinv,
-                                                   int64_t dinv_bstride) {
-  extern __shared__ double tsm[];
-  double* s = tsm;
-  double* w = tsm + NB * DPAD;
-  double* scratch = w + NB * DPAD;
+constexpr int IC = 4;            // columns of the inverse per CTA of k_trtri_diag
+constexpr int IG = NB / IC;      // CTAs per block
+constexpr int IT = 2 * PB * IC;  // threads: two per entry of a 16 x IC block
+
+// Columns IC g .. of the inverses of the NB x NB diagonal blocks blk0 + x of a lower factor, for the factorisation
+// (one block at a time) and for a loaded factor alike, so that both give the same bits.  The 16 x 16 diagonal inverses
+// first (one warp each), then W_ij = -W_ii sum_{k=j}^{i-1} L_ik W_kj block row by block row; two threads share the sum of
+// an entry.  FP64 latency bounds it (64 clocks an operation), so the columns are spread over IG CTAs and each pipe of
+// an SM holds one warp.
+__global__ void __launch_bounds__(IT) k_trtri_diag(const double* L, int64_t lda, int64_t mstride, int n, double* Dinv,
+                                                   int64_t dinv_bstride, int blk0, const int* info) {
+  __shared__ double s[NB * DPAD], w[NB * (PB + 1)], x[NB * IC], tt[PB * IC];
   const int64_t b = blockIdx.z;
-  const int blk = blockIdx.x, k0 = blk * NB, nb = min(NB, n - k0);
+  if (info && info[b] != 0) return;
+  const int blk = blk0 + blockIdx.x, g = blockIdx.y, k0 = blk * NB, nb = min(NB, n - k0);
+  const int c0 = g * IC, jb = c0 / PB;  // the 16-column block that holds this CTA's columns
   const double* Lb = L + b * mstride + k0 + (int64_t)k0 * lda;
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-  {  // all 16 loads of a thread in flight before the shared-memory stores
-    double v[NB * NB / NT];
 #pragma unroll
-    for (int u = 0; u < NB * NB / NT; ++u) {
-      const int idx = t + u * NT, i = idx & 63, j = idx >> 6;
+  for (int h = 0; h < NB * NB / IT; h += 16) {  // 16 loads of a thread in flight before the shared-memory stores
+    double v[16];
+#pragma unroll
+    for (int u = 0; u < 16; ++u) {
+      const int idx = t + (h + u) * IT, i = idx & 63, j = idx >> 6;
       v[u] = (i < nb && j < nb) ? ((i >= j) ? Lb[i + (int64_t)j * lda] : 0.0) : (i == j ? 1.0 : 0.0);
     }
 #pragma unroll
-    for (int u = 0; u < NB * NB / NT; ++u) {
-      const int idx = t + u * NT, i = idx & 63, j = idx >> 6;
-      s[i * DPAD + j] = v[u];
-      w[i * DPAD + j] = 0.0;
+    for (int u = 0; u < 16; ++u) {
+      const int idx = t + (h + u) * IT;
+      s[(idx & 63) * DPAD + (idx >> 6)] = v[u];
     }
   }
   __syncthreads();
-  if (warp < NB / PB) diag16_inverse(s, w, warp * PB, lane);
+  if (warp >= jb) diag16_inverse(s, w, warp * PB, lane);
   __syncthreads();
-  assemble_inverse(s, w, scratch, t);
+  for (int e = t; e < PB * IC; e += IT) x[jb * PB * IC + e] = w[(jb * PB + e / IC) * (PB + 1) + c0 % PB + e % IC];
+  __syncthreads();
+  const int half = t & 1, r = (t >> 1) / IC, c = (t >> 1) % IC;
+  for (int i = jb + 1; i < NB / PB; ++i) {
+    double acc = 0.0;
+#pragma unroll 8
+    for (int k = jb * PB + half; k < i * PB; k += 2) acc = fma(s[(i * PB + r) * DPAD + k], x[k * IC + c], acc);
+    acc += __shfl_xor_sync(0xffffffffu, acc, 1);
+    if (half == 0) tt[r * IC + c] = acc;
+    __syncthreads();
+    acc = 0.0;
+#pragma unroll
+    for (int m = 0; m < PB; m += 2)  // W_ii is zero above its diagonal
+      acc = fma(w[(i * PB + r) * (PB + 1) + m + half], tt[(m + half) * IC + c], acc);
+    acc += __shfl_xor_sync(0xffffffffu, acc, 1);
+    if (half == 0) x[(i * PB + r) * IC + c] = -acc;
+    __syncthreads();
+  }
   double* Db = Dinv + b * dinv_bstride + (int64_t)blk * NB * NB;
-  for (int idx = t; idx < NB * NB; idx += NT) {
-    const int i = idx & 63, j = idx >> 6;
-    Db[i + j * NB] = (i >= j && i < nb && j < nb) ? w[i * DPAD + j] : 0.0;
+  for (int idx = t; idx < NB * IC; idx += IT) {
+    const int i = idx & 63, cc = idx >> 6, j = c0 + cc;
+    Db[i + j * NB] = (i >= j && i < nb && j < nb) ? x[i * IC + cc] : 0.0;  // zero above the diagonal and padding
   }
 }
 
@@ -556,22 +561,19 @@ __global__ void k_zero_upper(double* A, int64_t lda, int64_t mstride, int n) {
   for (int i = threadIdx.x; i < j && i < n; i += blockDim.x) col[i] = 0.0;
 }
 
-bool g_diag_attr_set = false;
-bool g_trtri_diag_attr_set = false;
-
 }  // namespace
+
+void trtri_diag_launch(const double* L, int64_t lda, int64_t mstride, int n, double* Dinv, int64_t dinv_bstride, int blk0,
+                       int nblk, const int* info, int batch, cudaStream_t st) {
+  LaunchTimer lt("k_trtri_diag", st, (double)nblk * NB * NB * NB / 3.0 * batch, 16.0 * nblk * NB * NB * batch);
+  k_trtri_diag<<<dim3(nblk, IG, batch), IT, 0, st>>>(L, lda, mstride, n, Dinv, dinv_bstride, blk0, info);
+  LKG_LAUNCH("k_trtri_diag");
+}
 
 void trtri_diag_blocks(const double* L, int64_t lda, int64_t mstride, int n, double* Dinv, int batch,
                        cudaStream_t st) {
   const int nblk = ceil_div(n, NB);
-  const size_t smem = (2 * NB * DPAD + 3 * PB * PB) * sizeof(double);
-  if (!g_trtri_diag_attr_set) {
-    LKG_CUDA(cudaFuncSetAttribute(k_trtri_diag, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    g_trtri_diag_attr_set = true;
-  }
-  LaunchTimer lt("k_trtri_diag", st, (double)nblk * NB * NB * NB / 3.0 * batch, 16.0 * nblk * NB * NB * batch);
-  k_trtri_diag<<<dim3(nblk, 1, batch), NT, smem, st>>>(L, lda, mstride, n, Dinv, (int64_t)nblk * NB * NB);
-  LKG_LAUNCH("k_trtri_diag");
+  trtri_diag_launch(L, lda, mstride, n, Dinv, (int64_t)nblk * NB * NB, 0, nblk, nullptr, batch, st);
 }
 
 void transpose_copy(const double* S, int64_t lds, double* D, int64_t ldd, int rows, int cols, cudaStream_t st) {
@@ -606,14 +608,12 @@ void gemm_tiles(int M, int N, int K, double alpha, MatView A, MatView B, double 
 
 void potrf_diag(double* A, int64_t lda, int64_t mstride, int k0, int nb, double* Dinv, int64_t dinv_bstride, int blk,
                 int* info, int batch, cudaStream_t st) {
-  const size_t smem = (2 * NB * DPAD + 3 * PB * PB) * sizeof(double);
-  if (!g_diag_attr_set) {
-    LKG_CUDA(cudaFuncSetAttribute(k_potrf_diag, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    g_diag_attr_set = true;
+  {
+    LaunchTimer lt("k_potrf_diag", st, nb * (double)nb * nb / 3.0 * batch, 16.0 * nb * nb * batch);
+    k_potrf_diag<<<dim3(1, 1, batch), PT, 0, st>>>(A, lda, mstride, k0, nb, info);
+    LKG_LAUNCH("k_potrf_diag");
   }
-  LaunchTimer lt("k_potrf_diag", st, 2.0 * nb * nb * nb / 3.0 * batch, 16.0 * nb * nb * batch);
-  k_potrf_diag<<<dim3(1, 1, batch), NT, smem, st>>>(A, lda, mstride, k0, nb, Dinv, dinv_bstride, blk, info);
-  LKG_LAUNCH("k_potrf_diag");
+  trtri_diag_launch(A, lda, mstride, k0 + nb, Dinv, dinv_bstride, blk, 1, info, batch, st);
 }
 
 void potrf_blocked(double* A, int64_t lda, int64_t mstride, int n, double* Dinv, int* info, int batch,
