@@ -11,8 +11,18 @@
 // the cells that intersect the cube of half-width sqrt(r2) around p are visited: a few cells per step once the
 // ordering has covered the domain.  The argmax runs on a two-level 64-ary tournament tree in shared memory (level 1
 // holds one (max, index) per 64 grid slots, level 2 one per 64 level-1 nodes) that is updated only where distances
-// changed.  One CTA runs the steps one after another (each needs the previous argmax); a launch runs a bounded
-// number of steps and rebuilds the tree from the distances it left behind.  The cell range of a query is computed
+// changed.  One CTA runs the steps; a launch runs a bounded number of them and rebuilds the tree from the distances it
+// left behind.
+//
+// Steps are taken in rounds.  All points whose distance reaches a threshold tau (the current maximum times a ratio, so
+// that there are at most 1024 of them, one per thread) are the round's candidates.  As long as the largest distance
+// among them reaches tau, it is the global maximum, because no other point does and distances only fall: the candidates
+// alone decide the next steps, with no memory beyond registers and shared memory -- an argmax over the block and the
+// distance of each candidate to the point taken, in FP32 with error bounds, which settles all but the rare candidate
+// that neither surely keeps its distance nor surely falls below tau (that one takes the FP64 distance).  Then all points
+// taken update their neighbourhoods at once, with atomic minima, and the tree follows.  A step alone costs 5.3 us, a chain
+// of dependent loads and FP64 operations; in a round it costs an argmax.  Ties beyond 1024 candidates (or an infinite
+// maximum) fall back to a step alone.  Measured, n = 32768, d = 3: 172.6 ms by single steps, 29.5 ms in rounds.  The cell range of a query is computed
 // with the same monotone floating-point map as the cells of the points, with a 1e-12 relative margin on the radius,
 // so every point that can change lies in a visited cell.
 //
@@ -38,10 +48,13 @@ namespace {
 constexpr unsigned FULL = 0xffffffffu;
 constexpr int MAXD = 8;
 constexpr int G1 = 64;                 // grid slots per level-1 node
-constexpr int NG1_MAX = 16384;         // level-1 nodes in shared memory (n <= 2^20 at G1 = 64; larger n widens G1)
-constexpr int NG2_MAX = 256;           // level-2 nodes (64 level-1 nodes each)
+constexpr int NG1_MAX = 8192;          // level-1 nodes in shared memory (n <= 2^19 at G1 = 64; larger n widens G1)
+constexpr int NG2_MAX = 128;           // level-2 nodes (64 level-1 nodes each)
 constexpr int LIST_MAX = 2048;         // dirty level-1 nodes tracked per step; more -> every node is rebuilt
 constexpr int MM_THREADS = 1024;
+constexpr int CAND_MAX = MM_THREADS;   // candidates of a round, one per thread
+constexpr int ROUND_FROM = 32;         // steps taken one by one before the first round
+constexpr int QUEUE = 64;              // a warp's queue of distances to take in FP64
 constexpr int KNN_BRUTE = 2048;        // positions up to this scan the earlier points directly
 constexpr double RADIUS_MARGIN = 1e-12;
 
@@ -141,13 +154,18 @@ __global__ void k_grid_scatter(int n, const int* __restrict__ cell, int* __restr
 }
 
 // slot arrays of the maxmin grid: coordinates, original index, slot of every point, running distance = +inf
-__global__ void k_grid_slots(int n, int d, const double* __restrict__ Xp, const int* __restrict__ perm,
-                             double* __restrict__ Xs, int* __restrict__ orig, int* __restrict__ slot_of,
-                             double* __restrict__ dist) {
+// (Xf: FP32 differences from the grid's lower corner)
+__global__ void k_grid_slots(int n, int d, const double* __restrict__ Xp, const int* __restrict__ perm, GridDesc g,
+                             double* __restrict__ Xs, float* __restrict__ Xf, int* __restrict__ orig,
+                             int* __restrict__ slot_of, double* __restrict__ dist) {
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= n) return;
   const int i = perm[s];
-  for (int k = 0; k < d; ++k) Xs[(int64_t)s * d + k] = Xp[(int64_t)i * d + k];
+  for (int k = 0; k < d; ++k) {
+    const double x = Xp[(int64_t)i * d + k];
+    Xs[(int64_t)s * d + k] = x;
+    Xf[(int64_t)s * d + k] = (float)(x - g.lo[k]);
+  }
   orig[s] = i;
   slot_of[i] = s;
   dist[s] = INFINITY;
@@ -160,11 +178,31 @@ struct MaxminArgs {
   GridDesc g;
   const int* cell_start;
   const double* Xs;
+  const float* Xf;
   const int* orig;
   const int* slot_of;
-  double* dist;
+  double* dist;  // read past L1 (rounds update it with atomics)
   int* order;
+  float eps[MAXD];  // bound on the error of a difference of two Xf in dimension k
 };
+
+// a float above the non-negative double with these bits (its 24 leading bits, plus one unit), by integer operations
+__device__ __forceinline__ float f32_above(long long bits) {
+  const int hi = (int)(bits >> 32), e = (hi >> 20) & 0x7FF;
+  if (e <= 896) return 1.2e-38f;
+  if (e >= 1150) return INFINITY;
+  return __int_as_float((((e - 896) << 23) | ((hi & 0xFFFFF) << 3) | (int)((unsigned)bits >> 29)) + 1);
+}
+
+// the largest (key, lowest index) of a warp and the lane that holds it; -1 keys mean none (index INT_MAX)
+__device__ __forceinline__ void redux_argmax(long long key, int idx, long long& mkey, int& midx, int& mlane) {
+  const int hi = (int)(key >> 32), mh = __reduce_max_sync(FULL, hi);
+  const unsigned lo = hi == mh ? (unsigned)key : 0u, ml = __reduce_max_sync(FULL, lo);
+  const bool top = hi == mh && (unsigned)key == ml;
+  midx = __reduce_min_sync(FULL, top ? idx : INT_MAX);
+  mlane = __ffs(__ballot_sync(FULL, top && idx == midx)) - 1;
+  mkey = ((long long)mh << 32) | ml;
+}
 
 __global__ void __launch_bounds__(MM_THREADS, 1) k_maxmin_grid(MaxminArgs a) {
   extern __shared__ long long mm_smem[];
@@ -174,12 +212,20 @@ __global__ void __launch_bounds__(MM_THREADS, 1) k_maxmin_grid(MaxminArgs a) {
   int* l2i = reinterpret_cast<int*>(l2v + NG2_MAX);          // 256
   unsigned* dirty1 = reinterpret_cast<unsigned*>(l2i + NG2_MAX);  // ng1 bits
   int* list1 = reinterpret_cast<int*>(dirty1 + NG1_MAX / 32);     // LIST_MAX
+  int* cslot = list1 + LIST_MAX;                                  // CAND_MAX: a candidate's slot
+  int* taken = cslot + CAND_MAX;                                  // CAND_MAX: the candidates taken, in order
+  float* cx = reinterpret_cast<float*>(taken + CAND_MAX);         // d x CAND_MAX
+  int2* queue = reinterpret_cast<int2*>(cx + (size_t)a.d * CAND_MAX);  // QUEUE per warp: (slot, candidate taken)
   __shared__ unsigned dirty2[NG2_MAX / 32];
   __shared__ int nlist1, overflow;
   // the step's scalars, computed by warp 0 and read by every warp: the point taken, its slot and coordinates, and
   // the range of cells that can hold a changing point
   __shared__ int st_snext, st_clo[MAXD], st_chi[MAXD], st_rows;
   __shared__ double st_xn[MAXD];
+  // a round's: threshold, radius, sizes, and the warps' best candidates (two buffers)
+  __shared__ long long rd_max, rd_tau, rd_key[2][32];
+  __shared__ float rd_radius;
+  __shared__ int rd_nodes, rd_cands, rd_taken, rd_idx[2][32], rd_cand[2][32];
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5, nw = MM_THREADS / 32;
   const int d = a.d, n = a.n, gs = a.g1, per = gs / 32;
 
@@ -200,7 +246,7 @@ __global__ void __launch_bounds__(MM_THREADS, 1) k_maxmin_grid(MaxminArgs a) {
     for (int q = 0; q < per; ++q) {
       const int s = gidx * gs + q * 32 + lane;
       if (s < n) {
-        const long long v = key_of(a.dist[s]);
+        const long long v = key_of(__ldcg(a.dist + s));
         const int i = a.orig[s];
         if (beats(v, i, bv, bi)) {
           bv = v;
@@ -243,7 +289,278 @@ __global__ void __launch_bounds__(MM_THREADS, 1) k_maxmin_grid(MaxminArgs a) {
   for (int gidx = w; gidx < a.ng2; gidx += nw) reduce_l2(gidx);
   __syncthreads();
 
-  for (int t = a.t0; t < a.t1; ++t) {
+  // (c), (d): the tree where distances changed (every node after an overflowing list), then the marks are cleared
+  auto refresh_tree = [&]() {
+    const bool full = overflow != 0;
+    const int cnt = full ? a.ng1 : nlist1;
+    for (int q = w; q < cnt; q += nw) {
+      const int gidx = full ? q : list1[q];
+      reduce_l1(gidx);
+      if (lane == 0) atomicOr(&dirty2[(gidx >> 6) >> 5], 1u << ((gidx >> 6) & 31));
+    }
+    __syncthreads();
+    for (int c = w; c < a.ng2; c += nw)
+      if (dirty2[c >> 5] & (1u << (c & 31))) reduce_l2(c);
+    if (full) {
+      for (int q = tid; q < NG1_MAX / 32; q += MM_THREADS) dirty1[q] = 0u;
+    } else {
+      for (int q = tid; q < cnt; q += MM_THREADS) {
+        const int gidx = list1[q];
+        atomicAnd(&dirty1[gidx >> 5], ~(1u << (gidx & 31)));
+      }
+    }
+    __syncthreads();
+    if (tid < NG2_MAX / 32) dirty2[tid] = 0u;
+    if (tid == 0) {
+      nlist1 = 0;
+      overflow = 0;
+    }
+    __syncthreads();
+  };
+
+  double ratio = 0.9;         // uniform over the block, like the next two
+  int singles = ROUND_FROM;   // position up to which steps are taken alone
+  int wait = 512;             // steps alone after ties that no round can hold, doubled each time they come again
+  int t = a.t0;
+  while (t < a.t1) {
+    bool single = t < singles;
+    double now = ratio;
+    while (!single) {  // the round's candidates; a smaller range of distances when there are too many
+      if (w == 0) {
+        long long bv = LLONG_MIN;
+        for (int c = lane; c < a.ng2; c += 32) bv = l2v[c] > bv ? l2v[c] : bv;
+        for (int o = 16; o > 0; o >>= 1) {
+          const long long ov = __shfl_xor_sync(FULL, bv, o);
+          bv = ov > bv ? ov : bv;
+        }
+        if (lane == 0) {
+          const double mx = __longlong_as_double(bv);
+          rd_max = bv;
+          rd_tau = key_of(mx * now);
+          rd_radius = __double2float_ru(sqrt(mx) * (1.0 + 1e-6));
+          rd_nodes = 0;
+          rd_cands = 0;
+        }
+      }
+      __syncthreads();
+      if (rd_max >= key_of(INFINITY)) {
+        single = true;
+        break;
+      }
+      if (rd_max == 0) {  // every point left coincides with one already taken: they follow by ascending index
+        for (int i0 = 0; i0 < n && t < a.t1; i0 += MM_THREADS) {
+          const int i = i0 + tid, s = i < n ? a.slot_of[i] : 0;
+          const bool left = i < n && key_of(__ldcg(a.dist + s)) >= 0;
+          const unsigned mask = __ballot_sync(FULL, left);
+          if (lane == 0) rd_idx[0][w] = __popc(mask);
+          __syncthreads();
+          int before = __popc(mask & ((1u << lane) - 1u)), total = 0;
+          for (int q = 0; q < nw; ++q) {
+            before += q < w ? rd_idx[0][q] : 0;
+            total += rd_idx[0][q];
+          }
+          if (left && t + before < a.t1) {
+            a.order[t + before] = i;
+            __stcg(a.dist + s, -INFINITY);
+          }
+          t = min(t + total, a.t1);
+          __syncthreads();
+        }
+        return;  // the last step of this launch; the next one rebuilds the tree
+      }
+      const long long tau = rd_tau;
+      for (int g = tid; g < a.ng1; g += MM_THREADS)
+        if (l1v[g] >= tau) {
+          const int pos = atomicAdd(&rd_nodes, 1);
+          if (pos < LIST_MAX) list1[pos] = g;
+        }
+      __syncthreads();
+      const int nodes = rd_nodes;
+      if (nodes <= LIST_MAX)
+        for (int q = w; q < nodes; q += nw) {
+          for (int h = 0; h < per; ++h) {
+            const int s = list1[q] * gs + h * 32 + lane;
+            const bool in = s < n && key_of(__ldcg(a.dist + s)) >= tau;
+            const unsigned mask = __ballot_sync(FULL, in);
+            int base = 0;
+            if (lane == 0 && mask) base = atomicAdd(&rd_cands, __popc(mask));
+            base = __shfl_sync(FULL, base, 0);
+            const int pos = base + __popc(mask & ((1u << lane) - 1u));
+            if (in && pos < CAND_MAX) cslot[pos] = s;
+          }
+        }
+      __syncthreads();
+      const int nc = nodes <= LIST_MAX ? rd_cands : CAND_MAX + 1;
+      __syncthreads();
+      if (nc <= CAND_MAX) {
+        ratio = nc < CAND_MAX / 4 ? fmax(0.5, 1.0 - 1.5 * (1.0 - now)) : now;
+        break;
+      }
+      now = 1.0 - (nc < 4 * CAND_MAX ? 0.5 : 0.125) * (1.0 - now);
+      if (now > 1.0 - 1e-9) {  // more than CAND_MAX points share the maximum, or nearly: that may last for a while
+        singles = t + wait;
+        wait *= 2;
+        single = true;
+      }
+    }
+    if (!single) {
+      const int nc = rd_cands, nact = (nc + 31) / 32;
+      if (w < nact) {
+        const long long tau = rd_tau;
+        const float tauf = __double2float_rd(__longlong_as_double(tau));
+        const bool mine = tid < nc;
+        const int slot = mine ? cslot[tid] : 0;
+        long long key = mine ? key_of(__ldcg(a.dist + slot)) : -1;
+        int idx = mine ? a.orig[slot] : INT_MAX;
+        float vhi = mine ? f32_above(key) : 0.0f;
+        for (int k = 0; k < d; ++k) cx[k * CAND_MAX + tid] = mine ? a.Xf[(int64_t)slot * d + k] : 0.0f;
+        int s = 0;
+        for (int buf = 0;; buf ^= 1) {
+          long long mk;
+          int mi, ml;
+          redux_argmax(key, idx, mk, mi, ml);
+          if (lane == ml) {
+            rd_key[buf][w] = mk;
+            rd_idx[buf][w] = mi;
+            rd_cand[buf][w] = tid;
+          }
+          asm volatile("bar.sync 1, %0;" ::"r"(nact * 32) : "memory");
+          const bool ok = lane < nact;
+          redux_argmax(ok ? rd_key[buf][lane] : -1, ok ? rd_idx[buf][lane] : INT_MAX, mk, mi, ml);
+          if (mk < tau) break;  // no candidate reaches the threshold any more
+          const int c = rd_cand[buf][ml];
+          if (tid == 0) {
+            a.order[t + s] = mi;
+            taken[s] = c;
+          }
+          ++s;
+          if (t + s == a.t1) break;
+          if (tid == c) {
+            key = -1;
+            idx = INT_MAX;
+          } else if (key >= 0) {
+            float lb = 0.0f, ub = 0.0f;
+            for (int k = 0; k < d; ++k) {
+              const float dx = fabsf(cx[k * CAND_MAX + tid] - cx[k * CAND_MAX + c]), e = a.eps[k];
+              const float dl = fmaxf(dx - e, 0.0f), du = dx + e;
+              lb = fmaf(dl, dl, lb);
+              ub = fmaf(du, du, ub);
+            }
+            if (!(lb * (1.0f - 0x1p-18f) >= vhi)) {    // it may fall
+              if (ub * (1.0f + 0x1p-18f) < tauf) {     // below the threshold for sure: out of the round
+                key = -1;
+                idx = INT_MAX;
+              } else {
+                const long long dk =
+                    key_of(sqdist(a.Xs + (int64_t)slot * d, a.Xs + (int64_t)cslot[c] * d, d));
+                if (dk < key) {
+                  key = dk;
+                  vhi = f32_above(key);
+                }
+              }
+            }
+          }
+        }
+        if (tid == 0) rd_taken = s;
+      }
+      __syncthreads();
+      const int nt = rd_taken;
+      t += nt;
+      for (int q = tid; q < nt; q += MM_THREADS) {
+        const int s = cslot[taken[q]];
+        __stcg(a.dist + s, -INFINITY);
+        mark_dirty(s / gs);
+      }
+      __syncthreads();
+      // the neighbourhoods of the points taken: one warp per point, its cells' slots spread over the lanes; the FP32
+      // bound clears most of them, the others wait in the warp's queue for 32 FP64 distances at a time
+      {
+        int2* qu = queue + w * QUEUE;
+        int qn = 0;
+        auto drain = [&](int cnt) {
+          __syncwarp();
+          if (lane < cnt) {
+            const int2 e = qu[lane];
+            const long long dk = key_of(sqdist(a.Xs + (int64_t)e.x * d, a.Xs + (int64_t)cslot[e.y] * d, d));
+            if (atomicMin(reinterpret_cast<long long*>(a.dist + e.x), dk) > dk) mark_dirty(e.x / gs);
+          }
+          __syncwarp();
+        };
+        const float rf = rd_radius;
+        for (int q = w; q < nt; q += nw) {
+          const int c = taken[q];
+          // cells within the radius, in FP32 with a margin for its rounding
+          int clo = 0, chi = 0;
+          if (lane < d) {
+            const float x = cx[lane * CAND_MAX + c], ih = (float)a.g.inv_h[lane];
+            const float marg = 1e-3f + (float)a.g.G[lane] * 0x1p-19f;
+            clo = (int)fminf(fmaxf((x - rf) * ih - marg, 0.0f), (float)(a.g.G[lane] - 1));
+            chi = (int)fminf(fmaxf((x + rf) * ih + marg, 0.0f), (float)(a.g.G[lane] - 1));
+          }
+          int rows = 1;
+          for (int k = 1; k < d; ++k)
+            rows *= __shfl_sync(FULL, chi, k) - __shfl_sync(FULL, clo, k) + 1;
+          const int c0 = __shfl_sync(FULL, clo, 0), c1 = __shfl_sync(FULL, chi, 0);
+          for (int r0 = 0; r0 < rows; r0 += 32) {
+            int rem = r0 + lane;
+            long long cb = c0;
+            for (int k = 1; k < d; ++k) {
+              const int lo = __shfl_sync(FULL, clo, k), span = __shfl_sync(FULL, chi, k) - lo + 1;
+              cb += (long long)(lo + rem % span) * a.g.stride[k];
+              rem /= span;
+            }
+            int s0 = 0, len = 0;
+            if (r0 + lane < rows) {
+              s0 = a.cell_start[cb];
+              len = a.cell_start[cb + (c1 - c0) + 1] - s0;
+            }
+            int inc = len;  // slots of this row and the rows before it
+            for (int o = 1; o < 32; o <<= 1) {
+              const int y = __shfl_up_sync(FULL, inc, o);
+              if (lane >= o) inc += y;
+            }
+            const int total = __shfl_sync(FULL, inc, 31);
+            for (int e0 = 0; e0 < total; e0 += 32) {
+              const int e = e0 + lane;
+              int row = 0;  // the row that holds entry e: rows whose running count is at most e lie before it
+              for (int o = 16; o > 0; o >>= 1)
+                if (__shfl_sync(FULL, inc, row + o - 1) <= e) row += o;
+              row = min(row, 31);
+              const int s = __shfl_sync(FULL, s0, row) + e - (__shfl_sync(FULL, inc, row) - __shfl_sync(FULL, len, row));
+              bool hit = false;
+              if (e < total) {
+                const long long dv = key_of(__ldcg(a.dist + s));
+                if (dv >= 0) {
+                  float lb = 0.0f;
+                  for (int k = 0; k < d; ++k) {
+                    const float dl = fmaxf(fabsf(a.Xf[(int64_t)s * d + k] - cx[k * CAND_MAX + c]) - a.eps[k], 0.0f);
+                    lb = fmaf(dl, dl, lb);
+                  }
+                  hit = !(lb * (1.0f - 0x1p-18f) >= f32_above(dv));
+                }
+              }
+              const unsigned mask = __ballot_sync(FULL, hit);
+              if (hit) qu[qn + __popc(mask & ((1u << lane) - 1u))] = make_int2(s, c);
+              qn += __popc(mask);
+              if (qn >= 32) {
+                drain(32);
+                int2 keep = make_int2(0, 0);
+                if (lane < qn - 32) keep = qu[32 + lane];
+                __syncwarp();
+                if (lane < qn - 32) qu[lane] = keep;
+                qn -= 32;
+                __syncwarp();
+              }
+            }
+          }
+        }
+        drain(qn);
+      }
+      __syncthreads();
+      refresh_tree();
+      continue;
+    }
+    // ---- one step alone ----
     // (a) warp 0: the next point (the root of the tree) and the cells that can hold a changing point
     if (w == 0) {
       int next;
@@ -302,7 +619,7 @@ __global__ void __launch_bounds__(MM_THREADS, 1) k_maxmin_grid(MaxminArgs a) {
         const int s0 = a.cell_start[cbase], s1 = a.cell_start[cbase + (st_chi[0] - st_clo[0]) + 1];
         for (int s = s0 + lane; s < s1; s += 32) {
           if (s == snext) continue;
-          const long long dv = key_of(a.dist[s]);
+          const long long dv = key_of(__ldcg(a.dist + s));
           if (dv < 0) continue;  // already ordered (-inf)
           const double d2 = sqdist(a.Xs + (int64_t)s * d, xn, d);
           if (key_of(d2) < dv) {
@@ -313,37 +630,11 @@ __global__ void __launch_bounds__(MM_THREADS, 1) k_maxmin_grid(MaxminArgs a) {
       }
     }
     __syncthreads();
-    // (c) level 1 where distances changed (every node after an overflowing step)
-    const bool full = overflow != 0;
-    const int cnt = full ? a.ng1 : nlist1;
-    for (int q = w; q < cnt; q += nw) {
-      const int gidx = full ? q : list1[q];
-      reduce_l1(gidx);
-      if (lane == 0) atomicOr(&dirty2[(gidx >> 6) >> 5], 1u << ((gidx >> 6) & 31));
-    }
-    __syncthreads();
-    // (d) level 2, then clear the marks
-    for (int c = w; c < a.ng2; c += nw)
-      if (dirty2[c >> 5] & (1u << (c & 31))) reduce_l2(c);
-    if (full) {
-      for (int q = tid; q < NG1_MAX / 32; q += MM_THREADS) dirty1[q] = 0u;
-    } else {
-      for (int q = tid; q < cnt; q += MM_THREADS) {
-        const int gidx = list1[q];
-        atomicAnd(&dirty1[gidx >> 5], ~(1u << (gidx & 31)));
-      }
-    }
-    __syncthreads();
-    if (tid < NG2_MAX / 32) dirty2[tid] = 0u;
-    if (tid == 0) {
-      nlist1 = 0;
-      overflow = 0;
-    }
-    __syncthreads();
+    refresh_tree();
+    ++t;
   }
 }
 
-// ------------------------------------------------------------------------------------------------ neighbour sets
 // sorted per-warp list of the best k (squared distance, index) keys: insert the qualifying lanes' candidates
 __device__ __forceinline__ void knn_offer(double dj, int ij, bool valid, int k, int lane, double* kd, int* ki,
                                           int& cnt, double& thr, int& thri) {
@@ -557,6 +848,7 @@ void vecchia_sets_grid(int n, int d, const double* hX, const double* dX, int fir
       hi[k] = std::max(hi[k], hX[i + (size_t)k * n]);
     }
   DevBuf<double> Xp((size_t)n * d), Xs((size_t)n * d), dist(n);
+  DevBuf<float> Xf((size_t)n * d);
   DevBuf<int> cell(n), perm(n), orig(n), slot_of(n);
   k_points_major<<<ceil_div(n, 256), 256, 0, st>>>(n, d, dX, nullptr, Xp.p, nullptr);
   LKG_LAUNCH("k_points_major");
@@ -567,7 +859,7 @@ void vecchia_sets_grid(int n, int d, const double* hX, const double* dX, int fir
     const long long nc = grid_cells(g);
     DevBuf<int> cstart(nc + 1), cursor(nc);
     grid_sort(n, Xp.p, g, cell.p, cstart.p, cursor.p, perm.p, st);
-    k_grid_slots<<<ceil_div(n, 256), 256, 0, st>>>(n, d, Xp.p, perm.p, Xs.p, orig.p, slot_of.p, dist.p);
+    k_grid_slots<<<ceil_div(n, 256), 256, 0, st>>>(n, d, Xp.p, perm.p, g, Xs.p, Xf.p, orig.p, slot_of.p, dist.p);
     LKG_LAUNCH("k_grid_slots");
     int gs = G1;
     while (ceil_div(n, gs) > NG1_MAX) gs *= 2;
@@ -581,13 +873,17 @@ void vecchia_sets_grid(int n, int d, const double* hX, const double* dX, int fir
     a.g = g;
     a.cell_start = cstart.p;
     a.Xs = Xs.p;
+    a.Xf = Xf.p;
+    // |x - lo| <= ext: two roundings to FP32 and the subtraction's own
+    for (int k = 0; k < d; ++k) a.eps[k] = std::nextafter((float)((hi[k] - lo[k]) * 0x1p-22), INFINITY);
     a.orig = orig.p;
     a.slot_of = slot_of.p;
     a.dist = dist.p;
     a.order = dorder;
     const size_t smem = sizeof(long long) * a.ng1 + sizeof(int) * ((a.ng1 + 1) & ~1) +
                         (sizeof(long long) + sizeof(int)) * NG2_MAX + sizeof(unsigned) * (NG1_MAX / 32) +
-                        sizeof(int) * LIST_MAX;
+                        sizeof(int) * LIST_MAX + (2 * sizeof(int) + d * sizeof(float)) * CAND_MAX +
+                        sizeof(int2) * QUEUE * (MM_THREADS / 32);
     LKG_CUDA(cudaFuncSetAttribute(k_maxmin_grid, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     const int chunk = 65536;  // steps per launch: each launch stays well under a second
     for (int t0 = 0; t0 < n; t0 += chunk) {
