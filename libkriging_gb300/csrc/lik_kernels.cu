@@ -18,6 +18,20 @@ namespace {
 
 constexpr int T = 64;  // tile edge
 
+// CTAs per 64 x 64 tile: a tile's 4096 pairs take one SM 50 (covariance) to 90 us (gradient sums) whatever the size of the
+// matrix, so matrices of few tiles are cut into column slices of 64 / parts, enough to give most SMs of the chip one (more
+// would not pay: a slice of the gradient sums ends with a block reduction of 2 d + 4 values).  It depends on the size
+// alone, so that a matrix gives the same bits alone and in a batch.  Measured, n = 200, d = 3 (10 tiles): covariance
+// 55 -> 20 us, gradient sums 90 -> 33 us.
+int tile_parts(int64_t ntiles) {
+  int parts = 1;
+  while (parts < 16 && ntiles * parts < 128) parts *= 2;
+  return parts;
+}
+// the gradient sums of a single tile stay in one order: fits of a few dozen points without noise end where R is singular to
+// working precision, and their path turns on the sums' last bits
+int adjoint_parts(int64_t ntiles) { return ntiles == 1 ? 1 : tile_parts(ntiles); }
+
 __device__ __forceinline__ void lower_tile_of(int64_t x, int& I, int& J) {
   I = (int)((sqrt(8.0 * (double)x + 1.0) - 1.0) * 0.5);
   while ((int64_t)(I + 1) * (I + 2) / 2 <= x) ++I;
@@ -67,7 +81,7 @@ __global__ void __launch_bounds__(256) k_cov_lower(int n, int d, const double* _
     xr[k] = xi[k][ri];
     ck[k] = cov_scale<K>() / fabs(th[k]);
   }
-  for (int s = 0; s < 16; ++s) {
+  for (int s = blockIdx.y; s < 16; s += gridDim.y) {
     const int cj = (t >> 6) + 4 * s, j = c0 + cj;
     if (j >= n || j > i) continue;
     double v;
@@ -101,7 +115,7 @@ __global__ void __launch_bounds__(256) k_cov_cross(int n_o, int q, int d, const 
   __syncthreads();
   const int ri = t & 63, i = r0 + ri;
   if (i >= n_o) return;
-  for (int s = 0; s < 16; ++s) {
+  for (int s = blockIdx.z; s < 16; s += gridDim.z) {
     const int cj = (t >> 6) + 4 * s, j = c0 + cj;
     if (j >= q) continue;
     double sum = 0.0, prod = 1.0;
@@ -158,7 +172,7 @@ __global__ void __launch_bounds__(256) k_dcov_cross(int n_o, int q, int d, const
   __syncthreads();
   const int ri = t & 63, i = r0 + ri;
   if (i >= n_o) return;
-  for (int s = 0; s < 16; ++s) {
+  for (int s = blockIdx.z; s < 16; s += gridDim.z) {
     const int cj = (t >> 6) + 4 * s, j = c0 + cj;
     if (j >= q) continue;
     double sum = 0.0, prod = 1.0;
@@ -225,7 +239,7 @@ __global__ void __launch_bounds__(256) k_adjoint(int n, int d, const double* __r
     // division; the 1 / theta_k (and 1/3) factor is applied once per accumulator after the pair loop.  The row's
     // coordinates and the scales stay in shared memory (the loop is bound by the FP64 pipe, not by its loads).
     const double x_i = vi[ri];
-    for (int s = 0; s < 16; ++s) {
+    for (int s = blockIdx.y; s < 16; s += gridDim.y) {
       const int cj = (t >> 6) + 4 * s, j = c0 + cj;
       if (j >= n || j > i) continue;
       const double rinv = Rb[i + (int64_t)j * ldr];
@@ -345,7 +359,7 @@ __global__ void __launch_bounds__(256) k_adjoint(int n, int d, const double* __r
     else a = 2 * DM + (t - 2 * d);
     double s = 0.0;
     for (int q = 0; q < 8; ++q) s += red[a][q];
-    partials[(b * ntiles + blockIdx.x) * nacc + t] = s;
+    partials[(b * ntiles * gridDim.y + blockIdx.x * gridDim.y + blockIdx.y) * nacc + t] = s;
   }
 }
 
@@ -479,7 +493,7 @@ __global__ void __launch_bounds__(256) k_loo_gradR(int n, int d, const double* _
   const int ri = t & 63, i = r0 + ri;
   if (i >= n) return;
   const double inv = 1.0 / theta[kdim];
-  for (int s = 0; s < 16; ++s) {
+  for (int s = blockIdx.z; s < 16; s += gridDim.z) {
     const int cj = (t >> 6) + 4 * s, j = c0 + cj;
     if (j >= n) continue;
     double v = 0.0;
@@ -551,7 +565,8 @@ struct LooGradRLaunch {
   static void run(int n, int d, const double* X, const double* theta, double factor, int kdim, double* G,
                   int64_t ldg, cudaStream_t st) {
     LaunchTimer lt("k_loo_gradR", st, (double)n * n, 8.0 * n * n);
-    k_loo_gradR<K, DM><<<dim3(ceil_div(n, T), ceil_div(n, T), 1), 256, 0, st>>>(n, d, X, theta, factor, kdim, G,
+    const int nb = ceil_div(n, T);
+    k_loo_gradR<K, DM><<<dim3(nb, nb, tile_parts((int64_t)nb * nb)), 256, 0, st>>>(n, d, X, theta, factor, kdim, G,
                                                                                            ldg);
     LKG_LAUNCH("k_loo_gradR");
   }
@@ -564,7 +579,7 @@ struct CovLowerLaunch {
     const int nb = ceil_div(n, T);
     const int64_t ntiles = (int64_t)nb * (nb + 1) / 2;
     LaunchTimer lt("k_cov_lower", st, 0.5 * n * (n - 1.0) * batch, 4.0 * n * (n + 1.0) * batch);
-    k_cov_lower<K, DM><<<dim3((unsigned)ntiles, 1, batch), 256, 0, st>>>(n, d, X, xb, theta, factor, diag, A, lda,
+    k_cov_lower<K, DM><<<dim3((unsigned)ntiles, tile_parts(ntiles), batch), 256, 0, st>>>(n, d, X, xb, theta, factor, diag, A, lda,
                                                                          mstride, nvalid);
     LKG_LAUNCH("k_cov_lower");
   }
@@ -575,7 +590,8 @@ struct CovCrossLaunch {
   static void run(int n_o, int q, int d, const double* Xo, const double* Xn, const double* theta, double factor,
                   double* R, bool snap, cudaStream_t st) {
     LaunchTimer lt("k_cov_cross", st, (double)n_o * q, 8.0 * n_o * q);
-    k_cov_cross<K, DM><<<dim3(ceil_div(n_o, T), ceil_div(q, T), 1), 256, 0, st>>>(n_o, q, d, Xo, Xn, theta, factor,
+    const int nx = ceil_div(n_o, T), ny = ceil_div(q, T);
+    k_cov_cross<K, DM><<<dim3(nx, ny, tile_parts((int64_t)nx * ny)), 256, 0, st>>>(n_o, q, d, Xo, Xn, theta, factor,
                                                                                    R, snap);
     LKG_LAUNCH("k_cov_cross");
   }
@@ -586,7 +602,8 @@ struct DCovCrossLaunch {
   static void run(int n_o, int q, int d, const double* Xo, const double* Xn, const double* theta, double factor,
                   double* DR, cudaStream_t st) {
     LaunchTimer lt("k_dcov_cross", st, (double)n_o * q * (1.0 + d), 8.0 * n_o * q * d);
-    k_dcov_cross<K, DM><<<dim3(ceil_div(n_o, T), ceil_div(q, T), 1), 256, 0, st>>>(n_o, q, d, Xo, Xn, theta, factor,
+    const int nx = ceil_div(n_o, T), ny = ceil_div(q, T);
+    k_dcov_cross<K, DM><<<dim3(nx, ny, tile_parts((int64_t)nx * ny)), 256, 0, st>>>(n_o, q, d, Xo, Xn, theta, factor,
                                                                                     DR);
     LKG_LAUNCH("k_dcov_cross");
   }
@@ -598,7 +615,7 @@ struct AdjointLaunch {
                   const double* xv, int64_t xvb, const double* Rinv, int64_t ldr, int64_t rstride, double* partials,
                   int64_t ntiles, int batch, cudaStream_t st) {
     LaunchTimer lt("k_adjoint", st, 0.5 * n * (n - 1.0) * batch, 4.0 * n * (n + 1.0) * batch);
-    k_adjoint<K, DM><<<dim3((unsigned)ntiles, 1, batch), 256, 0, st>>>(n, d, X, xb, theta, factor, xv, xvb, Rinv, ldr,
+    k_adjoint<K, DM><<<dim3((unsigned)ntiles, adjoint_parts(ntiles), batch), 256, 0, st>>>(n, d, X, xb, theta, factor, xv, xvb, Rinv, ldr,
                                                                         rstride, partials, ntiles);
     LKG_LAUNCH("k_adjoint");
   }
@@ -626,8 +643,8 @@ void dcov_cross(int kernel, int n_o, int q, int d, const double* Xo, const doubl
 }
 
 size_t adjoint_partials_size(int n, int d, int batch) {
-  const int nb = ceil_div(n, T);
-  return (size_t)nb * (nb + 1) / 2 * adjoint_nacc(d) * batch;
+  const int64_t nb = ceil_div(n, T), ntiles = nb * (nb + 1) / 2;
+  return (size_t)ntiles * adjoint_parts(ntiles) * adjoint_nacc(d) * batch;
 }
 
 void adjoint_sums(int kernel, int n, int d, const double* X, int64_t x_bstride, const double* theta,
@@ -638,8 +655,9 @@ void adjoint_sums(int kernel, int n, int d, const double* X, int64_t x_bstride, 
   dispatch_kd<AdjointLaunch>(kernel, d, n, d, X, x_bstride, theta, factor, xv, xv_bstride, Rinv, ldr, rstride,
                              partials, ntiles, batch, st);
   const int nacc = adjoint_nacc(d);
-  LaunchTimer lt("k_reduce_partials", st, 0.0, 8.0 * ntiles * nacc * batch);
-  k_reduce_partials<<<dim3(nacc, 1, batch), 1024, 0, st>>>(partials, ntiles, nacc, out);
+  const int64_t np = ntiles * adjoint_parts(ntiles);
+  LaunchTimer lt("k_reduce_partials", st, 0.0, 8.0 * np * nacc * batch);
+  k_reduce_partials<<<dim3(nacc, 1, batch), 1024, 0, st>>>(partials, np, nacc, out);
   LKG_LAUNCH("k_reduce_partials");
 }
 
