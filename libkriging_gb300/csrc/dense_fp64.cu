@@ -456,9 +456,9 @@ void trsv_launch(const double* L, int64_t lda, int64_t mstride, const double* Di
 }
 
 __global__ void __launch_bounds__(256) k_copy_dinv_block(const double* __restrict__ Dinv, int64_t dinv_bstride,
-                                                         int blk, double* W, int64_t ldw, int64_t wstride, int k0,
-                                                         int nb) {
+                                                         double* W, int64_t ldw, int64_t wstride, int n) {
   const int64_t b = blockIdx.z;
+  const int blk = blockIdx.x, k0 = blk * NB, nb = min(NB, n - k0);
   const double* D = Dinv + b * dinv_bstride + (int64_t)blk * NB * NB;
   double* Wb = W + b * wstride + k0 + (int64_t)k0 * ldw;
   double v[NB * NB / 256];
@@ -637,10 +637,15 @@ void potrf_blocked(double* A, int64_t lda, int64_t mstride, int n, double* Dinv,
   }
 }
 
-void copy_dinv_block(const double* Dinv, int64_t dinv_bstride, int blk, double* W, int64_t ldw, int64_t wstride,
-                     int k0, int nb, int batch, cudaStream_t st) {
-  LaunchTimer lt("k_copy_dinv_block", st, 0.0, 16.0 * nb * nb * batch);
-  k_copy_dinv_block<<<dim3(1, 1, batch), 256, 0, st>>>(Dinv, dinv_bstride, blk, W, ldw, wstride, k0, nb);
+void inverse_init(const double* Dinv, int n, double* W, int64_t ldw, int64_t wstride, int batch, cudaStream_t st) {
+  const int nblk = ceil_div(n, NB);
+  if (wstride == ldw * n)
+    LKG_CUDA(cudaMemsetAsync(W, 0, sizeof(double) * (size_t)wstride * batch, st));
+  else
+    for (int b = 0; b < batch; ++b)
+      LKG_CUDA(cudaMemset2DAsync(W + b * wstride, ldw * sizeof(double), 0, n * sizeof(double), n, st));
+  LaunchTimer lt("k_copy_dinv_block", st, 0.0, 16.0 * n * NB * batch);
+  k_copy_dinv_block<<<dim3(nblk, 1, batch), 256, 0, st>>>(Dinv, (int64_t)nblk * NB * NB, W, ldw, wstride, n);
   LKG_LAUNCH("k_copy_dinv_block");
 }
 
@@ -648,11 +653,9 @@ void trtri_blocked(const double* L, int64_t lda, int64_t mstride, int n, const d
                    int64_t wstride, int batch, cudaStream_t st) {
   const int nblk = ceil_div(n, NB);
   const int64_t dstride = (int64_t)nblk * NB * NB;
-  for (int b = 0; b < batch; ++b)
-    LKG_CUDA(cudaMemset2DAsync(W + b * wstride, ldw * sizeof(double), 0, n * sizeof(double), n, st));
+  inverse_init(Dinv, n, W, ldw, wstride, batch, st);
   for (int k = 0; k < nblk; ++k) {
     const int k0 = k * NB, nb = std::min(NB, n - k0);
-    copy_dinv_block(Dinv, dstride, k, W, ldw, wstride, k0, nb, batch, st);
     if (k0 > 0) {
       // W(k0:k0+nb, 0:k0) = -Dinv_k * Acc(k0:k0+nb, 0:k0)   (in place per column tile)
       MatView d{Dinv + (int64_t)k * NB * NB, 1, NB, dstride};

@@ -42,9 +42,9 @@ void trtri_blocked(const double* L, int64_t lda, int64_t mstride, int n, const d
 void wtw_lower(const double* W, int64_t ldw, int64_t wstride, int n, double* C, int64_t ldc, int64_t cstride,
                int batch, cudaStream_t st);
 
-// W(k0:k0+nb, k0:k0+nb) = Dinv block blk (full NB x NB block with its zero upper part).
-void copy_dinv_block(const double* Dinv, int64_t dinv_bstride, int blk, double* W, int64_t ldw, int64_t wstride,
-                     int k0, int nb, int batch, cudaStream_t st);
+// W = 0 with the Dinv blocks (full NB x NB blocks with their zero upper parts) on its diagonal: what the triangular
+// inverses start from (no later step of theirs writes a diagonal block).
+void inverse_init(const double* Dinv, int n, double* W, int64_t ldw, int64_t wstride, int batch, cudaStream_t st);
 
 // Digit-product variants: the O(n^3) products on the bf16 tensor cores by error-free splitting into 7-bit digits
 // (ozaki7.cuh); the diagonal blocks stay FP64.  With 8 digits (56-bit operands, one rounding per 256 columns) they

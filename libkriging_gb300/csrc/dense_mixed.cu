@@ -92,15 +92,14 @@ void potrf_blocked_mixed7(double* A, int64_t lda, int64_t mstride, int n, double
   }
 }
 
-// The 64-wide steps of one 256-row block of the triangular inverse (rows K0 .. K0 + Wd): D^-1 blocks onto the
-// diagonal, W(k0:k0+nb, 0:k0) = -Dinv_k Acc(k0:k0+nb, 0:k0), then the block's rows below accumulate
+// The 64-wide steps of one 256-row block of the triangular inverse (rows K0 .. K0 + Wd, the D^-1 blocks on the diagonal
+// already): W(k0:k0+nb, 0:k0) = -Dinv_k Acc(k0:k0+nb, 0:k0), then the block's rows below accumulate
 // L(k0+nb:, k0:k0+nb) W(k0:k0+nb, 0:k0+nb).
 void trtri_block7(const double* L, int64_t lda, int64_t mstride, int n, int K0, int Wd, const double* Dinv,
                   int64_t dstride, double* W, int64_t ldw, int64_t wstride, int batch, Split7& SA, Split7& SB,
                   cudaStream_t st) {
   for (int k0 = K0; k0 < K0 + Wd; k0 += NB) {
     const int nb = std::min(NB, n - k0), k = k0 / NB;
-    copy_dinv_block(Dinv, dstride, k, W, ldw, wstride, k0, nb, batch, st);
     if (k0 > 0) {  // W(k0:k0+nb, 0:k0) = -Dinv_k Acc(k0:k0+nb, 0:k0): B rows are the columns of Acc
       oz7_split2(nb, nb, Dinv + (int64_t)k * NB * NB, 1, NB, dstride, SA, k0, nb, W + k0, ldw, 1, wstride, SB,
                  batch, st);
@@ -123,8 +122,7 @@ void trtri_blocked_mixed7(const double* L, int64_t lda, int64_t mstride, int n, 
                           int64_t ldw, int64_t wstride, int batch, const MixedWorkspace& ws, cudaStream_t st) {
   const int nblk = ceil_div(n, NB);
   const int64_t dstride = (int64_t)nblk * NB * NB;
-  for (int b = 0; b < batch; ++b)
-    LKG_CUDA(cudaMemset2DAsync(W + b * wstride, ldw * sizeof(double), 0, n * sizeof(double), n, st));
+  inverse_init(Dinv, n, W, ldw, wstride, batch, st);
   const int S = ws.digits_inv;
   Split7 SL = oz7_buffer(ws.panel, ws.panel_exp, S, ws.n, OZ7_KB, OZ7_KB, ws.wide);
   Split7 SR = oz7_buffer(ws.rowblk, ws.rowblk_exp, S, ws.n, OZ7_KB, OZ7_KB, ws.wide);

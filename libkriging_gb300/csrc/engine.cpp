@@ -163,6 +163,9 @@ Engine::~Engine() {
   if (ev_strip_) cudaEventDestroy(ev_strip_);
   if (ev_panel_) cudaEventDestroy(ev_panel_);
   if (side_st_) cudaStreamDestroy(side_st_);
+  if (ev_fork_) cudaEventDestroy(ev_fork_);
+  if (ev_join_) cudaEventDestroy(ev_join_);
+  if (solve_st_) cudaStreamDestroy(solve_st_);
   if (st_) cudaStreamDestroy(st_);
 }
 
@@ -344,10 +347,28 @@ MixedWorkspace Engine::digit_workspace(int batch, bool long_products) {
 void Engine::ensure_grad_buffers() {
   if (dW_) return;
   buffers_changed();
+  if (!solve_st_) {
+    int least = 0, greatest = 0;
+    LKG_CUDA(cudaDeviceGetStreamPriorityRange(&least, &greatest));
+    LKG_CUDA(cudaStreamCreateWithPriority(&solve_st_, cudaStreamNonBlocking, greatest));
+    LKG_CUDA(cudaEventCreateWithFlags(&ev_fork_, cudaEventDisableTiming));
+    LKG_CUDA(cudaEventCreateWithFlags(&ev_join_, cudaEventDisableTiming));
+  }
   dalloc(&dW_, (size_t)mstride_ * cap_);
   dalloc(&dRinv_, (size_t)mstride_ * cap_);
   part_size_ = adjoint_partials_size(n_, d_, cap_);
   dalloc(&dpart_, part_size_);
+}
+
+void Engine::solve_phase(int batch, cudaStream_t st) {
+  const int n = n_, p = p_;
+  trsm_lower_left(dA_, lda_, mstride_, n, dDinv_, dFY_, n, fystride_, p + 1, batch, st);
+  gram_and_logdet(n, p + 1, dFY_, n, fystride_, dA_, lda_, mstride_, dgram_, gram_stride_, batch, st);
+  if (p > 0)
+    gls_solve(p, dgram_, gram_stride_, dbeta_, p, drstar_, p * p, dgls_info_, batch, st);
+  else
+    LKG_CUDA(cudaMemsetAsync(dgls_info_, 0, sizeof(int) * batch, st));
+  residual_sse(n, p, dFY_, n, fystride_, dbeta_, std::max(p, 1), dEstar_, n, dsse_, 1, batch, st);
 }
 
 const double* Engine::factor_inverse() {
@@ -562,12 +583,67 @@ void Engine::evaluate(int batch, const double* thetas, const double* factors, bo
         potrf_blocked(dA_, lda_, mstride_, n, dDinv_, dinfo_, batch, st_);
     }, graphs_ok);
   };
+  // [F y] of every entry's design (outside the sequences: the entries' designs change between evaluations)
+  auto load_fy = [&] {
+    for (int b = 0; b < batch; ++b) {
+      double* fy = dFY_ + (size_t)b * fystride_;
+      const size_t e = entry_design_[b];
+      if (p > 0)
+        LKG_CUDA(cudaMemcpyAsync(fy, dF_ + e * n * p, sizeof(double) * n * p, cudaMemcpyDeviceToDevice, st_));
+      LKG_CUDA(cudaMemcpyAsync(fy + (size_t)n * p, dY_ + e * n, sizeof(double) * n, cudaMemcpyDeviceToDevice, st_));
+    }
+  };
+  // With a gradient, W = L^-1 and the column sums that decide rcond follow the factorisation without a look at the host
+  // (the FP64 path: a failed factor only costs them), and the solves, a chain of short launches (257 for n = 16384), run beside the
+  // inverse on their own stream: 705 -> 579 us for n = 200, 2.75 -> 2.23 ms for 1003, 15.6 -> 13.6 ms for 4096, 64
+  // entries of 2048 75.2 -> 74.1 ms.  Per-stage timing takes the stages one after another instead.
+  const bool early_inverse = with_grad && rcond_check;
+  const bool beside = early_inverse && bench == nullptr;
+  bool solved = false;
+  auto inverse_phase = [&] {
+    ensure_grad_buffers();
+    const std::string key = "inverse:b=" + std::to_string(batch) + ":m=" +
+                            std::to_string(digit ? mw.digits_inv + 100 * mw.wide : 0) + ":t=" +
+                            std::to_string(oz7_tile()) + ":g=" + std::to_string(buf_gen_);
+    if (beside) load_fy();
+    run_phase(key, [&] {
+      if (beside) {
+        LKG_CUDA(cudaEventRecord(ev_fork_, st_));
+        LKG_CUDA(cudaStreamWaitEvent(solve_st_, ev_fork_, 0));
+        solve_phase(batch, solve_st_);
+        LKG_CUDA(cudaMemcpyAsync(dxv_, dEstar_, sizeof(double) * n * batch, cudaMemcpyDeviceToDevice, solve_st_));
+        trsm_lower_left_t(dA_, lda_, mstride_, n, dDinv_, dxv_, n, n, 1, batch, solve_st_);
+        LKG_CUDA(cudaEventRecord(ev_join_, solve_st_));
+      }
+      if (digit)
+        trtri_blocked_mixed(dA_, lda_, mstride_, n, dDinv_, dW_, lda_, mstride_, batch, mw, st_);
+      else
+        trtri_blocked(dA_, lda_, mstride_, n, dDinv_, dW_, lda_, mstride_, batch, st_);
+      lower_colsum_abs(n, dA_, lda_, mstride_, dcol_, batch, st_);
+      lower_colsum_abs(n, dW_, lda_, mstride_, dvec_, batch, st_);
+      if (beside) LKG_CUDA(cudaStreamWaitEvent(st_, ev_join_, 0));
+    }, graphs_ok);
+    w_valid = true;
+    solved = beside;
+  };
   for (int attempt = 0;; ++attempt) {
+    w_valid = solved = false;
     LKG_CUDA(cudaMemcpyAsync(ddiag_, diag.data(), sizeof(double) * batch, cudaMemcpyHostToDevice, st_));
     factor_phase(digit);
-    if (slices_ > 0 && !retreated) {
+    std::vector<double> cl, cw;
+    auto factor_to_host = [&](bool inverse) {
+      if (inverse) {
+        inverse_phase();
+        cl.resize((size_t)n * batch);
+        cw.resize((size_t)n * batch);
+        LKG_CUDA(cudaMemcpyAsync(cl.data(), dcol_, sizeof(double) * n * batch, cudaMemcpyDeviceToHost, st_));
+        LKG_CUDA(cudaMemcpyAsync(cw.data(), dvec_, sizeof(double) * n * batch, cudaMemcpyDeviceToHost, st_));
+      }
       LKG_CUDA(cudaMemcpyAsync(info.data(), dinfo_, sizeof(int) * batch, cudaMemcpyDeviceToHost, st_));
       LKG_CUDA(cudaStreamSynchronize(st_));
+    };
+    if (slices_ > 0 && !retreated) {
+      factor_to_host(false);  // a failed factor is redone: its inverse is not worth starting
       bool any_fail = false;
       for (int b = 0; b < batch; ++b) any_fail = any_fail || (info[b] != 0 && !dead[b]);
       if (any_fail) {  // retreat: redo this factorisation on the FP64 path before the nugget-retry rules apply
@@ -578,45 +654,29 @@ void Engine::evaluate(int batch, const double* thetas, const double* factors, bo
         factor_phase(digit);
       }
     }
-    LKG_CUDA(cudaMemcpyAsync(info.data(), dinfo_, sizeof(int) * batch, cudaMemcpyDeviceToHost, st_));
-    LKG_CUDA(cudaStreamSynchronize(st_));
-    w_valid = false;
-    if (rcond_check) {
-      if (with_grad) {
-        // The gradient needs W = L^-1 anyway: rcond_exact = 1 / (|L|_1 |L^-1|_1) <= the dlacn2 estimate, so
-        // rcond_exact^2 >= min_rcond already decides "no retry"; only entries below it run the estimator.
-        ensure_grad_buffers();
-        if (digit)
-          trtri_blocked_mixed(dA_, lda_, mstride_, n, dDinv_, dW_, lda_, mstride_, batch, mw, st_);
-        else
-          trtri_blocked(dA_, lda_, mstride_, n, dDinv_, dW_, lda_, mstride_, batch, st_);
-        w_valid = true;
-        std::vector<double> cl((size_t)n * batch), cw((size_t)n * batch);
-        lower_colsum_abs(n, dA_, lda_, mstride_, dcol_, batch, st_);
-        LKG_CUDA(cudaMemcpyAsync(cl.data(), dcol_, sizeof(double) * n * batch, cudaMemcpyDeviceToHost, st_));
-        lower_colsum_abs(n, dW_, lda_, mstride_, dvec_, batch, st_);
-        LKG_CUDA(cudaMemcpyAsync(cw.data(), dvec_, sizeof(double) * n * batch, cudaMemcpyDeviceToHost, st_));
-        LKG_CUDA(cudaStreamSynchronize(st_));
-        bool need_est = false;
-        for (int b = 0; b < batch; ++b) {
-          double an = 0.0, wn = 0.0;
-          for (int j = 0; j < nv_entry[b]; ++j) {  // the valid block's columns only
-            an = std::max(an, cl[(size_t)b * n + j]);
-            wn = std::max(wn, cw[(size_t)b * n + j]);
-          }
-          const double rc = (an > 0.0 && wn > 0.0 && std::isfinite(wn)) ? (1.0 / an) / wn : 0.0;
-          rc2[b] = rc * rc;
-          if (info[b] == 0 && !dead[b] && !(rc2[b] >= cfg.min_rcond)) need_est = true;
+    factor_to_host(early_inverse);
+    if (early_inverse) {
+      // The gradient needs W = L^-1 anyway: rcond_exact = 1 / (|L|_1 |L^-1|_1) <= the dlacn2 estimate, so
+      // rcond_exact^2 >= min_rcond already decides "no retry"; only entries below it run the estimator.
+      bool need_est = false;
+      for (int b = 0; b < batch; ++b) {
+        double an = 0.0, wn = 0.0;
+        for (int j = 0; j < nv_entry[b]; ++j) {  // the valid block's columns only
+          an = std::max(an, cl[(size_t)b * n + j]);
+          wn = std::max(wn, cw[(size_t)b * n + j]);
         }
-        if (need_est) {
-          std::vector<double> est;
-          rcond_batch(batch, est, nv_entry);
-          for (int b = 0; b < batch; ++b)
-            if (!(rc2[b] >= cfg.min_rcond)) rc2[b] = est[b];
-        }
-      } else {
-        rcond_batch(batch, rc2, nv_entry);
+        const double rc = (an > 0.0 && wn > 0.0 && std::isfinite(wn)) ? (1.0 / an) / wn : 0.0;
+        rc2[b] = rc * rc;
+        if (info[b] == 0 && !dead[b] && !(rc2[b] >= cfg.min_rcond)) need_est = true;
       }
+      if (need_est) {
+        std::vector<double> est;
+        rcond_batch(batch, est, nv_entry);
+        for (int b = 0; b < batch; ++b)
+          if (!(rc2[b] >= cfg.min_rcond)) rc2[b] = est[b];
+      }
+    } else if (rcond_check) {
+      rcond_batch(batch, rc2, nv_entry);
     }
     bool retry = false;
     for (int b = 0; b < batch; ++b) {
@@ -659,33 +719,33 @@ void Engine::evaluate(int batch, const double* thetas, const double* factors, bo
   // graph after its first run) ----
   if (with_grad) ensure_grad_buffers();
   const std::string post_key = "post:b=" + std::to_string(batch) + ":m=" + std::to_string(digit ? mw.digits_inv + 100 * mw.wide : 0) +
-                               ":gr=" + std::to_string(with_grad) + ":w=" + std::to_string(w_valid) + ":sa=" +
+                               ":gr=" + std::to_string(with_grad) + ":w=" + std::to_string(w_valid) +
+                               std::to_string(solved) + ":sa=" +
                                std::to_string(skip_adjoint_) + ":xe=" + std::to_string(dXb == dXe_) + ":t=" +
                                std::to_string(oz7_tile()) + ":g=" + std::to_string(buf_gen_);
-  // [F y] of every entry's design (outside the sequence: the entries' designs change between evaluations)
-  for (int b = 0; b < batch; ++b) {
-    double* fy = dFY_ + (size_t)b * fystride_;
-    const size_t e = entry_design_[b];
-    if (p > 0)
-      LKG_CUDA(cudaMemcpyAsync(fy, dF_ + e * n * p, sizeof(double) * n * p, cudaMemcpyDeviceToDevice, st_));
-    LKG_CUDA(cudaMemcpyAsync(fy + (size_t)n * p, dY_ + e * n, sizeof(double) * n, cudaMemcpyDeviceToDevice, st_));
-  }
+  if (!solved) load_fy();
   run_phase(post_key, [&] {
-    trsm_lower_left(dA_, lda_, mstride_, n, dDinv_, dFY_, n, fystride_, p + 1, batch, st_);
-    tm.lap("F* = L \\ F, y* = L \\ y");
-    gram_and_logdet(n, p + 1, dFY_, n, fystride_, dA_, lda_, mstride_, dgram_, gram_stride_, batch, st_);
-    if (p > 0) {
-      gls_solve(p, dgram_, gram_stride_, dbeta_, p, drstar_, p * p, dgls_info_, batch, st_);
-    } else {
-      LKG_CUDA(cudaMemsetAsync(dgls_info_, 0, sizeof(int) * batch, st_));
+    if (!solved && bench) {  // stage by stage
+      trsm_lower_left(dA_, lda_, mstride_, n, dDinv_, dFY_, n, fystride_, p + 1, batch, st_);
+      tm.lap("F* = L \\ F, y* = L \\ y");
+      gram_and_logdet(n, p + 1, dFY_, n, fystride_, dA_, lda_, mstride_, dgram_, gram_stride_, batch, st_);
+      if (p > 0) {
+        gls_solve(p, dgram_, gram_stride_, dbeta_, p, drstar_, p * p, dgls_info_, batch, st_);
+      } else {
+        LKG_CUDA(cudaMemsetAsync(dgls_info_, 0, sizeof(int) * batch, st_));
+      }
+      tm.lap("^b = R*^-1 R*'^-1 F*'y*");
+      residual_sse(n, p, dFY_, n, fystride_, dbeta_, std::max(p, 1), dEstar_, n, dsse_, 1, batch, st_);
+      tm.lap("z = L \\ (y - F*b), SSE = z'z");
+    } else if (!solved) {
+      solve_phase(batch, st_);
     }
-    tm.lap("^b = R*^-1 R*'^-1 F*'y*");
-    residual_sse(n, p, dFY_, n, fystride_, dbeta_, std::max(p, 1), dEstar_, n, dsse_, 1, batch, st_);
-    tm.lap("z = L \\ (y - F*b), SSE = z'z");
 
     if (with_grad) {
-      LKG_CUDA(cudaMemcpyAsync(dxv_, dEstar_, sizeof(double) * n * batch, cudaMemcpyDeviceToDevice, st_));
-      trsm_lower_left_t(dA_, lda_, mstride_, n, dDinv_, dxv_, n, n, 1, batch, st_);
+      if (!solved) {
+        LKG_CUDA(cudaMemcpyAsync(dxv_, dEstar_, sizeof(double) * n * batch, cudaMemcpyDeviceToDevice, st_));
+        trsm_lower_left_t(dA_, lda_, mstride_, n, dDinv_, dxv_, n, n, 1, batch, st_);
+      }
       tm.lap("x = tL \\ z");
       if (digit) {
         if (!w_valid) trtri_blocked_mixed(dA_, lda_, mstride_, n, dDinv_, dW_, lda_, mstride_, batch, mw, st_);

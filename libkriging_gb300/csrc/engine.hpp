@@ -143,6 +143,8 @@ class Engine {
 
  private:
   void ensure_grad_buffers();
+  // [F* y*] = L \ [F y], the GLS solve, E* and SSE of all entries, on st
+  void solve_phase(int batch, cudaStream_t st);
   void ensure_loo_buffers(bool with_product);
   // A' = L^-T F* Rstar^-1 (n x p per entry, stride n p) into dloo_at_ for entries [0, batch)
   void build_At(int batch);
@@ -188,6 +190,8 @@ class Engine {
   int wchunk_k_ = 0;  // columns that dwchunk_ holds
   cudaStream_t side_st_ = nullptr;  // look-ahead stream of the mixed Cholesky (single-matrix evaluations)
   cudaEvent_t ev_strip_ = nullptr, ev_panel_ = nullptr;
+  cudaStream_t solve_st_ = nullptr;  // the solves of an evaluation with gradient, beside the inverse
+  cudaEvent_t ev_fork_ = nullptr, ev_join_ = nullptr;
   int64_t lda_, mstride_, dstride_, fystride_;
   cudaStream_t st_ = nullptr;
   double *dX_ = nullptr, *dY_ = nullptr, *dF_ = nullptr;
