@@ -15,14 +15,19 @@
 // left behind.
 //
 // Steps are taken in rounds.  All points whose distance reaches a threshold tau (the current maximum times a ratio, so
-// that there are at most 1024 of them, one per thread) are the round's candidates.  As long as the largest distance
-// among them reaches tau, it is the global maximum, because no other point does and distances only fall: the candidates
-// alone decide the next steps, with no memory beyond registers and shared memory -- an argmax over the block and the
-// distance of each candidate to the point taken, in FP32 with error bounds, which settles all but the rare candidate
-// that neither surely keeps its distance nor surely falls below tau (that one takes the FP64 distance).  Then all points
-// taken update their neighbourhoods at once, with atomic minima, and the tree follows.  A step alone costs 5.3 us, a chain
-// of dependent loads and FP64 operations; in a round it costs an argmax.  Ties beyond 1024 candidates (or an infinite
-// maximum) fall back to a step alone.  Measured, n = 32768, d = 3: 172.6 ms by single steps, 29.5 ms in rounds.  The cell range of a query is computed
+// that there are at most 512 of them) are the round's candidates.  As long as the largest distance among them reaches
+// tau, it is the global maximum, because no other point does and distances only fall: the candidates alone decide the
+// next steps.  They are sorted by (distance, index), and all pairs are compared in FP32 with error bounds: taking one
+// leaves another one alone, or brings it below tau (out of the round), or neither is sure.  One warp then takes the steps
+// 32 candidates at a time from these bits; pairs that are not sure, or that come down to a distance that still reaches
+// tau, go step by step with FP64 distances (146 of 32768 steps).  The other warps meanwhile update the neighbourhoods of
+// the points taken, with atomic minima, and the tree follows.  A step alone costs 5.3 us, a chain of dependent loads and
+// FP64 operations.  More candidates than 512 make the pairs dearer than the rounds they save (an argmax over up to 1024
+// candidates and their distances to the point taken, step after step, cost 0.65 us a step).  Ties beyond 512
+// candidates (or an infinite maximum) fall back to a step alone.  Measured, n = 32768, d = 3: 172.6 ms by single steps,
+// 29.5 ms with an argmax per step, 11.1 ms with the pairs: neighbourhoods 6 ms, then finding the candidates, sorting
+// them, the pairs and the tree about 1 ms each.
+// The cell range of a query is computed
 // with the same monotone floating-point map as the cells of the points, with a 1e-12 relative margin on the radius,
 // so every point that can change lies in a visited cell.
 //
@@ -52,8 +57,9 @@ constexpr int NG1_MAX = 8192;          // level-1 nodes in shared memory (n <= 2
 constexpr int NG2_MAX = 128;           // level-2 nodes (64 level-1 nodes each)
 constexpr int LIST_MAX = 2048;         // dirty level-1 nodes tracked per step; more -> every node is rebuilt
 constexpr int MM_THREADS = 1024;
-constexpr int CAND_MAX = MM_THREADS;   // candidates of a round, one per thread
-constexpr int ROUND_FROM = 32;         // steps taken one by one before the first round
+constexpr int CAND_MAX = 512;          // candidates of a round
+constexpr int CWORDS = CAND_MAX / 32;
+constexpr int ROUND_FROM = 1;           // steps taken one by one before the first round
 constexpr int QUEUE = 64;              // a warp's queue of distances to take in FP64
 constexpr int KNN_BRUTE = 2048;        // positions up to this scan the earlier points directly
 constexpr double RADIUS_MARGIN = 1e-12;
@@ -174,6 +180,7 @@ __global__ void k_grid_slots(int n, int d, const double* __restrict__ Xp, const 
 // ------------------------------------------------------------------------------------------------ maxmin steps
 struct MaxminArgs {
   int n, d, t0, t1, first, g1;  // steps [t0, t1); t0 == 0 takes `first` with an infinite radius
+  int singles;                  // steps below this position are taken one by one
   int ng1, ng2;
   GridDesc g;
   const int* cell_start;
@@ -190,7 +197,7 @@ struct MaxminArgs {
 __device__ __forceinline__ float f32_above(long long bits) {
   const int hi = (int)(bits >> 32), e = (hi >> 20) & 0x7FF;
   if (e <= 896) return 1.2e-38f;
-  if (e >= 1150) return INFINITY;
+  if (e >= 1150) return NAN;  // beyond FP32: no bound (every comparison with it fails)
   return __int_as_float((((e - 896) << 23) | ((hi & 0xFFFFF) << 3) | (int)((unsigned)bits >> 29)) + 1);
 }
 
@@ -204,7 +211,20 @@ __device__ __forceinline__ void redux_argmax(long long key, int idx, long long& 
   mkey = ((long long)mh << 32) | ml;
 }
 
+// coordinates a candidate takes in shared memory: FP32, and FP64 up to d = 4 (for more there is no room)
+__host__ __device__ constexpr int cand_stride(int d) { return d <= 4 ? 4 : 8; }
+__host__ __device__ constexpr int cand_stride64(int d) { return d <= 4 ? 4 : 0; }
+
+size_t maxmin_smem(int ng1, int d) {
+  return sizeof(long long) * ng1 + sizeof(int) * ((ng1 + 1) & ~1) + (sizeof(long long) + sizeof(int)) * NG2_MAX +
+         sizeof(unsigned) * (NG1_MAX / 32) + sizeof(int) * LIST_MAX + sizeof(int2) * QUEUE * (MM_THREADS / 32) +
+         CAND_MAX * (sizeof(uint2) * CWORDS + sizeof(long long) + sizeof(double) * cand_stride64(d) + 3 * sizeof(int) +
+                     (cand_stride(d) + 1) * sizeof(float));
+}
+
+template <int DM>  // d <= DM
 __global__ void __launch_bounds__(MM_THREADS, 1) k_maxmin_grid(MaxminArgs a) {
+  constexpr int DP = cand_stride(DM);
   extern __shared__ long long mm_smem[];
   long long* l1v = mm_smem;                                  // ng1 keys
   int* l1i = reinterpret_cast<int*>(l1v + a.ng1);            // ng1
@@ -212,20 +232,33 @@ __global__ void __launch_bounds__(MM_THREADS, 1) k_maxmin_grid(MaxminArgs a) {
   int* l2i = reinterpret_cast<int*>(l2v + NG2_MAX);          // 256
   unsigned* dirty1 = reinterpret_cast<unsigned*>(l2i + NG2_MAX);  // ng1 bits
   int* list1 = reinterpret_cast<int*>(dirty1 + NG1_MAX / 32);     // LIST_MAX
-  int* cslot = list1 + LIST_MAX;                                  // CAND_MAX: a candidate's slot
-  int* taken = cslot + CAND_MAX;                                  // CAND_MAX: the candidates taken, in order
-  float* cx = reinterpret_cast<float*>(taken + CAND_MAX);         // d x CAND_MAX
-  int2* queue = reinterpret_cast<int2*>(cx + (size_t)a.d * CAND_MAX);  // QUEUE per warp: (slot, candidate taken)
+  int2* queue = reinterpret_cast<int2*>(list1 + LIST_MAX);  // QUEUE per warp: (slot, candidate taken)
+  // a round's candidates (CAND_MAX each) by descending distance: FP64 key and coordinates, FP32 coordinates, conflicts
+  // with the others (.x: a point that may fall when this one is taken, .y: that surely falls below the threshold)
+  long long* skey = reinterpret_cast<long long*>(queue + QUEUE * (MM_THREADS / 32));
+  double* cxd = reinterpret_cast<double*>(skey + CAND_MAX);
+  float* cx = reinterpret_cast<float*>(cxd + cand_stride64(DM) * CAND_MAX);
+  uint2* pairs = reinterpret_cast<uint2*>(cx + DP * CAND_MAX);
+  float* cthr = reinterpret_cast<float*>(pairs + CWORDS * CAND_MAX);
+  int* cslot = reinterpret_cast<int*>(cthr + CAND_MAX);
+  int* cidx = cslot + CAND_MAX;
+  int* taken = cidx + CAND_MAX;  // the candidates taken, in order
+  // as they were found: where the conflicts go once they are sorted
+  long long* ukey = reinterpret_cast<long long*>(pairs);
+  int* uslot = reinterpret_cast<int*>(ukey + CAND_MAX);
+  int* uidx = uslot + CAND_MAX;
+  int* rank = uidx + CAND_MAX;
   __shared__ unsigned dirty2[NG2_MAX / 32];
   __shared__ int nlist1, overflow;
   // the step's scalars, computed by warp 0 and read by every warp: the point taken, its slot and coordinates, and
   // the range of cells that can hold a changing point
   __shared__ int st_snext, st_clo[MAXD], st_chi[MAXD], st_rows;
   __shared__ double st_xn[MAXD];
-  // a round's: threshold, radius, sizes, and the warps' best candidates (two buffers)
-  __shared__ long long rd_max, rd_tau, rd_key[2][32];
+  // a round's: threshold, radius, sizes; number of steps, and whether there will be no more
+  __shared__ long long rd_max, rd_tau;
   __shared__ float rd_radius;
-  __shared__ int rd_nodes, rd_cands, rd_taken, rd_idx[2][32], rd_cand[2][32];
+  __shared__ int rd_nodes, rd_cands, rd_taken, rd_count[32];
+  __shared__ volatile int rd_done;
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5, nw = MM_THREADS / 32;
   const int d = a.d, n = a.n, gs = a.g1, per = gs / 32;
 
@@ -239,30 +272,47 @@ __global__ void __launch_bounds__(MM_THREADS, 1) k_maxmin_grid(MaxminArgs a) {
         overflow = 1;
     }
   };
-  // level-1 node g: argmax of dist over slots [g gs, (g + 1) gs), ties to the lowest original index
-  auto reduce_l1 = [&](int gidx) {
-    long long bv = LLONG_MIN;
-    int bi = 0x7fffffff;
-    for (int q = 0; q < per; ++q) {
-      const int s = gidx * gs + q * 32 + lane;
-      if (s < n) {
-        const long long v = key_of(__ldcg(a.dist + s));
-        const int i = a.orig[s];
-        if (beats(v, i, bv, bi)) {
-          bv = v;
-          bi = i;
-        }
-      }
+  // level-1 nodes: argmax of dist over the slots [g gs, (g + 1) gs), ties to the lowest original index.  A warp takes
+  // four nodes at a time (-1: none), so that their loads are in flight together.
+  auto reduce_l1 = [&](const int (&gi)[4]) {
+    long long bv[4];
+    int bi[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      bv[u] = LLONG_MIN;
+      bi[u] = INT_MAX;
     }
-    warp_argmax(bv, bi);
-    if (lane == 0) {
-      l1v[gidx] = bv;
-      l1i[gidx] = bi;
+    for (int q = 0; q < per; ++q) {
+      long long v[4];
+      int i[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int s = gi[u] * gs + q * 32 + lane;
+        const bool in = gi[u] >= 0 && s < n;
+        v[u] = in ? key_of(__ldcg(a.dist + s)) : LLONG_MIN;
+        i[u] = in ? a.orig[s] : INT_MAX;
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (beats(v[u], i[u], bv[u], bi[u])) {
+          bv[u] = v[u];
+          bi[u] = i[u];
+        }
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      long long mv;
+      int mi, ml;
+      redux_argmax(bv[u], bi[u], mv, mi, ml);
+      if (lane == 0 && gi[u] >= 0) {
+        l1v[gi[u]] = mv;
+        l1i[gi[u]] = mi;
+      }
     }
   };
   auto reduce_l2 = [&](int gidx) {
     long long bv = LLONG_MIN;
-    int bi = 0x7fffffff;
+    int bi = INT_MAX;
     for (int q = 0; q < 2; ++q) {
       const int c = gidx * 64 + q * 32 + lane;
       if (c < a.ng1 && beats(l1v[c], l1i[c], bv, bi)) {
@@ -270,7 +320,8 @@ __global__ void __launch_bounds__(MM_THREADS, 1) k_maxmin_grid(MaxminArgs a) {
         bi = l1i[c];
       }
     }
-    warp_argmax(bv, bi);
+    int ml;
+    redux_argmax(bv, bi, bv, bi, ml);
     if (lane == 0) {
       l2v[gidx] = bv;
       l2i[gidx] = bi;
@@ -278,7 +329,12 @@ __global__ void __launch_bounds__(MM_THREADS, 1) k_maxmin_grid(MaxminArgs a) {
   };
 
   // rebuild the tree from the distances of the previous launch
-  for (int gidx = w; gidx < a.ng1; gidx += nw) reduce_l1(gidx);
+  for (int g0 = w; g0 < a.ng1; g0 += 4 * nw) {
+    int gi[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) gi[u] = g0 + u * nw < a.ng1 ? g0 + u * nw : -1;
+    reduce_l1(gi);
+  }
   for (int q = tid; q < NG1_MAX / 32; q += MM_THREADS) dirty1[q] = 0u;
   if (tid < NG2_MAX / 32) dirty2[tid] = 0u;
   if (tid == 0) {
@@ -293,10 +349,15 @@ __global__ void __launch_bounds__(MM_THREADS, 1) k_maxmin_grid(MaxminArgs a) {
   auto refresh_tree = [&]() {
     const bool full = overflow != 0;
     const int cnt = full ? a.ng1 : nlist1;
-    for (int q = w; q < cnt; q += nw) {
-      const int gidx = full ? q : list1[q];
-      reduce_l1(gidx);
-      if (lane == 0) atomicOr(&dirty2[(gidx >> 6) >> 5], 1u << ((gidx >> 6) & 31));
+    for (int q0 = w; q0 < cnt; q0 += 4 * nw) {
+      int gi[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int q = q0 + u * nw;
+        gi[u] = q < cnt ? (full ? q : list1[q]) : -1;
+        if (lane == 0 && q < cnt) atomicOr(&dirty2[(gi[u] >> 6) >> 5], 1u << ((gi[u] >> 6) & 31));
+      }
+      reduce_l1(gi);
     }
     __syncthreads();
     for (int c = w; c < a.ng2; c += nw)
@@ -319,7 +380,7 @@ __global__ void __launch_bounds__(MM_THREADS, 1) k_maxmin_grid(MaxminArgs a) {
   };
 
   double ratio = 0.9;         // uniform over the block, like the next two
-  int singles = ROUND_FROM;   // position up to which steps are taken alone
+  int singles = a.singles;    // position up to which steps are taken alone
   int wait = 512;             // steps alone after ties that no round can hold, doubled each time they come again
   int t = a.t0;
   while (t < a.t1) {
@@ -340,6 +401,7 @@ __global__ void __launch_bounds__(MM_THREADS, 1) k_maxmin_grid(MaxminArgs a) {
           rd_radius = __double2float_ru(sqrt(mx) * (1.0 + 1e-6));
           rd_nodes = 0;
           rd_cands = 0;
+          rd_done = 0;
         }
       }
       __syncthreads();
@@ -352,12 +414,12 @@ __global__ void __launch_bounds__(MM_THREADS, 1) k_maxmin_grid(MaxminArgs a) {
           const int i = i0 + tid, s = i < n ? a.slot_of[i] : 0;
           const bool left = i < n && key_of(__ldcg(a.dist + s)) >= 0;
           const unsigned mask = __ballot_sync(FULL, left);
-          if (lane == 0) rd_idx[0][w] = __popc(mask);
+          if (lane == 0) rd_count[w] = __popc(mask);
           __syncthreads();
           int before = __popc(mask & ((1u << lane) - 1u)), total = 0;
           for (int q = 0; q < nw; ++q) {
-            before += q < w ? rd_idx[0][q] : 0;
-            total += rd_idx[0][q];
+            before += q < w ? rd_count[q] : 0;
+            total += rd_count[q];
           }
           if (left && t + before < a.t1) {
             a.order[t + before] = i;
@@ -377,23 +439,35 @@ __global__ void __launch_bounds__(MM_THREADS, 1) k_maxmin_grid(MaxminArgs a) {
       __syncthreads();
       const int nodes = rd_nodes;
       if (nodes <= LIST_MAX)
-        for (int q = w; q < nodes; q += nw) {
+        for (int q0 = w; q0 < nodes; q0 += 4 * nw)
           for (int h = 0; h < per; ++h) {
-            const int s = list1[q] * gs + h * 32 + lane;
-            const bool in = s < n && key_of(__ldcg(a.dist + s)) >= tau;
-            const unsigned mask = __ballot_sync(FULL, in);
-            int base = 0;
-            if (lane == 0 && mask) base = atomicAdd(&rd_cands, __popc(mask));
-            base = __shfl_sync(FULL, base, 0);
-            const int pos = base + __popc(mask & ((1u << lane) - 1u));
-            if (in && pos < CAND_MAX) cslot[pos] = s;
+            int s[4];
+            long long v[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {  // four nodes' loads in flight
+              const int q = q0 + u * nw;
+              s[u] = q < nodes ? list1[q] * gs + h * 32 + lane : n;
+              v[u] = s[u] < n ? key_of(__ldcg(a.dist + s[u])) : -1;
+            }
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+              const unsigned mask = __ballot_sync(FULL, v[u] >= tau);
+              int base = 0;
+              if (lane == 0 && mask) base = atomicAdd(&rd_cands, __popc(mask));
+              base = __shfl_sync(FULL, base, 0);
+              const int pos = base + __popc(mask & ((1u << lane) - 1u));
+              if (v[u] >= tau && pos < CAND_MAX) {
+                uslot[pos] = s[u];
+                ukey[pos] = v[u];
+              }
+            }
           }
-        }
       __syncthreads();
       const int nc = nodes <= LIST_MAX ? rd_cands : CAND_MAX + 1;
       __syncthreads();
       if (nc <= CAND_MAX) {
-        ratio = nc < CAND_MAX / 4 ? fmax(0.5, 1.0 - 1.5 * (1.0 - now)) : now;
+        // the next round's range of distances: about 3/4 of the candidates there is room for
+        ratio = fmax(0.5, 1.0 - (1.0 - now) * fmin(1.5, 0.75 * CAND_MAX / nc));
         break;
       }
       now = 1.0 - (nc < 4 * CAND_MAX ? 0.5 : 0.125) * (1.0 - now);
@@ -404,77 +478,184 @@ __global__ void __launch_bounds__(MM_THREADS, 1) k_maxmin_grid(MaxminArgs a) {
       }
     }
     if (!single) {
-      const int nc = rd_cands, nact = (nc + 31) / 32;
-      if (w < nact) {
-        const long long tau = rd_tau;
-        const float tauf = __double2float_rd(__longlong_as_double(tau));
-        const bool mine = tid < nc;
-        const int slot = mine ? cslot[tid] : 0;
-        long long key = mine ? key_of(__ldcg(a.dist + slot)) : -1;
-        int idx = mine ? a.orig[slot] : INT_MAX;
-        float vhi = mine ? f32_above(key) : 0.0f;
-        for (int k = 0; k < d; ++k) cx[k * CAND_MAX + tid] = mine ? a.Xf[(int64_t)slot * d + k] : 0.0f;
-        int s = 0;
-        for (int buf = 0;; buf ^= 1) {
-          long long mk;
-          int mi, ml;
-          redux_argmax(key, idx, mk, mi, ml);
-          if (lane == ml) {
-            rd_key[buf][w] = mk;
-            rd_idx[buf][w] = mi;
-            rd_cand[buf][w] = tid;
+      const int nc = rd_cands;
+      const long long tau = rd_tau;
+      // by descending distance, ties by ascending index: a candidate's rank is the number of those that beat it
+      if (tid < nc) {
+        uidx[tid] = a.orig[uslot[tid]];
+        rank[tid] = 0;
+        taken[tid] = -1;
+      }
+      __syncthreads();
+      {
+        constexpr int PARTS = MM_THREADS / CAND_MAX;
+        const int i = tid % CAND_MAX;
+        if (i < nc) {
+          const long long key = ukey[i];
+          const int idx = uidx[i];
+          int r = 0;
+          for (int j = tid / CAND_MAX; j < nc; j += PARTS) r += beats(ukey[j], uidx[j], key, idx);
+          atomicAdd(&rank[i], r);
+        }
+      }
+      __syncthreads();
+      // FP32 bounds: with E the length of the error bounds of the differences and d2 the FP32 squared distance, the true
+      // one is at least (sqrt(d2) - E)^2 and at most (sqrt(d2) + E)^2, up to 2^-19 for the rounding of at most 8 terms
+      // and of the square roots
+      float E = 0.0f;
+#pragma unroll
+      for (int k = 0; k < DM; ++k) E = k < d ? fmaf(a.eps[k], a.eps[k], E) : E;
+      E = sqrtf(E) * (1.0f + 0x1p-20f);
+      if (tid < nc) {
+        const int r = rank[tid], s = uslot[tid];
+        skey[r] = ukey[tid];
+        cslot[r] = s;
+        cidx[r] = uidx[tid];
+#pragma unroll
+        for (int k = 0; k < DM; ++k) {
+          cx[r * DP + k] = k < d ? a.Xf[(int64_t)s * d + k] : 0.0f;
+          if (DM <= 4 && k < d) cxd[r * 4 + k] = a.Xs[(int64_t)s * d + k];
+        }
+        const float v = sqrtf(f32_above(ukey[tid])) + E;
+        cthr[r] = v * v * (1.0f + 0x1p-17f);  // d2 at least this: it keeps its distance
+      }
+      __syncthreads();
+      // (a) every pair: lane j of a warp against all rows
+      {
+        const float tauf = __double2float_rd(__longlong_as_double(tau)), vd = fmaxf(sqrtf(tauf) - E, 0.0f);
+        const float thr_gone = tauf > 1e-30f ? vd * vd * (1.0f - 0x1p-17f) : 0.0f;  // d2 below this: it falls below tau
+        const int word = w % CWORDS, j = word * 32 + lane;
+        if (word * 32 < nc) {
+          float xj[DM];
+#pragma unroll
+          for (int k = 0; k < DM; ++k) xj[k] = cx[j * DP + k];
+          const float thr = cthr[j];
+#pragma unroll 4
+          for (int i = w / CWORDS; i < nc; i += nw / CWORDS) {
+            float d2 = 0.0f;
+#pragma unroll
+            for (int k = 0; k < DM; ++k) {
+              const float dx = xj[k] - cx[i * DP + k];
+              d2 = fmaf(dx, dx, d2);
+            }
+            const unsigned may = __ballot_sync(FULL, !(d2 >= thr)), gone = __ballot_sync(FULL, d2 < thr_gone);
+            if (lane == 0) pairs[i * CWORDS + word] = make_uint2(may, gone);
           }
-          asm volatile("bar.sync 1, %0;" ::"r"(nact * 32) : "memory");
-          const bool ok = lane < nact;
-          redux_argmax(ok ? rd_key[buf][lane] : -1, ok ? rd_idx[buf][lane] : INT_MAX, mk, mi, ml);
-          if (mk < tau) break;  // no candidate reaches the threshold any more
-          const int c = rd_cand[buf][ml];
-          if (tid == 0) {
-            a.order[t + s] = mi;
-            taken[s] = c;
+        }
+      }
+      __syncthreads();
+      if (w == 0) {
+        // (b) the steps.  Lane l holds the candidates 32 l .. 32 l + 31: those still in place (alive), and those that came
+        // down but not below tau (late).
+        unsigned alive = lane < CWORDS ? (nc >= lane * 32 + 32 ? FULL : nc > lane * 32 ? (1u << (nc - lane * 32)) - 1u : 0u) : 0u;
+        unsigned late = 0u;
+        long long lkey = -1;
+        int lidx = INT_MAX, lcand = -1, s = 0, hold = 0;
+        for (;;) {
+          const unsigned m = __ballot_sync(FULL, alive != 0u);
+          // 32 candidates at once, as long as every conflict of theirs puts a point out of the round (most do): a
+          // candidate is taken when no earlier one that it conflicts with is
+          if (m && lkey < 0 && --hold < 0) {
+            const int l0 = __ffs(m) - 1;
+            const unsigned A = __shfl_sync(FULL, alive, l0);
+            unsigned may = 0u, gone = 0u;  // bit j: candidate j of the 32 takes this lane's away (surely)
+#pragma unroll 8
+            for (int j = 0; j < 32; ++j) {
+              const uint2 pr = pairs[(l0 * 32 + j) * CWORDS + l0];
+              may |= ((pr.x >> lane) & 1u) << j;
+              gone |= ((pr.y >> lane) & 1u) << j;
+            }
+            const bool in = (A >> lane) & 1u;
+            may &= in ? A & ((1u << lane) - 1u) : 0u;
+            if (!__any_sync(FULL, (may & ~gone) != 0u)) {
+              unsigned T = 0u;
+              for (unsigned U = A; U;) {  // the first of U is decided every time
+                const bool open = (U >> lane) & 1u, out = open && (may & T);
+                const unsigned tk = __ballot_sync(FULL, open && !out && !(may & U));
+                U &= ~(tk | __ballot_sync(FULL, out));
+                T |= tk;
+              }
+              unsigned go = 0u, stay = 0u;  // what they do to the other candidates
+#pragma unroll 8
+              for (int j = 0; j < 32; ++j)
+                if (((T >> j) & 1u) && lane < CWORDS) {
+                  const uint2 pr = pairs[(l0 * 32 + j) * CWORDS + lane];
+                  go |= pr.y;
+                  stay |= pr.x & ~pr.y;
+                }
+              const unsigned others = lane == l0 ? 0u : alive;
+              if (!__any_sync(FULL, (stay & others) != 0u)) {
+                alive = others & ~go;
+                const int pos = s + __popc(T & ((1u << lane) - 1u));
+                if (((T >> lane) & 1u) && t + pos < a.t1) *(volatile int*)(taken + pos) = l0 * 32 + lane;
+                s += __popc(T);
+                if (t + s >= a.t1) {
+                  s = a.t1 - t;
+                  break;
+                }
+                continue;
+              }
+            }
+            hold = 8;
           }
+          // one step: the first candidate in place or the best of the late ones
+          int c = lcand;
+          if (m) {
+            const int l0 = __ffs(m) - 1;
+            const int h = l0 * 32 + __ffs(__shfl_sync(FULL, alive, l0)) - 1;
+            if (lkey < 0 || beats(skey[h], cidx[h], lkey, lidx)) c = h;
+          } else if (lkey < 0) {
+            break;  // no candidate reaches the threshold any more
+          }
+          if (lane == 0) *(volatile int*)(taken + s) = c;
           ++s;
           if (t + s == a.t1) break;
-          if (tid == c) {
-            key = -1;
-            idx = INT_MAX;
-          } else if (key >= 0) {
-            float lb = 0.0f, ub = 0.0f;
-            for (int k = 0; k < d; ++k) {
-              const float dx = fabsf(cx[k * CAND_MAX + tid] - cx[k * CAND_MAX + c]), e = a.eps[k];
-              const float dl = fmaxf(dx - e, 0.0f), du = dx + e;
-              lb = fmaf(dl, dl, lb);
-              ub = fmaf(du, du, ub);
-            }
-            if (!(lb * (1.0f - 0x1p-18f) >= vhi)) {    // it may fall
-              if (ub * (1.0f + 0x1p-18f) < tauf) {     // below the threshold for sure: out of the round
-                key = -1;
-                idx = INT_MAX;
-              } else {
-                const long long dk =
-                    key_of(sqdist(a.Xs + (int64_t)slot * d, a.Xs + (int64_t)cslot[c] * d, d));
-                if (dk < key) {
-                  key = dk;
-                  vhi = f32_above(key);
+          const uint2 pr = lane < CWORDS ? pairs[c * CWORDS + lane] : make_uint2(0u, 0u);
+          const unsigned self = lane == (c >> 5) ? 1u << (c & 31) : 0u;
+          const unsigned hit = pr.x & (alive | late) & ~self, gone = hit & pr.y;
+          unsigned open = hit & ~gone;
+          const bool look = open != 0u || (late & (gone | self)) != 0u;
+          alive &= ~(gone | self);
+          late &= ~(gone | self);
+          if (__any_sync(FULL, look)) {
+            for (; open; open &= open - 1u) {
+              const unsigned bit = open & (0u - open);
+              const int j = lane * 32 + __ffs(open) - 1;
+              const long long dk = key_of(DM <= 4 ? sqdist(cxd + j * 4, cxd + c * 4, d)
+                                                  : sqdist(a.Xs + (int64_t)cslot[j] * d, a.Xs + (int64_t)cslot[c] * d, d));
+              if (dk < skey[j]) {
+                alive &= ~bit;
+                late &= ~bit;
+                if (dk >= tau) {
+                  late |= bit;
+                  skey[j] = dk;
                 }
               }
             }
+            long long bk = -1;
+            int bi = INT_MAX, bc = -1, ml;
+            for (unsigned u = late; u; u &= u - 1u) {
+              const int j = lane * 32 + __ffs(u) - 1;
+              if (beats(skey[j], cidx[j], bk, bi)) {
+                bk = skey[j];
+                bi = cidx[j];
+                bc = j;
+              }
+            }
+            redux_argmax(bk, bi, lkey, lidx, ml);
+            lcand = __shfl_sync(FULL, bc, ml);
+            __syncwarp();
           }
         }
-        if (tid == 0) rd_taken = s;
-      }
-      __syncthreads();
-      const int nt = rd_taken;
-      t += nt;
-      for (int q = tid; q < nt; q += MM_THREADS) {
-        const int s = cslot[taken[q]];
-        __stcg(a.dist + s, -INFINITY);
-        mark_dirty(s / gs);
-      }
-      __syncthreads();
-      // the neighbourhoods of the points taken: one warp per point, its cells' slots spread over the lanes; the FP32
-      // bound clears most of them, the others wait in the warp's queue for 32 FP64 distances at a time
-      {
+        if (lane == 0) {
+          rd_taken = s;
+          __threadfence_block();
+          rd_done = 1;
+        }
+      } else {
+        // (c) meanwhile the other warps: the neighbourhoods of the points taken, one warp per point, its cells' slots
+        // spread over the lanes; the FP32 bound clears most of them, the others wait in the warp's queue for 32 FP64
+        // distances at a time
         int2* qu = queue + w * QUEUE;
         int qn = 0;
         auto drain = [&](int cnt) {
@@ -487,12 +668,32 @@ __global__ void __launch_bounds__(MM_THREADS, 1) k_maxmin_grid(MaxminArgs a) {
           __syncwarp();
         };
         const float rf = rd_radius;
-        for (int q = w; q < nt; q += nw) {
-          const int c = taken[q];
+        // with few candidates several warps share a point's rows of cells
+        const int share = min(32, max(1, 512 / nc));
+        for (int unit = w - 1; unit < nc * share; unit += nw - 1) {
+          const int q = unit / share, part = unit % share;
+          int c = -1;
+          for (;;) {  // until step q is there, or will not come: warp 0 ends after at most nc steps
+            if (lane == 0) {
+              const int done = rd_done;
+              __threadfence_block();
+              c = *(volatile int*)(taken + q);
+              if (c < 0 && done) c = -2;
+            }
+            c = __shfl_sync(FULL, c, 0);
+            if (c != -1) break;
+            __nanosleep(100);
+          }
+          if (c < 0) break;
+          if (lane == 0 && part == 0) {
+            a.order[t + q] = cidx[c];
+            __stcg(a.dist + cslot[c], -INFINITY);
+            mark_dirty(cslot[c] / gs);
+          }
           // cells within the radius, in FP32 with a margin for its rounding
           int clo = 0, chi = 0;
           if (lane < d) {
-            const float x = cx[lane * CAND_MAX + c], ih = (float)a.g.inv_h[lane];
+            const float x = cx[c * DP + lane], ih = (float)a.g.inv_h[lane];
             const float marg = 1e-3f + (float)a.g.G[lane] * 0x1p-19f;
             clo = (int)fminf(fmaxf((x - rf) * ih - marg, 0.0f), (float)(a.g.G[lane] - 1));
             chi = (int)fminf(fmaxf((x + rf) * ih + marg, 0.0f), (float)(a.g.G[lane] - 1));
@@ -501,7 +702,7 @@ __global__ void __launch_bounds__(MM_THREADS, 1) k_maxmin_grid(MaxminArgs a) {
           for (int k = 1; k < d; ++k)
             rows *= __shfl_sync(FULL, chi, k) - __shfl_sync(FULL, clo, k) + 1;
           const int c0 = __shfl_sync(FULL, clo, 0), c1 = __shfl_sync(FULL, chi, 0);
-          for (int r0 = 0; r0 < rows; r0 += 32) {
+          for (int r0 = part * 32; r0 < rows; r0 += 32 * share) {
             int rem = r0 + lane;
             long long cb = c0;
             for (int k = 1; k < d; ++k) {
@@ -532,10 +733,12 @@ __global__ void __launch_bounds__(MM_THREADS, 1) k_maxmin_grid(MaxminArgs a) {
                 const long long dv = key_of(__ldcg(a.dist + s));
                 if (dv >= 0) {
                   float lb = 0.0f;
-                  for (int k = 0; k < d; ++k) {
-                    const float dl = fmaxf(fabsf(a.Xf[(int64_t)s * d + k] - cx[k * CAND_MAX + c]) - a.eps[k], 0.0f);
-                    lb = fmaf(dl, dl, lb);
-                  }
+#pragma unroll
+                  for (int k = 0; k < DM; ++k)
+                    if (k < d) {
+                      const float dl = fmaxf(fabsf(a.Xf[(int64_t)s * d + k] - cx[c * DP + k]) - a.eps[k], 0.0f);
+                      lb = fmaf(dl, dl, lb);
+                    }
                   hit = !(lb * (1.0f - 0x1p-18f) >= f32_above(dv));
                 }
               }
@@ -557,6 +760,7 @@ __global__ void __launch_bounds__(MM_THREADS, 1) k_maxmin_grid(MaxminArgs a) {
         drain(qn);
       }
       __syncthreads();
+      t += rd_taken;
       refresh_tree();
       continue;
     }
@@ -880,17 +1084,19 @@ void vecchia_sets_grid(int n, int d, const double* hX, const double* dX, int fir
     a.slot_of = slot_of.p;
     a.dist = dist.p;
     a.order = dorder;
-    const size_t smem = sizeof(long long) * a.ng1 + sizeof(int) * ((a.ng1 + 1) & ~1) +
-                        (sizeof(long long) + sizeof(int)) * NG2_MAX + sizeof(unsigned) * (NG1_MAX / 32) +
-                        sizeof(int) * LIST_MAX + (2 * sizeof(int) + d * sizeof(float)) * CAND_MAX +
-                        sizeof(int2) * QUEUE * (MM_THREADS / 32);
-    LKG_CUDA(cudaFuncSetAttribute(k_maxmin_grid, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    // FP32 squares of differences between 1e-18 and 1e18 stay in range; other boxes take every step alone
+    a.singles = ROUND_FROM;
+    for (int k = 0; k < d; ++k)
+      if (hi[k] > lo[k] && !(hi[k] - lo[k] > 1e-18 && hi[k] - lo[k] < 1e18)) a.singles = n;
+    const auto kernel = d <= 2 ? k_maxmin_grid<2> : d == 3 ? k_maxmin_grid<3> : d == 4 ? k_maxmin_grid<4> : k_maxmin_grid<8>;
+    const size_t smem = maxmin_smem(a.ng1, d);
+    LKG_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     const int chunk = 65536;  // steps per launch: each launch stays well under a second
     for (int t0 = 0; t0 < n; t0 += chunk) {
       a.t0 = t0;
       a.t1 = std::min(n, t0 + chunk);
       LaunchTimer lt("k_maxmin_grid", st, 0.0, 8.0 * (a.t1 - t0) * 64.0);
-      k_maxmin_grid<<<1, MM_THREADS, smem, st>>>(a);
+      kernel<<<1, MM_THREADS, smem, st>>>(a);
       LKG_LAUNCH("k_maxmin_grid");
     }
     LKG_CUDA(cudaStreamSynchronize(st));  // cstart / cursor are freed at scope exit
