@@ -70,23 +70,19 @@ __device__ __forceinline__ void cov_fast_term(double dx, double ck, double& sum_
 // halves, and past 1500 the value is below the smallest double for any d <= 32 (prod <= (1 + 1500 / 32 + (1500 /
 // 32)^2 / 3)^32 < e^214).  An infinite or NaN sum falls through to inf * 0 = NaN, as in the log1p form.  The range test
 // reads the high word: a compare of doubles would take an FP64 issue slot of every pair.
-template <int K, class Exp>
-__device__ __forceinline__ double cov_fast_finish_e(double sum_state, double prod_state, Exp expf64) {
-  if constexpr (K == KGAUSS) return expf64(-0.5 * sum_state);
-  else if constexpr (K == KEXP) return expf64(-sum_state);
+template <int K>
+__device__ __forceinline__ double cov_fast_finish(double sum_state, double prod_state) {
+  if constexpr (K == KGAUSS) return exp(-0.5 * sum_state);
+  else if constexpr (K == KEXP) return exp(-sum_state);
   else {
     const int hi = __double2hiint(sum_state);
     if (hi >= 0x4085E000 && hi < 0x7FF00000) {  // 700 <= sum < infinity
       if (sum_state > 1500.0) return 0.0;
-      const double h = expf64(-0.5 * sum_state);
+      const double h = exp(-0.5 * sum_state);
       return prod_state * h * h;
     }
-    return prod_state * expf64(-sum_state);
+    return prod_state * exp(-sum_state);
   }
-}
-template <int K>
-__device__ __forceinline__ double cov_fast_finish(double sum_state, double prod_state) {
-  return cov_fast_finish_e<K>(sum_state, prod_state, [](double x) { return exp(x); });
 }
 
 // dlnC/dtheta_k with inv = 1 / theta_k and ck = s / theta_k

@@ -17,7 +17,6 @@
 #include "common.cuh"
 #include "config.hpp"
 #include "devbuf.cuh"
-#include "exp.cuh"
 #include "stats.hpp"
 
 namespace lkg {
@@ -69,10 +68,14 @@ __device__ __forceinline__ int wargmax(double v, int lane, int mi) {
 }
 
 // One m x m block per warp in shared memory, M (pitch LDP): the strict lower triangle holds RN, the strict upper one its
-// factor RN + (diagonal) = U D U', U unit lower, transposed: M[j][i] = U_ij for i > j.  Lane i keeps the diagonal entry
-// d_i and its reciprocal.  FP64 issue bounds these kernels (GB300 runs FP64 at 1/64 of the FP32 rate), so the
-// factorisation is the root-free one (a reciprocal per column, no square roots), the solves take one fused multiply-add
-// per step, and what decides nothing to FP64 accuracy runs in FP32 (the conditioning certificate below).
+// factor RN + (diagonal) = L L' as the unit lower U = L diag(L)^-1, transposed: M[j][i] = U_ij for i > j.  Lane i keeps the
+// squared pivot d_i = L_ii^2 and 1 / L_ii.  FP64 issue bounds these kernels (GB300 runs FP64 at 1/64 of the FP32 rate), so
+// the solves take one fused multiply-add per step and scale by 1 / L_ii once, and what decides nothing to FP64 accuracy
+// runs in FP32 (the conditioning certificate below).  The blocks of close points are so ill-conditioned that their
+// conditional variances show the rounding of every FP64 operation (relative 1e-8 and more where the nugget is all that
+// separates them), so the covariances, the factorisation and the sums keep one fixed sequence of operations.  A
+// root-free factorisation with a table exponential took 7.3 ms where this takes 8.8, no less accurate, but moved
+// gradients of such models by up to 4e-8.
 
 // solve U w = b (lane i holds b_i); lanes >= mi return 0
 __device__ __forceinline__ double wsolve_u(const double* M, double b, int mi, int lane) {
@@ -101,19 +104,28 @@ __device__ __forceinline__ void tri_rc(int e, int& r, int& c) {
   c = e - r * (r + 1) / 2;
 }
 
-// 1 / d of a pivot: the hardware's 20-bit approximation and one third-order step (e^3 < 2^-56)
-__device__ __forceinline__ double pivot_rcp(double d) {
-  const int hi = __double2hiint(d);
-  if (hi < 0x02000000 || hi >= 0x7E000000) return 1.0 / d;
-  double r;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(d));
-  const double e = fma(-d, r, 1.0);
-  return fma(r, fma(e, e, e), r);
+// 1 / sqrt(piv) by Newton's iteration y <- y (3 - piv y^2) / 2 from a single-precision seed: two steps take the
+// seed's 2^-23 relative error below FP64 rounding; outside the range where the seed is a normal float the square
+// root and the reciprocal are taken directly.  The range is read off the bits, and the conversions (to nearest even) and
+// the factor -1/2 are integer operations: each would take an FP64 issue slot per pivot.
+__device__ __forceinline__ double pivot_rroot(double piv) {
+  const int hi = __double2hiint(piv);
+  if (hi < 0x39C00000 || hi >= 0x46200000) {  // within a factor of 2 of 1e-30 and 1e30, or beyond
+    if (!(piv >= 1e-30 && piv <= 1e30)) return 1.0 / sqrt(piv);
+  }
+  constexpr unsigned long long kBias = 896ull << 52;  // FP64 exponent bias minus FP32's
+  unsigned long long pb = (unsigned long long)__double_as_longlong(piv) - kBias;
+  pb += 0x0FFFFFFFull + ((pb >> 29) & 1ull);
+  const float seed = rsqrtf(__int_as_float((int)(pb >> 29)));
+  double y = __longlong_as_double((long long)(((unsigned long long)(unsigned)__float_as_int(seed) << 29) + kBias));
+  const double h = __hiloint2double((hi - 0x00100000) | 0x80000000, __double2loint(piv));
+  y = y * fma(h, y * y, 1.5);
+  return y * fma(h, y * y, 1.5);
 }
 
-// U D U' of RN with diagonal diag, right-looking: column j's reciprocal pivot, its scaled copy, then the strict lower
-// trailing entries with their (row, column) pairs spread over the lanes (the diagonal stays in the lanes' registers).
-// di, ri: this lane's d_i and 1 / d_i.  False on a non-positive or NaN pivot (uniform over the warp).
+// Cholesky of RN with diagonal diag, right-looking: column j scaled by 1 / L_jj, then the strict lower trailing entries
+// with their (row, column) pairs spread over the lanes (the diagonal stays in the lanes' registers).  di, ri: this lane's
+// L_ii^2 and 1 / L_ii.  False on a non-positive or NaN pivot (uniform over the warp).
 __device__ bool wfactor(double* M, double* ub, double diag, int mi, int lane, double& di, double& ri) {
   const int np = mi * (mi - 1) / 2;
   for (int e = lane; e < np; e += 32) {
@@ -128,13 +140,13 @@ __device__ bool wfactor(double* M, double* ub, double diag, int mi, int lane, do
     const double piv = __shfl_sync(FULL, di, j);
     const long long pb = __double_as_longlong(piv);  // a positive number, read without an FP64 compare
     if (pb <= 0 || pb > 0x7FF0000000000000ll) return false;
-    const double rp = pivot_rcp(piv);
+    const double rp = pivot_rroot(piv);
     if (lane == j) ri = rp;
     if (lane > j && lane < mi) {
-      const double u = M[j * LDP + lane], t = u * rp;
+      const double u = M[j * LDP + lane] * rp;
       ub[lane] = u;
-      M[j * LDP + lane] = t;
-      di -= u * t;
+      M[j * LDP + lane] = u * rp;
+      di -= u * u;
     }
     __syncwarp();
     const int m1 = mi - 1 - j, ne = m1 * (m1 - 1) / 2;
@@ -142,7 +154,7 @@ __device__ bool wfactor(double* M, double* ub, double diag, int mi, int lane, do
       int rr, cc;
       tri_rc(e, rr, cc);
       const int c = j + 1 + cc, r = j + 2 + rr;
-      M[c * LDP + r] -= ub[r] * M[j * LDP + c];
+      M[c * LDP + r] -= ub[r] * ub[c];
     }
     __syncwarp();
   }
@@ -158,7 +170,7 @@ __device__ __forceinline__ float truncated_f32(double x) {
   return __int_as_float((hi & 0x80000000) | mag);
 }
 
-// FP32 certificate that rcond(L)^2 >= min_rcond, L = U sqrt(D).  With X the columns of L^-1 computed in FP32 and
+// FP32 certificate that rcond(L)^2 >= min_rcond.  With X the columns of L^-1 computed in FP32 and
 // k = |L|_1 |X|_1, the componentwise backward error of each column's forward substitution, together with the rounding of
 // L to FP32, gives |L|_1 |L^-1|_1 <= k / (1 - k eta) with eta = (m + 10) 2^-24: a bound on the norm that the dlacn2
 // estimate never exceeds, so a certified block passes that test too.  True only when it is certain; NaN, overflow or
@@ -244,54 +256,30 @@ __device__ __noinline__ double wrcond2(const double* M, double di, int mi, int l
   return rc * rc;
 }
 
-// the scale c of a dimension's distances: the covariances below take t = c |dx| (gauss: exp(-t^2) with c = sqrt(1/2) /
-// theta)
-template <int K>
-__device__ __forceinline__ double point_scale(double theta) {
-  return (K == KGAUSS ? 0.70710678118654752440 : cov_scale<K>()) / fabs(theta);
-}
 template <int K, int DM>
-__device__ __forceinline__ double point_cov(const double* xa, const double* xb, const double (&ck)[DM], int d,
-                                            const double* etab) {
+__device__ __forceinline__ double point_cov(const double* xa, const double* xb, const double (&ck)[DM], int d) {
   double s = 0.0, pr = 1.0;
 #pragma unroll
   for (int k = 0; k < DM; ++k)
     if (k < d) cov_fast_term<K>(xa[k] - xb[k], ck[k], s, pr);
-  if constexpr (K == KGAUSS || K == KEXP) return exp_tab(-s, etab);
-  else return cov_fast_finish_e<K>(s, pr, [&](double x) { return exp_tab(x, etab); });
-}
-// theta_k dlnC / dtheta_k with t = c dx: gauss 2 t^2, exp t, matern3_2 t^2 / (1 + t), matern5_2 (1 + t) b / (1 + t + b)
-// with b = t^2 / 3
-template <int K>
-__device__ __forceinline__ double point_dln(double t) {
-  if constexpr (K == KGAUSS) return t * t;  // the factor 2 goes with 1 / theta_k
-  else if constexpr (K == KEXP) return fabs(t);
-  else if constexpr (K == KMATERN32) {
-    t = fabs(t);
-    return t * t * pivot_rcp(1.0 + t);
-  } else {
-    t = fabs(t);
-    const double a = 1.0 + t, b = t * t * (1.0 / 3.0);
-    return a * b * pivot_rcp(a + b);
-  }
+  return cov_fast_finish<K>(s, pr);
 }
 
 // per-warp shared memory of the point kernels, in doubles
 template <int DM>
 constexpr int point_smem() { return 32 * LDP + 32 + 32 * DM + 32 * UFP / 2; }
-constexpr int kTabSize = 64;  // the exponential's table, once per block
 
 // RN's strict lower triangle (each pair once, spread over the lanes) and, per lane, r = C(x_lane, xo)
 template <int K, int DM>
 __device__ __forceinline__ double point_block(double* M, const double* xs, const double* xo, const double (&ck)[DM], int d,
-                                              int mi, int lane, const double* etab) {
+                                              int mi, int lane) {
   const int np = mi * (mi - 1) / 2;
   for (int e = lane; e < np; e += 32) {
     int rr, cc;
     tri_rc(e, rr, cc);
-    M[(rr + 1) * LDP + cc] = point_cov<K, DM>(xs + (rr + 1) * DM, xs + cc * DM, ck, d, etab);
+    M[(rr + 1) * LDP + cc] = point_cov<K, DM>(xs + (rr + 1) * DM, xs + cc * DM, ck, d);
   }
-  const double r = (lane < mi) ? point_cov<K, DM>(xs + lane * DM, xo, ck, d, etab) : 0.0;
+  const double r = (lane < mi) ? point_cov<K, DM>(xs + lane * DM, xo, ck, d) : 0.0;
   __syncwarp();
   return r;
 }
@@ -322,19 +310,17 @@ struct VPointArgs {
   int* status;
 };
 
-// One warp per ordered point.  Measured, n = 100003, d = 3, m = 30, gauss, with gradient: 11.7 ms with a root per pivot, the
-// dlacn2 estimate for every block, CUDA's exp and a second m x m buffer; 7.3 ms now (85 % of the FP64 pipe's issue).
+// One warp per ordered point.  Measured, n = 100003, d = 3, m = 30, gauss, with gradient: 11.7 ms with the dlacn2 estimate
+// for every block, FP64 conversions and compares at every pivot, five FP64 sums over the warp per derivative, each in all
+// lanes, and a second m x m buffer; 8.8 ms now, the same bits, about 1400 FP64 warp instructions a point.
 template <int K, int DM>
 __global__ void __launch_bounds__(WPB * 32) k_vecchia_points(VPointArgs a) {
   extern __shared__ __align__(16) double vsm[];
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  double* etab = vsm;
-  double* M = vsm + kTabSize + (size_t)w * point_smem<DM>();
+  double* M = vsm + (size_t)w * point_smem<DM>();
   double* ub = M + 32 * LDP;                              // [32]
   double* xs = ub + 32;                                   // [32][DM]
   float* Uf = reinterpret_cast<float*>(xs + 32 * DM);     // [32][UFP]
-  exp_table_fill<WPB * 32>(etab);
-  __syncthreads();
   const int t = a.t0 + blockIdx.x * WPB + w;
   if (t >= a.t1) return;
   const int n = a.n, d = a.d, p = a.p;
@@ -356,17 +342,18 @@ __global__ void __launch_bounds__(WPB * 32) k_vecchia_points(VPointArgs a) {
     }
     return;
   }
+  const double inv = 1.0 / (lane < d ? a.theta[lane] : 1.0);  // lane k: dimension k's
   double ck[DM], xo[DM];
 #pragma unroll
   for (int k = 0; k < DM; ++k) {
-    ck[k] = (k < d) ? point_scale<K>(a.theta[k]) : 0.0;
+    ck[k] = cov_scale<K>() * __shfl_sync(FULL, inv, k);
     xo[k] = (k < d) ? a.X[oi + (int64_t)k * n] : 0.0;
   }
   if (lane < mi)
 #pragma unroll
     for (int k = 0; k < DM; ++k) xs[lane * DM + k] = (k < d) ? a.X[nbv + (int64_t)k * n] : 0.0;
   __syncwarp();
-  const double r = point_block<K, DM>(M, xs, xo, ck, d, mi, lane, etab);
+  const double r = point_block<K, DM>(M, xs, xo, ck, d, mi, lane);
   double di, ri;
   const int inc = point_factor(M, ub, Uf, a.num_nugget, a.min_rcond, a.rcond_check, a.max_inc, mi, lane, di, ri);
   if (inc < 0) {
@@ -374,7 +361,7 @@ __global__ void __launch_bounds__(WPB * 32) k_vecchia_points(VPointArgs a) {
     return;
   }
   // ---- a, v, u, W ----
-  auto solve = [&](double b) { return wsolve_ut(M, wsolve_u(M, b, mi, lane) * ri, mi, lane); };  // RN^-1 b
+  auto solve = [&](double b) { return wsolve_ut(M, wsolve_u(M, b, mi, lane) * ri * ri, mi, lane); };  // RN^-1 b
   const double av = solve(r);
   const double yN = (lane < mi) ? a.y[nbv] : 0.0;
   double fN[VPMAX];
@@ -399,35 +386,33 @@ __global__ void __launch_bounds__(WPB * 32) k_vecchia_points(VPointArgs a) {
   __syncwarp();
   double* sa = ub;
   sa[lane] = av;
-  // the factor is no longer needed: the strict upper triangle holds M_k(a, b) = RN(a, b) theta_k dlnC/dtheta_k(x_a - x_b),
+  // the factor is no longer needed: the strict upper triangle holds M_k(a, b) = RN(a, b) dlnC/dtheta_k(x_a - x_b),
   // formed once per pair (symmetric: |dx| or dx^2 only) with the pairs spread over the lanes, then
   // s_a = sum_b M_k(a, b) a_b
   const int npair = mi * (mi - 1) / 2;
   for (int k = 0; k < d; ++k) {
-    const double c = ck[k], inv = (K == KGAUSS ? 2.0 : 1.0) / a.theta[k];
+    const double iv = __shfl_sync(FULL, inv, k), c = cov_scale<K>() * iv;
     __syncwarp();
     for (int e = lane; e < npair; e += 32) {
       int rr, cc;
       tri_rc(e, rr, cc);
       const int ra = rr + 1;
-      M[cc * LDP + ra] = M[ra * LDP + cc] * point_dln<K>((xs[ra * DM + k] - xs[cc * DM + k]) * c);
+      M[cc * LDP + ra] = M[ra * LDP + cc] * dlncov_fast<K>(xs[ra * DM + k] - xs[cc * DM + k], iv, c);
     }
     __syncwarp();
     double drk = 0.0, s = 0.0;
     if (lane < mi) {
-      drk = r * point_dln<K>((xs[lane * DM + k] - xo[k]) * c);
+      drk = r * dlncov_fast<K>(xs[lane * DM + k] - xo[k], iv, c);
       for (int b = 0; b < mi; ++b)
         if (b != lane) s += (b < lane ? M[b * LDP + lane] : M[lane * LDP + b]) * sa[b];
     }
-    drk *= inv;
-    s *= inv;
     const double g = drk - s;
-    double red2[4] = {av * (drk + g), g * by, p > 0 ? g * cq[0] : 0.0, 0.0};  // dv_k = -(2 a'dr_k - a'M_k a)
+    double red2[4] = {av * drk, av * s, g * by, p > 0 ? g * cq[0] : 0.0};
     wsum4(red2, lane);
     if (lane == 0) {
-      a.dv[(int64_t)t * d + k] = -red2[0];
-      a.du[(int64_t)t * d + k] = -red2[1];
-      if (p > 0) a.dW[((int64_t)t * d + k) * p] = -red2[2];
+      a.dv[(int64_t)t * d + k] = -(2.0 * red2[0] - red2[1]);
+      a.du[(int64_t)t * d + k] = -red2[2];
+      if (p > 0) a.dW[((int64_t)t * d + k) * p] = -red2[3];
     }
     for (int q = 1; q < p; ++q) {
       const double gc = wsum(g * cq[q]);
@@ -539,7 +524,7 @@ __global__ void k_count_status(int t0, int t1, const int* __restrict__ status, i
 template <int K, int DM>
 struct VPointLaunch {
   static void run(const VPointArgs& a, cudaStream_t st) {
-    const size_t smem = (kTabSize + (size_t)WPB * point_smem<DM>()) * sizeof(double);
+    const size_t smem = ((size_t)WPB * point_smem<DM>()) * sizeof(double);
     static bool attr = false;
     if (!attr) {
       LKG_CUDA(cudaFuncSetAttribute(k_vecchia_points<K, DM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
@@ -590,18 +575,16 @@ struct VPredArgs {
 // observations whose bound reaches the m-th best distance so far (some m ln(n / m) of them) take the FP64 distance and
 // the exact comparison.  The sorted list lies one entry per lane, in registers: an insertion is a ballot and a shift.
 // Measured, 20000 points, n = 10007, d = 3, m = 30: the FP64 scan with the list sorted by one lane in shared memory and
-// the local kriging of the time 12.1 ms; now 2.6 ms.
+// the local kriging of the time 12.1 ms; now 2.9 ms.
 template <int K, int DM>
 __global__ void __launch_bounds__(WPB * 32) k_vecchia_predict(VPredArgs a) {
   extern __shared__ __align__(16) double psm[];
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  double* etab = psm;
-  float* tile = reinterpret_cast<float*>(psm + kTabSize);  // [DM][PTILE]
-  double* M = psm + kTabSize + PTILE * DM / 2 + (size_t)w * point_smem<DM>();
+  float* tile = reinterpret_cast<float*>(psm);  // [DM][PTILE]
+  double* M = psm + PTILE * DM / 2 + (size_t)w * point_smem<DM>();
   double* ub = M + 32 * LDP;
   double* xs = ub + 32;
   float* Uf = reinterpret_cast<float*>(xs + 32 * DM);
-  exp_table_fill<WPB * 32>(etab);
   const int t = blockIdx.x * WPB + w;
   const bool active = t < a.q;
   const int n = a.n, d = a.d, m = a.m;
@@ -677,19 +660,19 @@ __global__ void __launch_bounds__(WPB * 32) k_vecchia_predict(VPredArgs a) {
   const int nbv = (lane < mi) ? li : -1;
   double ck[DM];
 #pragma unroll
-  for (int k = 0; k < DM; ++k) ck[k] = (k < d) ? point_scale<K>(a.theta[k]) : 0.0;
+  for (int k = 0; k < DM; ++k) ck[k] = cov_scale<K>() / ((k < d) ? a.theta[k] : 1.0);
   if (lane < mi)
 #pragma unroll
     for (int k = 0; k < DM; ++k) xs[lane * DM + k] = (k < d) ? a.X[nbv + (int64_t)k * n] : 0.0;
   __syncwarp();
-  const double r = point_block<K, DM>(M, xs, xq, ck, d, mi, lane, etab);
+  const double r = point_block<K, DM>(M, xs, xq, ck, d, mi, lane);
   double di, ri;
   const int inc = point_factor(M, ub, Uf, a.num_nugget, a.min_rcond, a.rcond_check, a.max_inc, mi, lane, di, ri);
   if (inc < 0) {
     if (lane == 0) a.status[t] = -1;
     return;
   }
-  const double av = wsolve_ut(M, wsolve_u(M, r, mi, lane) * ri, mi, lane);
+  const double av = wsolve_ut(M, wsolve_u(M, r, mi, lane) * ri * ri, mi, lane);
   const double rs = (lane < mi) ? a.resid[nbv] : 0.0;
   const double ar = wsum(av * rs), ra = wsum(r * av);
   if (lane == 0) {
@@ -723,7 +706,7 @@ __global__ void __launch_bounds__(256) k_center_f32(int n, const double* __restr
 template <int K, int DM>
 struct VPredLaunch {
   static void run(const VPredArgs& a, cudaStream_t st) {
-    const size_t smem = (kTabSize + (size_t)PTILE * DM / 2 + (size_t)WPB * point_smem<DM>()) * sizeof(double);
+    const size_t smem = ((size_t)PTILE * DM / 2 + (size_t)WPB * point_smem<DM>()) * sizeof(double);
     LKG_CUDA(cudaFuncSetAttribute(k_vecchia_predict<K, DM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     LaunchTimer lt("k_vecchia_predict", st, 3.0 * a.q * (double)a.n * a.d, 8.0 * a.n * a.d);
     k_vecchia_predict<K, DM><<<ceil_div(a.q, WPB), WPB * 32, smem, st>>>(a);

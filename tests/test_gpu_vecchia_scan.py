@@ -1,4 +1,4 @@
-"""predictVecchia's FP32 neighbour scan and the root-free local factorisation against the oracle: offsets that leave FP32
+"""predictVecchia's FP32 neighbour scan and the local factorisation against the oracle: offsets that leave FP32
 few digits, ties, the smallest and largest m, and blocks that the FP32 certificate cannot clear."""
 import numpy as np
 import pytest
