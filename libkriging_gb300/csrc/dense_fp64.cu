@@ -101,6 +101,66 @@ __global__ void __launch_bounds__(NT) k_gemm_tiles(int M, int N, int K, double a
   tile_store(M, N, alpha, beta, C + b * c_batch, ldc, m0, n0, lower_only, acc);
 }
 
+// ---- products of few tiles ----
+// A 64 x 64 tile with K = 64 holds its SM's FP64 pipes for 63 us (1024 DFMAs of each of its 8 warps), and a matrix of a
+// few blocks has only a few tiles, so here 128 threads take one entry each: TM x TN = 128 entries a CTA, 32 times as many
+// CTAs.  2 x 64 and 64 x 2 serve the in-place products, whose CTAs own whole rows (columns) of C.  Every entry adds its
+// terms in ascending k, as in the large tiles, so the two give the same bits and the choice may look at the batch.
+// Measured, products of an LL + gradient at n = 191: 840 us in 9 launches of large tiles, 102 us of small ones.
+constexpr int SM_THREADS = 128;
+constexpr int SM_K = 64;
+constexpr int SM_LD = SM_K + 1;
+
+// s[i][k] = p[i sr + k sk] for i < cnt, k < kc, zero up to T rows and SM_K columns
+template <int T>
+__device__ __forceinline__ void stage_rows(const double* __restrict__ p, int64_t sr, int64_t sk, int cnt, int kc,
+                                           double (*s)[SM_LD]) {
+  constexpr int PER = T * SM_K / SM_THREADS;
+  double v[PER];
+#pragma unroll
+  for (int u = 0; u < PER; ++u) {
+    const int idx = threadIdx.x + u * SM_THREADS;
+    const int i = sr == 1 ? idx % T : idx / SM_K, k = sr == 1 ? idx / T : idx % SM_K;
+    v[u] = (i < cnt && k < kc) ? p[i * sr + k * sk] : 0.0;
+  }
+#pragma unroll
+  for (int u = 0; u < PER; ++u) {
+    const int idx = threadIdx.x + u * SM_THREADS;
+    s[sr == 1 ? idx % T : idx / SM_K][sr == 1 ? idx / T : idx % SM_K] = v[u];
+  }
+}
+
+// skip_rows: the terms k < m0 rounded down to a block are zero (W^T W)
+template <int TM, int TN>
+__global__ void __launch_bounds__(SM_THREADS) k_gemm_small(int M, int N, int K, double alpha, MatView A, MatView B,
+                                                           double beta, double* C, int64_t ldc, int64_t c_batch,
+                                                           bool lower_only, bool skip_rows) {
+  static_assert(TM * TN == SM_THREADS);
+  const int m0 = blockIdx.x * TM, n0 = blockIdx.y * TN;
+  if (lower_only && m0 + TM - 1 < n0) return;
+  __shared__ double as[TM][SM_LD], bs[TN][SM_LD];
+  const int64_t b = blockIdx.z;
+  const double* Ap = A.p + b * A.batch + m0 * A.sr;
+  const double* Bp = B.p + b * B.batch + n0 * B.sc;
+  const int m = threadIdx.x % TM, c = threadIdx.x / TM;
+  double acc = 0.0;
+  for (int k0 = skip_rows ? m0 / SM_K * SM_K : 0; k0 < K; k0 += SM_K) {
+    const int kc = min(SM_K, K - k0);
+    stage_rows<TM>(Ap + k0 * A.sc, A.sr, A.sc, M - m0, kc, as);
+    stage_rows<TN>(Bp + k0 * B.sr, B.sc, B.sr, N - n0, kc, bs);
+    __syncthreads();
+    const int kr = (kc + KC - 1) / KC * KC;
+#pragma unroll 16
+    for (int k = 0; k < kr; ++k) acc = fma(as[m][k], bs[c][k], acc);
+    __syncthreads();
+  }
+  const int r = m0 + m, cc = n0 + c;
+  if (r < M && cc < N && (!lower_only || r >= cc)) {
+    double* cp = C + b * c_batch + r + (int64_t)cc * ldc;
+    *cp = (beta == 0.0) ? alpha * acc : fma(alpha, acc, beta * *cp);
+  }
+}
+
 // ---- diagonal block: Cholesky + inverse in shared memory (one CTA per batch entry) ----
 constexpr int DPAD = NB + 1;
 
@@ -595,9 +655,37 @@ void zero_upper(double* A, int64_t lda, int64_t mstride, int n, int batch, cudaS
   LKG_LAUNCH("k_zero_upper");
 }
 
+namespace {
+
+// Up to two waves of large tiles take the small ones: the FP64 pipes need as long for the same terms, but all SMs have some.
+bool few_tiles(int64_t tiles) { return tiles <= 2 * 152; }
+
+template <int TM, int TN>
+void gemm_small_launch(int M, int N, int K, double alpha, MatView A, MatView B, double beta, double* C, int64_t ldc,
+                       int64_t c_batch, int batch, bool lower_only, bool skip_rows, cudaStream_t st) {
+  k_gemm_small<TM, TN><<<dim3(ceil_div(M, TM), ceil_div(N, TN), batch), SM_THREADS, 0, st>>>(
+      M, N, K, alpha, A, B, beta, C, ldc, c_batch, lower_only, skip_rows);
+  LKG_LAUNCH("k_gemm_small");
+}
+
+}  // namespace
+
 void gemm_tiles(int M, int N, int K, double alpha, MatView A, MatView B, double beta, double* C, int64_t ldc,
                 int64_t c_batch, int batch, bool lower_only, cudaStream_t st) {
   if (M <= 0 || N <= 0) return;
+  const int64_t mt = ceil_div(M, TB), nt = ceil_div(N, TB);
+  if (few_tiles((lower_only ? (mt * nt + mt) / 2 : mt * nt) * batch)) {
+    const double fl = (lower_only && M == N) ? (double)K * M * (M + 1.0) : 2.0 * M * N * K;
+    LaunchTimer lt("k_gemm_small", st, fl * batch,
+                   8.0 * ((double)M * K + (double)K * N + (beta == 0.0 ? 1.0 : 2.0) * M * N) * batch);
+    if (C == A.p)  // in place: a CTA reads its rows before it writes them
+      gemm_small_launch<2, 64>(M, N, K, alpha, A, B, beta, C, ldc, c_batch, batch, lower_only, false, st);
+    else if (C == B.p)
+      gemm_small_launch<64, 2>(M, N, K, alpha, A, B, beta, C, ldc, c_batch, batch, lower_only, false, st);
+    else
+      gemm_small_launch<8, 16>(M, N, K, alpha, A, B, beta, C, ldc, c_batch, batch, lower_only, false, st);
+    return;
+  }
   dim3 grid(ceil_div(M, TB), ceil_div(N, TB), batch);
   const double fl = (lower_only && M == N) ? (double)K * M * (M + 1.0) : 2.0 * M * N * K;
   const double by = 8.0 * ((double)M * K + (double)K * N + (beta == 0.0 ? 1.0 : 2.0) * M * N);
@@ -676,6 +764,12 @@ void wtw_lower(const double* W, int64_t ldw, int64_t wstride, int n, double* C, 
                int batch, cudaStream_t st) {
   const int nblk = ceil_div(n, TB);
   const int64_t ntiles = (int64_t)nblk * (nblk + 1) / 2;
+  if (few_tiles(ntiles * batch)) {
+    LaunchTimer lt("k_gemm_small", st, (double)n * (n + 1.0) * (n + 2.0) / 3.0 * batch, 8.0 * n * (n + 1.0) * batch);
+    const MatView wt{W, ldw, 1, wstride}, w{W, 1, ldw, wstride};
+    gemm_small_launch<8, 16>(n, n, n, 1.0, wt, w, 0.0, C, ldc, cstride, batch, true, true, st);
+    return;
+  }
   // sum over the lower triangle of 2 (n - i) flops per entry = n (n + 1) (n + 2) / 3
   LaunchTimer lt("k_wtw", st, (double)n * (n + 1.0) * (n + 2.0) / 3.0 * batch, 8.0 * n * (n + 1.0) * batch);
   k_wtw<<<dim3((unsigned)ntiles, 1, batch), NT, 0, st>>>(W, ldw, wstride, n, C, ldc, cstride);
