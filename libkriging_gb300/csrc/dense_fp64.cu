@@ -113,7 +113,7 @@ constexpr int SM_LD = SM_K + 1;
 
 // s[i][k] = p[i sr + k sk] for i < cnt, k < kc, zero up to T rows and SM_K columns
 template <int T>
-__device__ __forceinline__ void stage_rows(const double* __restrict__ p, int64_t sr, int64_t sk, int cnt, int kc,
+__device__ __forceinline__ void stage_rows(const double* p, int64_t sr, int64_t sk, int cnt, int kc,
                                            double (*s)[SM_LD]) {
   constexpr int PER = T * SM_K / SM_THREADS;
   double v[PER];
@@ -137,6 +137,8 @@ __global__ void __launch_bounds__(SM_THREADS) k_gemm_small(int M, int N, int K, 
                                                            bool lower_only, bool skip_rows) {
   static_assert(TM * TN == SM_THREADS);
   const int m0 = blockIdx.x * TM, n0 = blockIdx.y * TN;
+  chain_next();
+  chain_wait();
   if (lower_only && m0 + TM - 1 < n0) return;
   __shared__ double as[TM][SM_LD], bs[TN][SM_LD];
   const int64_t b = blockIdx.z;
@@ -232,14 +234,22 @@ constexpr int PW = 6 * 32;        // of them, those that update the trailing ent
 // block with its inverse; now 49 us, and 16 us for the inverse in k_trtri_diag, whose columns go to 16 CTAs.
 __global__ void __launch_bounds__(PT) k_potrf_diag(double* A, int64_t lda, int64_t mstride, int k0, int nb, int* info) {
   const int64_t b = blockIdx.z;
-  if (info[b] != 0) return;  // an earlier block of this matrix already failed
   __shared__ double s[NB * DPAD];  // s[j * DPAD + i]: column j
   __shared__ double l[2][NB];      // the factor's column of the current and of the next step
   __shared__ unsigned short tab[(NB - 2) * (NB - 1) / 2];
   __shared__ int bad;
   double* Ab = A + b * mstride + k0 + (int64_t)k0 * lda;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  chain_next();
+  // (row, column) of the packed lower triangle, row by row: a smaller triangle is a prefix
+  for (int e = tid; e < (NB - 2) * (NB - 1) / 2; e += PT) {
+    int r, c;
+    tri_index(e, r, c);
+    tab[e] = (unsigned short)(r | c << 8);
+  }
   if (tid == 0) bad = 0;
+  chain_wait();
+  if (info[b] != 0) return;  // an earlier block of this matrix already failed
   {  // all 16 loads of a thread in flight before the shared-memory stores
     double v[NB * NB / PT];
 #pragma unroll
@@ -252,12 +262,6 @@ __global__ void __launch_bounds__(PT) k_potrf_diag(double* A, int64_t lda, int64
       const int idx = tid + q * PT;
       s[(idx >> 6) * DPAD + (idx & 63)] = v[q];
     }
-  }
-  // (row, column) of the packed lower triangle, row by row: a smaller triangle is a prefix
-  for (int e = tid; e < (NB - 2) * (NB - 1) / 2; e += PT) {
-    int r, c;
-    tri_index(e, r, c);
-    tab[e] = (unsigned short)(r | c << 8);
   }
   __syncthreads();
   // column c: minus the product with column c - 1 (its own earlier ones are applied), then scaled by its pivot's root
@@ -352,7 +356,7 @@ constexpr int TS_LD = NB + 1;  // padded row of the staged L tile (TRANS)
 
 // Dinv_k staged column-major with a padded leading dimension (conflict-free for both access orders)
 // (loads batched in registers ahead of the shared-memory stores, so that a thread keeps 16 loads in flight)
-__device__ __forceinline__ void ts_stage_dinv(const double* __restrict__ D, double* ds) {
+__device__ __forceinline__ void ts_stage_dinv(const double* D, double* ds) {
 #pragma unroll
   for (int h = 0; h < NB * NB / TS_THREADS; h += 16) {
     double v[16];
@@ -396,10 +400,12 @@ __global__ void __launch_bounds__(TS_THREADS) k_trsv_step(const double* L, int64
   const int t = threadIdx.x;
   double* Bb = B + b * bstride;
   const double* Db = Dinv + b * dstride;
+  chain_next();  // L and its diagonal inverses are there from before the chain: they are loaded before the wait for B
   if ((int)blockIdx.x == nupd) {  // writer: X_kw over B_kw
     const int w0 = kw * NB, nbw = min(NB, n - w0);
-    for (int idx = t; idx < nbw * r; idx += TS_THREADS) bs[idx] = Bb[w0 + idx % nbw + (int64_t)(idx / nbw) * ldb];
     ts_stage_dinv(Db + (int64_t)kw * NB * NB, ds);
+    chain_wait();
+    for (int idx = t; idx < nbw * r; idx += TS_THREADS) bs[idx] = Bb[w0 + idx % nbw + (int64_t)(idx / nbw) * ldb];
     __syncthreads();
     ts_block_apply(ds, bs, xs, nbw, r, TRANS);
     __syncthreads();
@@ -407,7 +413,6 @@ __global__ void __launch_bounds__(TS_THREADS) k_trsv_step(const double* L, int64
     return;
   }
   const int k0 = k * NB, nb = min(NB, n - k0);
-  for (int idx = t; idx < nb * r; idx += TS_THREADS) bs[idx] = Bb[k0 + idx % nb + (int64_t)(idx / nb) * ldb];
   ts_stage_dinv(Db + (int64_t)k * NB * NB, ds);
   const double* Lb = L + b * mstride;
   const int half = t >> 6, q = t & 63;  // two threads per row (column): kk halves
@@ -430,6 +435,8 @@ __global__ void __launch_bounds__(TS_THREADS) k_trsv_step(const double* L, int64
       }
     }
   }
+  chain_wait();
+  for (int idx = t; idx < nb * r; idx += TS_THREADS) bs[idx] = Bb[k0 + idx % nb + (int64_t)(idx / nb) * ldb];
   __syncthreads();
   ts_block_apply(ds, bs, xs, nb, r, TRANS);
   __syncthreads();
@@ -485,7 +492,8 @@ size_t trsv_smem(int r, bool trans) {
 
 template <bool TRANS, int RC>
 void trsv_launch_rc(const double* L, int64_t lda, int64_t mstride, const double* Dinv, int64_t dstride, double* B,
-                    int64_t ldb, int64_t bstride, int n, int k, int kw, int r, int nupd, int batch, cudaStream_t st) {
+                    int64_t ldb, int64_t bstride, int n, int k, int kw, int r, int nupd, int batch, cudaStream_t st,
+                    bool chained) {
   static bool attr_set = false;  // one flag per instantiation
   if (!attr_set) {
     LKG_CUDA(cudaFuncSetAttribute(k_trsv_step<TRANS, RC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -496,23 +504,26 @@ void trsv_launch_rc(const double* L, int64_t lda, int64_t mstride, const double*
   const double rows = (double)nupd * TS_ROWS;
   const char* name = TRANS ? "k_trsv_step_t" : "k_trsv_step";
   LaunchTimer lt(name, st, 2.0 * rows * NB * r * batch, 8.0 * (rows * NB + 2.0 * rows * r) * batch);
-  k_trsv_step<TRANS, RC><<<dim3(grid, 1, batch), TS_THREADS, trsv_smem(r, TRANS), st>>>(
-      L, lda, mstride, Dinv, dstride, B, ldb, bstride, n, k, kw, r, nupd);
-  LKG_LAUNCH(name);
+  // up to 2048 rows: more CTAs that wait with their operands in shared memory keep the inverse's products beside them off
+  // the SMs (n = 4096 13.6 -> 14.2 ms)
+  launch_chained(chained && nupd * batch <= 32, k_trsv_step<TRANS, RC>, dim3(grid, 1, batch), TS_THREADS, trsv_smem(r, TRANS), st, L, lda, mstride,
+                 Dinv, dstride, B, ldb, bstride, n, k, kw, r, nupd);
 }
 
 template <bool TRANS>
 void trsv_launch(const double* L, int64_t lda, int64_t mstride, const double* Dinv, int64_t dstride, double* B,
-                 int64_t ldb, int64_t bstride, int n, int k, int kw, int r, int nupd, int batch, cudaStream_t st) {
+                 int64_t ldb, int64_t bstride, int n, int k, int kw, int r, int nupd, int batch, cudaStream_t st,
+                 bool& chained) {
   if (nupd + (kw >= 0 ? 1 : 0) == 0) return;
   if (r == 1)
-    trsv_launch_rc<TRANS, 1>(L, lda, mstride, Dinv, dstride, B, ldb, bstride, n, k, kw, r, nupd, batch, st);
+    trsv_launch_rc<TRANS, 1>(L, lda, mstride, Dinv, dstride, B, ldb, bstride, n, k, kw, r, nupd, batch, st, chained);
   else if (r == 2)
-    trsv_launch_rc<TRANS, 2>(L, lda, mstride, Dinv, dstride, B, ldb, bstride, n, k, kw, r, nupd, batch, st);
+    trsv_launch_rc<TRANS, 2>(L, lda, mstride, Dinv, dstride, B, ldb, bstride, n, k, kw, r, nupd, batch, st, chained);
   else if (r <= 4)
-    trsv_launch_rc<TRANS, 4>(L, lda, mstride, Dinv, dstride, B, ldb, bstride, n, k, kw, r, nupd, batch, st);
+    trsv_launch_rc<TRANS, 4>(L, lda, mstride, Dinv, dstride, B, ldb, bstride, n, k, kw, r, nupd, batch, st, chained);
   else
-    trsv_launch_rc<TRANS, 8>(L, lda, mstride, Dinv, dstride, B, ldb, bstride, n, k, kw, r, nupd, batch, st);
+    trsv_launch_rc<TRANS, 8>(L, lda, mstride, Dinv, dstride, B, ldb, bstride, n, k, kw, r, nupd, batch, st, chained);
+  chained = true;
 }
 
 __global__ void __launch_bounds__(256) k_copy_dinv_block(const double* __restrict__ Dinv, int64_t dinv_bstride,
@@ -544,6 +555,8 @@ __global__ void __launch_bounds__(IT) k_trtri_diag(const double* L, int64_t lda,
                                                    int64_t dinv_bstride, int blk0, const int* info) {
   __shared__ double s[NB * DPAD], w[NB * (PB + 1)], x[NB * IC], tt[PB * IC];
   const int64_t b = blockIdx.z;
+  chain_next();
+  chain_wait();
   if (info && info[b] != 0) return;
   const int blk = blk0 + blockIdx.x, g = blockIdx.y, k0 = blk * NB, nb = min(NB, n - k0);
   const int c0 = g * IC, jb = c0 / PB;  // the 16-column block that holds this CTA's columns
@@ -624,16 +637,15 @@ __global__ void k_zero_upper(double* A, int64_t lda, int64_t mstride, int n) {
 }  // namespace
 
 void trtri_diag_launch(const double* L, int64_t lda, int64_t mstride, int n, double* Dinv, int64_t dinv_bstride, int blk0,
-                       int nblk, const int* info, int batch, cudaStream_t st) {
+                       int nblk, const int* info, int batch, cudaStream_t st, bool chained) {
   LaunchTimer lt("k_trtri_diag", st, (double)nblk * NB * NB * NB / 3.0 * batch, 16.0 * nblk * NB * NB * batch);
-  k_trtri_diag<<<dim3(nblk, IG, batch), IT, 0, st>>>(L, lda, mstride, n, Dinv, dinv_bstride, blk0, info);
-  LKG_LAUNCH("k_trtri_diag");
+  launch_chained(chained, k_trtri_diag, dim3(nblk, IG, batch), IT, 0, st, L, lda, mstride, n, Dinv, dinv_bstride, blk0, info);
 }
 
 void trtri_diag_blocks(const double* L, int64_t lda, int64_t mstride, int n, double* Dinv, int batch,
                        cudaStream_t st) {
   const int nblk = ceil_div(n, NB);
-  trtri_diag_launch(L, lda, mstride, n, Dinv, (int64_t)nblk * NB * NB, 0, nblk, nullptr, batch, st);
+  trtri_diag_launch(L, lda, mstride, n, Dinv, (int64_t)nblk * NB * NB, 0, nblk, nullptr, batch, st, false);
 }
 
 void transpose_copy(const double* S, int64_t lds, double* D, int64_t ldd, int rows, int cols, cudaStream_t st) {
@@ -663,9 +675,8 @@ bool few_tiles(int64_t tiles) { return tiles <= 2 * 152; }
 template <int TM, int TN>
 void gemm_small_launch(int M, int N, int K, double alpha, MatView A, MatView B, double beta, double* C, int64_t ldc,
                        int64_t c_batch, int batch, bool lower_only, bool skip_rows, cudaStream_t st) {
-  k_gemm_small<TM, TN><<<dim3(ceil_div(M, TM), ceil_div(N, TN), batch), SM_THREADS, 0, st>>>(
-      M, N, K, alpha, A, B, beta, C, ldc, c_batch, lower_only, skip_rows);
-  LKG_LAUNCH("k_gemm_small");
+  launch_chained(!skip_rows && batch == 1, k_gemm_small<TM, TN>, dim3(ceil_div(M, TM), ceil_div(N, TN), batch), SM_THREADS, 0, st, M, N, K,
+                 alpha, A, B, beta, C, ldc, c_batch, lower_only, skip_rows);
 }
 
 }  // namespace
@@ -695,13 +706,12 @@ void gemm_tiles(int M, int N, int K, double alpha, MatView A, MatView B, double 
 }
 
 void potrf_diag(double* A, int64_t lda, int64_t mstride, int k0, int nb, double* Dinv, int64_t dinv_bstride, int blk,
-                int* info, int batch, cudaStream_t st) {
+                int* info, int batch, cudaStream_t st, bool chained) {
   {
     LaunchTimer lt("k_potrf_diag", st, nb * (double)nb * nb / 3.0 * batch, 16.0 * nb * nb * batch);
-    k_potrf_diag<<<dim3(1, 1, batch), PT, 0, st>>>(A, lda, mstride, k0, nb, info);
-    LKG_LAUNCH("k_potrf_diag");
+    launch_chained(chained && batch == 1, k_potrf_diag, dim3(1, 1, batch), PT, 0, st, A, lda, mstride, k0, nb, info);
   }
-  trtri_diag_launch(A, lda, mstride, k0 + nb, Dinv, dinv_bstride, blk, 1, info, batch, st);
+  trtri_diag_launch(A, lda, mstride, k0 + nb, Dinv, dinv_bstride, blk, 1, info, batch, st, batch == 1);
 }
 
 void potrf_blocked(double* A, int64_t lda, int64_t mstride, int n, double* Dinv, int* info, int batch,
@@ -711,7 +721,7 @@ void potrf_blocked(double* A, int64_t lda, int64_t mstride, int n, double* Dinv,
   LKG_CUDA(cudaMemsetAsync(info, 0, sizeof(int) * batch, st));
   for (int k = 0; k < nblk; ++k) {
     const int k0 = k * NB, nb = std::min(NB, n - k0);
-    potrf_diag(A, lda, mstride, k0, nb, Dinv, dstride, k, info, batch, st);
+    potrf_diag(A, lda, mstride, k0, nb, Dinv, dstride, k, info, batch, st, k > 0);
     const int M = n - k0 - nb;
     if (M <= 0) continue;
     double* A21 = A + (k0 + nb) + (int64_t)k0 * lda;
@@ -796,12 +806,14 @@ void trsm_lower_left(const double* L, int64_t lda, int64_t mstride, int n, const
     }
     return;
   }
-  // step k updates the rows below block k and writes X_{k-1}; the extra step writes the last block
+  // step k updates the rows below block k and writes X_{k-1}; the extra step writes the last block.  The first launch is
+  // not chained: the kernel before it may be the one that writes Dinv.
+  bool chained = false;
   for (int k = 0; k <= nblk; ++k) {
     const int k0 = k * NB;
     const int M = (k < nblk) ? n - k0 - std::min(NB, n - k0) : 0;
     trsv_launch<false>(L, lda, mstride, Dinv, dstride, B, ldb, bstride, n, k, k - 1, r, ceil_div(M, TS_ROWS), batch,
-                       st);
+                       st, chained);
   }
 }
 
@@ -825,10 +837,11 @@ void trsm_lower_left_t(const double* L, int64_t lda, int64_t mstride, int n, con
     return;
   }
   // step k (descending) updates the rows above block k and writes X_{k+1}; the extra step writes block 0
+  bool chained = false;
   for (int k = nblk - 1; k >= -1; --k) {
     const int nupd = (k >= 0) ? ceil_div(k * NB, TS_ROWS) : 0;
     trsv_launch<true>(L, lda, mstride, Dinv, dstride, B, ldb, bstride, n, k, (k + 1 < nblk) ? k + 1 : -1, r, nupd,
-                      batch, st);
+                      batch, st, chained);
   }
 }
 

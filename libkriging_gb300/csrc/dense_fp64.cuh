@@ -26,7 +26,7 @@ void gemm_tiles(int M, int N, int K, double alpha, MatView A, MatView B, double 
 // One Cholesky step on the diagonal block at (k0, k0) of each batch matrix (lda, stride mstride):
 // factors the nb x nb block in place and writes its inverse into Dinv (NB*NB per block, block index blk).
 void potrf_diag(double* A, int64_t lda, int64_t mstride, int k0, int nb, double* Dinv, int64_t dinv_bstride,
-                int blk, int* info, int batch, cudaStream_t st);
+                int blk, int* info, int batch, cudaStream_t st, bool chained = false);
 
 // Full blocked lower Cholesky of each batch matrix (n x n, lower triangle referenced), keeping the inverses of
 // the diagonal blocks in Dinv (nblk * NB * NB per matrix).  info[b] = 1-based column of the first non-positive

@@ -23,18 +23,20 @@ void factor_panel7(double* A, int64_t lda, int64_t mstride, int n, int K0, doubl
   const int nblk = ceil_div(n, NB);
   const int64_t dstride = (int64_t)nblk * NB * NB;
   const int W = std::min(OZ7_KB, n - K0);
+  const bool chained = max_ctas == 0;  // beside the other stream's products, kernels that wait are in their way
   for (int k0 = K0; k0 < K0 + W; k0 += NB) {
     const int nb = std::min(NB, n - k0), k = k0 / NB;
-    potrf_diag(A, lda, mstride, k0, nb, Dinv, dstride, k, info, batch, st);
+    potrf_diag(A, lda, mstride, k0, nb, Dinv, dstride, k, info, batch, st, chained && k0 > K0);
     const int M = n - k0 - nb;
     if (M <= 0) continue;
     double* A21 = A + (k0 + nb) + (int64_t)k0 * lda;
     // L21 = A21 Dinv_k^T: B rows are the rows of Dinv_k
-    oz7_split2(M, nb, A21, 1, lda, mstride, SA, nb, nb, Dinv + (int64_t)k * NB * NB, 1, NB, dstride, SD, batch, st);
+    oz7_split2(M, nb, A21, 1, lda, mstride, SA, nb, nb, Dinv + (int64_t)k * NB * NB, 1, NB, dstride, SD, batch, st,
+               chained);
     oz7_gemm_ex(M, nb, 0, 1, 1.0, SA, 0, SD, 0, 0.0, A21, lda, mstride, batch, false, max_ctas, st);
     const int wr = K0 + W - (k0 + nb);  // panel columns right of this block
     if (wr > 0) {  // A(k0+nb:, k0+nb:K0+W) -= L21 L21(0:wr, :)^T (the strict upper part written is never read)
-      oz7_split(M, nb, A21, 1, lda, mstride, batch, SA, st);
+      oz7_split(M, nb, A21, 1, lda, mstride, batch, SA, st, chained);
       oz7_gemm_ex(M, wr, 0, 1, -1.0, SA, 0, SA, 0, 1.0, A21 + (int64_t)nb * lda, lda, mstride, batch, false,
                   max_ctas, st);
     }
@@ -57,7 +59,7 @@ void potrf_blocked_mixed7(double* A, int64_t lda, int64_t mstride, int n, double
       if (M2 <= 0) continue;
       // A22 -= P2 P2^T, P2 = L(K0+W:, K0:K0+W), one 256-wide k block
       double* P2 = A + (K0 + W) + (int64_t)K0 * lda;
-      oz7_split(M2, W, P2, 1, lda, mstride, batch, P, st);
+      oz7_split(M2, W, P2, 1, lda, mstride, batch, P, st, true);
       oz7_gemm(M2, M2, 0, 1, -1.0, P, P, 1.0, P2 + (int64_t)W * lda, lda, mstride, batch, true, st);
     }
     return;
@@ -102,13 +104,13 @@ void trtri_block7(const double* L, int64_t lda, int64_t mstride, int n, int K0, 
     const int nb = std::min(NB, n - k0), k = k0 / NB;
     if (k0 > 0) {  // W(k0:k0+nb, 0:k0) = -Dinv_k Acc(k0:k0+nb, 0:k0): B rows are the columns of Acc
       oz7_split2(nb, nb, Dinv + (int64_t)k * NB * NB, 1, NB, dstride, SA, k0, nb, W + k0, ldw, 1, wstride, SB,
-                 batch, st);
+                 batch, st, true);
       oz7_gemm(nb, k0, 0, 1, -1.0, SA, SB, 0.0, W + k0, ldw, wstride, batch, false, st);
     }
     const int mr = K0 + Wd - (k0 + nb);  // rows of this 256-row block below the 64-row one
     if (mr > 0) {  // Acc(k0+nb:K0+Wd, 0:k0+nb) += L(k0+nb:K0+Wd, k0:k0+nb) W(k0:k0+nb, 0:k0+nb)
       oz7_split2(mr, nb, L + (k0 + nb) + (int64_t)k0 * lda, 1, lda, mstride, SA, k0 + nb, nb, W + k0, ldw, 1,
-                 wstride, SB, batch, st);
+                 wstride, SB, batch, st, true);
       oz7_gemm(mr, k0 + nb, 0, 1, 1.0, SA, SB, 1.0, W + k0 + nb, ldw, wstride, batch, false, st);
     }
   }
@@ -136,7 +138,7 @@ void trtri_blocked_mixed7(const double* L, int64_t lda, int64_t mstride, int n, 
     // Acc(K0+Wd:, 0:N) += L(K0+Wd:, K0:K0+Wd) W(K0:K0+Wd, 0:N), N = K0 + Wd
     const int N = K0 + Wd;
     oz7_split2(M2, Wd, L + (K0 + Wd) + (int64_t)K0 * lda, 1, lda, mstride, SL, N, Wd, W + K0, ldw, 1, wstride, SR,
-               batch, st);
+               batch, st, true);
     oz7_gemm(M2, N, 0, 1, 1.0, SL, SR, 1.0, W + K0 + Wd, ldw, wstride, batch, false, st);
   }
 }
@@ -180,7 +182,7 @@ void gemm_square_digits(int n, const double* A, int64_t lda, const double* B, in
                          kh, OZ7_KB, true);
   for (int c0 = 0; c0 < n; c0 += kh) {
     const int kc = std::min(kh, n - c0);
-    oz7_split2(n, kc, A + (int64_t)c0 * lda, 1, lda, 0, SA, n, kc, B + c0, ldb, 1, 0, SB, 1, st);
+    oz7_split2(n, kc, A + (int64_t)c0 * lda, 1, lda, 0, SA, n, kc, B + c0, ldb, 1, 0, SB, 1, st, c0 > 0);
     oz7_gemm(n, n, 0, SA.nblk, 1.0, SA, SB, c0 == 0 ? 0.0 : 1.0, C, ldc, 0, 1, false, st);
   }
 }
@@ -214,17 +216,19 @@ void trsm_lower_left_digits(const double* L, int64_t lda, int n, const double* D
     const int Wd = std::min(OZ7_KB, n - K0);
     for (int k0 = K0; k0 < K0 + Wd; k0 += NB) {
       const int nb = std::min(NB, n - k0), k = k0 / NB;
-      oz7_split2(nb, nb, Dinv + (int64_t)k * NB * NB, 1, NB, 0, sl, r, nb, B + k0, ldb, 1, 0, sx, 1, st);
+      oz7_split2(nb, nb, Dinv + (int64_t)k * NB * NB, 1, NB, 0, sl, r, nb, B + k0, ldb, 1, 0, sx, 1, st, k > 0);
       oz7_gemm(nb, r, 0, 1, 1.0, sl, sx, 0.0, B + k0, ldb, 0, 1, false, st);
       const int mr = K0 + Wd - (k0 + nb);
       if (mr > 0) {
-        oz7_split2(mr, nb, L + (k0 + nb) + (int64_t)k0 * lda, 1, lda, 0, sl, r, nb, B + k0, ldb, 1, 0, sx, 1, st);
+        oz7_split2(mr, nb, L + (k0 + nb) + (int64_t)k0 * lda, 1, lda, 0, sl, r, nb, B + k0, ldb, 1, 0, sx, 1, st,
+                   true);
         oz7_gemm(mr, r, 0, 1, -1.0, sl, sx, 1.0, B + k0 + nb, ldb, 0, 1, false, st);
       }
     }
     const int M2 = n - K0 - Wd;
     if (M2 <= 0) continue;
-    oz7_split2(M2, Wd, L + (K0 + Wd) + (int64_t)K0 * lda, 1, lda, 0, SL, r, Wd, B + K0, ldb, 1, 0, SX, 1, st);
+    oz7_split2(M2, Wd, L + (K0 + Wd) + (int64_t)K0 * lda, 1, lda, 0, SL, r, Wd, B + K0, ldb, 1, 0, SX, 1, st,
+               true);
     oz7_gemm(M2, r, 0, 1, -1.0, SL, SX, 1.0, B + K0 + Wd, ldb, 0, 1, false, st);
   }
 }

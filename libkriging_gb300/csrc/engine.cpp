@@ -525,6 +525,7 @@ void Engine::rcond_core(int batch, std::vector<double>& rc2, const std::vector<i
 
 void Engine::evaluate(int batch, const double* thetas, const double* factors, bool with_grad,
                       std::vector<EvalOut>& out, std::map<std::string, double>* bench, const int* designs) {
+  const Unchained unchained(!alone_);
   if (batch < 1 || batch > cap_) throw std::invalid_argument("Engine::evaluate: batch out of range");
   wp_valid_ = false;
   if (ndesign_ > 1 && !designs) throw std::invalid_argument("Engine::evaluate: design of each entry required");
@@ -598,7 +599,7 @@ void Engine::evaluate(int batch, const double* thetas, const double* factors, bo
   // inverse on their own stream: 705 -> 579 us for n = 200, 2.75 -> 2.23 ms for 1003, 15.6 -> 13.6 ms for 4096, 64
   // entries of 2048 75.2 -> 74.1 ms.  Per-stage timing takes the stages one after another instead.
   const bool early_inverse = with_grad && rcond_check;
-  const bool beside = early_inverse && bench == nullptr;
+  const bool beside = early_inverse && bench == nullptr && alone_;
   bool solved = false;
   auto inverse_phase = [&] {
     ensure_grad_buffers();

@@ -136,6 +136,7 @@ class NestedService : public DenseService {
       c.eng = std::make_unique<Engine>(kernel, c.n_pad, d, p, (int)c.designs.size(), X.data(), y.data(), F.data(),
                                        nv.data(), c.cap);
       c.eng->set_slices(slices);
+      c.eng->set_alone(false);
     }
   }
 
@@ -626,6 +627,7 @@ void NestedKriging::precompute_nk() {
     std::vector<int> nv;
     pack_class(ds, c->groups, np, d, 1, X, y, F, nv);
     c->eng = std::make_unique<Engine>(m_kernel, np, d, 1, ne, X.data(), y.data(), F.data(), nv.data(), ne);
+    c->eng->set_alone(false);
     c->eng->set_plain_chol(true, 1.0 + kJitter);
     std::vector<double> th((size_t)ne * d), fac(ne, 1.0);
     std::vector<int> des(ne);

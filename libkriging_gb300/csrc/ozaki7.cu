@@ -231,9 +231,11 @@ struct SplitJob {
 // launch serves two operands: CTAs x < nx0 the first, the rest the second.
 template <int S>
 __global__ void __launch_bounds__(256) k_oz7_split(SplitJob j0, SplitJob j1, int nx0) {
+  chain_next();
+  chain_wait();
   const bool second = (int)blockIdx.x >= nx0;
   const int rows = second ? j1.rows : j0.rows, K = second ? j1.K : j0.K;
-  const double* __restrict__ p = second ? j1.p : j0.p;
+  const double* p = second ? j1.p : j0.p;
   const int64_t s_r = second ? j1.s_r : j0.s_r, s_k = second ? j1.s_k : j0.s_k;
   const int64_t bstride = second ? j1.bstride : j0.bstride;
   const Split7 out = second ? j1.out : j0.out;
@@ -391,6 +393,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_oz7_gemm(Oz7Args g, long long n
   const int spb = g.SA.sub_per_blk;
   auto bar = [](const uint64_t& x) { return su32(&x); };
 
+  chain_next();
   if (t == 0) {
     for (int i = 0; i < NA; ++i) {
       mbar_init(bar(bars.a_full[i]), 1);
@@ -415,6 +418,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_oz7_gemm(Oz7Args g, long long n
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
   const uint32_t tmem = tslot;
+  chain_wait();
   bool ok = true;
 
   if (w == 0) {
@@ -672,7 +676,8 @@ void launch_oz7(const Oz7Args& a, long long ntiles, int batch, int max_ctas, cud
   }
   long long gx = std::min<long long>(ntiles, std::max(1, nsm / std::max(1, batch)));
   if (max_ctas > 0) gx = std::min<long long>(gx, max_ctas);
-  k_oz7_gemm<S, TN><<<dim3((unsigned)gx, 1, batch), NTHREADS, smem, st>>>(a, ntiles);
+  // after its split, or another product
+  launch_chained(batch == 1 && max_ctas == 0, k_oz7_gemm<S, TN>, dim3((unsigned)gx, 1, batch), NTHREADS, smem, st, a, ntiles);
   LKG_LAUNCH("k_oz7_gemm");
 }
 
@@ -739,7 +744,7 @@ void split_prepare(int rows, int K, Split7& out) {
     throw std::logic_error("oz7_split: operand larger than its buffer");
 }
 
-void split_launch(const SplitJob& j0, const SplitJob& j1, int batch, cudaStream_t st) {
+void split_launch(const SplitJob& j0, const SplitJob& j1, int batch, cudaStream_t st, bool chained) {
   const int nx0 = j0.rows > 0 ? j0.out.rows_pad / 8 : 0, nx1 = j1.rows > 0 ? j1.out.rows_pad / 8 : 0;
   const int ny = std::max(j0.rows > 0 ? j0.out.nblk : 0, j1.rows > 0 ? j1.out.nblk : 0);
   if (nx0 + nx1 == 0) return;
@@ -747,11 +752,12 @@ void split_launch(const SplitJob& j0, const SplitJob& j1, int batch, cudaStream_
   LaunchTimer lt("k_oz7_split", st, 0.0,
                  ((double)j0.rows * j0.K * (8.0 + 2.0 * j0.out.S) + (double)j1.rows * j1.K * (8.0 + 2.0 * j1.out.S)) *
                      batch);
+  chained = chained && batch == 1;
   switch (j0.rows > 0 ? j0.out.S : j1.out.S) {
-    case 5: k_oz7_split<5><<<grid, 256, 0, st>>>(j0, j1, nx0); break;
-    case 6: k_oz7_split<6><<<grid, 256, 0, st>>>(j0, j1, nx0); break;
-    case 7: k_oz7_split<7><<<grid, 256, 0, st>>>(j0, j1, nx0); break;
-    default: k_oz7_split<8><<<grid, 256, 0, st>>>(j0, j1, nx0); break;
+    case 5: launch_chained(chained, k_oz7_split<5>, grid, 256, 0, st, j0, j1, nx0); break;
+    case 6: launch_chained(chained, k_oz7_split<6>, grid, 256, 0, st, j0, j1, nx0); break;
+    case 7: launch_chained(chained, k_oz7_split<7>, grid, 256, 0, st, j0, j1, nx0); break;
+    default: launch_chained(chained, k_oz7_split<8>, grid, 256, 0, st, j0, j1, nx0); break;
   }
   LKG_LAUNCH("k_oz7_split");
 }
@@ -759,23 +765,23 @@ void split_launch(const SplitJob& j0, const SplitJob& j1, int batch, cudaStream_
 }  // namespace
 
 void oz7_split(int rows, int K, const double* p, int64_t s_r, int64_t s_k, int64_t bstride, int batch, Split7& out,
-               cudaStream_t st) {
+               cudaStream_t st, bool chained) {
   if (rows <= 0 || K <= 0) return;
   split_prepare(rows, K, out);
   const SplitJob j0{rows, K, p, s_r, s_k, bstride, out}, none{0, 0, nullptr, 0, 0, 0, Split7{}};
-  split_launch(j0, none, batch, st);
+  split_launch(j0, none, batch, st, chained);
 }
 
 void oz7_split2(int rows0, int K0, const double* p0, int64_t s_r0, int64_t s_k0, int64_t bstride0, Split7& out0,
                 int rows1, int K1, const double* p1, int64_t s_r1, int64_t s_k1, int64_t bstride1, Split7& out1,
-                int batch, cudaStream_t st) {
+                int batch, cudaStream_t st, bool chained) {
   const bool a = rows0 > 0 && K0 > 0, c = rows1 > 0 && K1 > 0;
   if (a) split_prepare(rows0, K0, out0);
   if (c) split_prepare(rows1, K1, out1);
   if (a && c && out0.S != out1.S) throw std::invalid_argument("oz7_split2: operands with different digit counts");
   const SplitJob none{0, 0, nullptr, 0, 0, 0, Split7{}};
   split_launch(a ? SplitJob{rows0, K0, p0, s_r0, s_k0, bstride0, out0} : none,
-               c ? SplitJob{rows1, K1, p1, s_r1, s_k1, bstride1, out1} : none, batch, st);
+               c ? SplitJob{rows1, K1, p1, s_r1, s_k1, bstride1, out1} : none, batch, st, chained);
 }
 
 void oz7_gemm(int M, int N, int kb0, int kb1, double alpha, const Split7& SA, const Split7& SB, double beta, double* C,
