@@ -267,12 +267,13 @@ int lkg_get_digit_tile(void);
 /* No counterpart in the reference: the mixed Cholesky's look-ahead (n >= 1024, single-matrix evaluations): the next
  * 256-wide panel is factored on a second stream on `ctas` SMs while the rest of the trailing update runs on the
  * others.  0 turns it off; -1 (the default, unless LKG_LOOKAHEAD_CTAS is set) uses the autotuned choice for the
- * matrix size (lkg_kriging_autotune_lookahead), else 16.  The factor is the same bit for bit either way.  Returns
- * the value set, or -2 on an argument outside -1 .. 64 (lkg_get_lookahead returns the setting). */
+ * matrix size (lkg_kriging_autotune_lookahead), else 64 up to n = 8192 and fewer beyond (32 at 16384).  The factor is
+ * the same bit for bit either way.  Returns the value set, or -2 on an argument outside -1 .. 64 (lkg_get_lookahead
+ * returns the setting). */
 int lkg_set_lookahead(int ctas);
 int lkg_get_lookahead(void);
-/* No counterpart in the reference: CUDA graphs for the two launch sequences of an evaluation (covariance build +
- * factorisation; solves, GLS, R^-1 and adjoint sums), captured on the second run of a configuration and replayed
+/* No counterpart in the reference: CUDA graphs for the launch sequences of an evaluation (covariance build +
+ * factorisation; L^-1 with the solves and GLS beside it; R^-1 and adjoint sums), captured on the second run of a configuration and replayed
  * afterwards; on by default unless LKG_GRAPHS=0, and off while per-launch timing (lkg_stats_enable) is on.  Results
  * are the same bit for bit either way.  Returns the previous setting (1 on, 0 off). */
 int lkg_set_graphs(int on);
