@@ -23,10 +23,11 @@
 // tau, go step by step with FP64 distances (146 of 32768 steps).  The other warps meanwhile update the neighbourhoods of
 // the points taken, with atomic minima, and the tree follows.  A step alone costs 5.3 us, a chain of dependent loads and
 // FP64 operations.  More candidates than 512 make the pairs dearer than the rounds they save (an argmax over up to 1024
-// candidates and their distances to the point taken, step after step, cost 0.65 us a step).  Ties beyond 512
-// candidates (or an infinite maximum) fall back to a step alone.  Measured, n = 32768, d = 3: 172.6 ms by single steps,
+// candidates and their distances to the point taken, step after step, cost 0.65 us a step).  An infinite
+// maximum, and ties in more than 2048 nodes of the tree, fall back to a step alone.  Measured, n = 32768, d = 3: 172.6 ms by single steps,
 // 29.5 ms with an argmax per step, 11.1 ms with the pairs: neighbourhoods 6 ms, then finding the candidates, sorting
-// them, the pairs and the tree about 1 ms each.
+// them, the pairs and the tree about 1 ms each.  Where more than 512 points share the maximum (lattices), a round takes
+// those of the lowest indices: lattices of 32768 points 179 ms by single steps, 20 ms.
 // The cell range of a query is computed
 // with the same monotone floating-point map as the cells of the points, with a 1e-12 relative margin on the radius,
 // so every point that can change lies in a visited cell.
@@ -381,11 +382,14 @@ __global__ void __launch_bounds__(MM_THREADS, 1) k_maxmin_grid(MaxminArgs a) {
 
   double ratio = 0.9;         // uniform over the block, like the next two
   int singles = a.singles;    // position up to which steps are taken alone
-  int wait = 512;             // steps alone after ties that no round can hold, doubled each time they come again
+  int wait = 512;             // steps alone after ties that no round can list, doubled each time they come again
+  bool ties = false;          // more than CAND_MAX points share the maximum: the round takes those of them below index cut
+  int cut = n;
   int t = a.t0;
   while (t < a.t1) {
     bool single = t < singles;
     double now = ratio;
+    int lo = 0, hi = n + 1;
     while (!single) {  // the round's candidates; a smaller range of distances when there are too many
       if (w == 0) {
         long long bv = LLONG_MIN;
@@ -397,7 +401,7 @@ __global__ void __launch_bounds__(MM_THREADS, 1) k_maxmin_grid(MaxminArgs a) {
         if (lane == 0) {
           const double mx = __longlong_as_double(bv);
           rd_max = bv;
-          rd_tau = key_of(mx * now);
+          rd_tau = ties ? bv : key_of(mx * now);
           rd_radius = __double2float_ru(sqrt(mx) * (1.0 + 1e-6));
           rd_nodes = 0;
           rd_cands = 0;
@@ -448,6 +452,7 @@ __global__ void __launch_bounds__(MM_THREADS, 1) k_maxmin_grid(MaxminArgs a) {
               const int q = q0 + u * nw;
               s[u] = q < nodes ? list1[q] * gs + h * 32 + lane : n;
               v[u] = s[u] < n ? key_of(__ldcg(a.dist + s[u])) : -1;
+              if (ties && v[u] >= tau && a.orig[s[u]] >= cut) v[u] = -1;
             }
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
@@ -465,6 +470,23 @@ __global__ void __launch_bounds__(MM_THREADS, 1) k_maxmin_grid(MaxminArgs a) {
       __syncthreads();
       const int nc = nodes <= LIST_MAX ? rd_cands : CAND_MAX + 1;
       __syncthreads();
+      if (ties && nodes <= LIST_MAX) {
+        // equal distances go by index, so the lowest of them are the next steps
+        // (none below lo, too many below hi)
+        if (nc > CAND_MAX) {
+          hi = cut;
+          cut = lo + max(CAND_MAX, (int)((hi - lo) * (0.75 * CAND_MAX / nc)));
+          continue;
+        }
+        if (nc == 0) {
+          lo = cut;
+          cut = hi <= n ? lo + max(CAND_MAX, (hi - lo) / 2) : lo > n / 4 ? n : 4 * lo;
+          continue;
+        }
+        if (cut == n) ties = false;
+        if (nc < CAND_MAX / 4) cut = cut > n / 2 ? n : 2 * cut;
+        break;
+      }
       if (nc <= CAND_MAX) {
         // the next round's range of distances: about 3/4 of the candidates there is room for
         ratio = fmax(0.5, 1.0 - (1.0 - now) * fmin(1.5, 0.75 * CAND_MAX / nc));
@@ -472,9 +494,15 @@ __global__ void __launch_bounds__(MM_THREADS, 1) k_maxmin_grid(MaxminArgs a) {
       }
       now = 1.0 - (nc < 4 * CAND_MAX ? 0.5 : 0.125) * (1.0 - now);
       if (now > 1.0 - 1e-9) {  // more than CAND_MAX points share the maximum, or nearly: that may last for a while
-        singles = t + wait;
-        wait *= 2;
-        single = true;
+        ties = nodes <= LIST_MAX;
+        if (ties) {
+          cut = max(CAND_MAX, (int)(n * (0.75 * CAND_MAX / nc)));
+          now = ratio;  // for when the ties are through
+        } else {
+          singles = t + wait;
+          wait *= 2;
+          single = true;
+        }
       }
     }
     if (!single) {
