@@ -284,6 +284,10 @@ int lkg_set_graphs(int on);
 int lkg_oz7_mode_check(int mode, int M, int N, int K, const double* A, const double* B, int S, double* C,
                        int* where_out);
 
+/* No counterpart in the reference: the square roots and their reciprocals that the Cholesky's diagonal blocks take of n
+ * pivots x, beside CUDA's: out (4 n) = root, 1 / root, sqrt(x), 1 / sqrt(x) rounded to nearest.  0, or -1. */
+int lkg_pivot_roots_check(int n, const double* x, double* out);
+
 /* ------------------------------------------------------------- NestedKriging -------------------------------------- */
 /* libkriging_c.h:394-455 lk_nested_kriging_* (NestedKriging.hpp:63-105): partition (kmeans | random), submodel
  * fits, common prior, aggregation PoE | gPoE | BCM | rBCM | NK.  warping must be empty (n_warping = 0): WarpKriging

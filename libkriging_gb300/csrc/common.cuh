@@ -71,6 +71,25 @@ void launch_chained(bool chained, void (*kernel)(KA...), dim3 grid, dim3 block, 
   LKG_CUDA(cudaLaunchKernelEx(&cfg, kernel, static_cast<KA>(args)...));
 }
 
+// x 2^k for a normal x and result: an integer operation (an FP64 product takes an issue slot of the scarce pipe)
+__device__ __forceinline__ double times_pow2(double x, int k) {
+  return __hiloint2double(__double2hiint(x) + k * 0x00100000, __double2loint(x));
+}
+
+// 1 / sqrt(x) as FP32 gives it, for 2^-99 <= x < 2^99 (rsqrt_seed_range, read off the bits): the conversions, to nearest
+// even, are integer operations
+__device__ __forceinline__ bool rsqrt_seed_range(double x) {
+  const int hi = __double2hiint(x);
+  return hi >= 0x39C00000 && hi < 0x46200000;
+}
+__device__ __forceinline__ double rsqrt_seed(double x) {
+  constexpr unsigned long long kBias = 896ull << 52;  // FP64 exponent bias minus FP32's
+  unsigned long long xb = (unsigned long long)__double_as_longlong(x) - kBias;
+  xb += 0x0FFFFFFFull + ((xb >> 29) & 1ull);
+  const float seed = rsqrtf(__int_as_float((int)(xb >> 29)));
+  return __longlong_as_double((long long)(((unsigned long long)(unsigned)__float_as_int(seed) << 29) + kBias));
+}
+
 // ---------------------------------------------------------------------------------------------------------------
 // device covariance functions.  dx is X_j - X_i (sign irrelevant for Cov and DlnCovDtheta)
 // ---------------------------------------------------------------------------------------------------------------

@@ -6,9 +6,13 @@
 //   solve(trimatl(L), B), solve(trimatu(L'), B) -> trsm_lower_left[_t] (blocked, uses the diagonal-block inverses)
 #include "dense_fp64.cuh"
 
+#include <stdexcept>
+
 #include "stats.hpp"
 
 namespace lkg {
+
+void set_last_error(const char* msg);
 
 namespace {
 
@@ -201,25 +205,40 @@ __device__ __forceinline__ void tri_index(int e, int& r, int& c) {
   c = e - r * (r + 1) / 2;
 }
 
-// root = sqrt(x) and rroot = 1 / root of a pivot, rounded as sqrt and the reciprocal round them: the hardware's 20-bit
-// approximation of 1 / sqrt(x), one third-order step (e^3 < 2^-56), and one correction step each; a chain of 10 operations
-// (640 clocks) instead of the library's two routines (990).  Outside the range where the approximation is a normal
-// number, the library's operations.  (Stopping at the uncorrected 1 / sqrt(x) is 8 us a block faster, but moves the last
-// bit of most entries, and with it which duplicate points need a numerical nugget.)
+// root = sqrt(x) and rroot = 1 / root of a pivot.  From an FP32 seed y of 1 / sqrt(x) (relative error below 2^-21.9), one
+// step of Goldschmidt's coupled iteration (Ercegovac, Imbert, Matula, Muller, Wei, "Improving Goldschmidt division, square
+// root, and square root reciprocal", IEEE Trans. Computers 49, 2000): g -> sqrt(x) and h -> 1 / (2 sqrt(x)), both to
+// 2^-43, then the residual corrections of Markstein, "Computation of elementary functions on the IBM RISC System/6000
+// processor" (IBM J. Res. Dev. 34, 1990): g + (x - g^2) h, within 2^-86 of sqrt(x) before its rounding, and twice
+// y + (1 - root y) y, whose second step starts within a unit in the last place and so rounds 1 / root correctly unless
+// the significand of root is all ones (then one unit below).  10 operations; the library's two routines take 990 clocks.
+// Outside 2^-99 .. 2^99 the library's operations.  (Stopping at an uncorrected 1 / sqrt(x) moves the last bit of most
+// entries, and with it which duplicate points need a numerical nugget.)
 __device__ __forceinline__ void pivot_roots(double x, double& root, double& rroot) {
-  const int hi = __double2hiint(x);
-  if (hi < 0x02000000 || hi >= 0x7E000000) {
+  if (!rsqrt_seed_range(x)) {
     root = sqrt(x);
     rroot = __drcp_rn(root);
     return;
   }
-  double r;
-  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
-  const double e = fma(-(x * r), r, 1.0);
-  const double y = fma(r * e, fma(e, 0.375, 0.5), r);
-  const double q = x * y;
-  root = fma(fma(-q, q, x), 0.5 * y, q);
+  const double y0 = rsqrt_seed(x), h0 = times_pow2(y0, -1);
+  const double g0 = x * y0;
+  const double r = fma(-g0, h0, 0.5);
+  const double g = fma(g0, r, g0), h = fma(h0, r, h0);
+  root = fma(fma(-g, g, x), h, g);
+  double y = times_pow2(h, 1);
+  y = fma(fma(-root, y, 1.0), y, y);
   rroot = fma(fma(-root, y, 1.0), y, y);
+}
+
+__global__ void __launch_bounds__(256) k_pivot_roots(int n, const double* x, double* out) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  double root, rroot;
+  pivot_roots(x[i], root, rroot);
+  out[i] = root;
+  out[n + (int64_t)i] = rroot;
+  out[2 * (int64_t)n + i] = sqrt(x[i]);
+  out[3 * (int64_t)n + i] = __drcp_rn(sqrt(x[i]));
 }
 
 constexpr int PT = 256;           // threads of k_potrf_diag
@@ -843,6 +862,25 @@ void trsm_lower_left_t(const double* L, int64_t lda, int64_t mstride, int n, con
     trsv_launch<true>(L, lda, mstride, Dinv, dstride, B, ldb, bstride, n, k, (k + 1 < nblk) ? k + 1 : -1, r, nupd,
                       batch, st, chained);
   }
+}
+
+// Diagnostic entry: the roots that the diagonal blocks take, beside CUDA's (see the declaration in the C ABI header)
+extern "C" int lkg_pivot_roots_check(int n, const double* x, double* out) {
+  double* d = nullptr;
+  int rc = -1;
+  try {
+    if (n < 1 || n > (1 << 26)) throw std::invalid_argument("lkg_pivot_roots_check: n out of range");
+    LKG_CUDA(cudaMalloc(&d, sizeof(double) * 5 * (size_t)n));
+    LKG_CUDA(cudaMemcpy(d, x, sizeof(double) * n, cudaMemcpyHostToDevice));
+    k_pivot_roots<<<ceil_div(n, 256), 256>>>(n, d, d + n);
+    LKG_LAUNCH("k_pivot_roots");
+    LKG_CUDA(cudaMemcpy(out, d + n, sizeof(double) * 4 * (size_t)n, cudaMemcpyDeviceToHost));
+    rc = 0;
+  } catch (const std::exception& e) {
+    set_last_error(e.what());
+  }
+  cudaFree(d);
+  return rc;
 }
 
 }  // namespace lkg

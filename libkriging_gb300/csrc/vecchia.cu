@@ -109,16 +109,11 @@ __device__ __forceinline__ void tri_rc(int e, int& r, int& c) {
 // root and the reciprocal are taken directly.  The range is read off the bits, and the conversions (to nearest even) and
 // the factor -1/2 are integer operations: each would take an FP64 issue slot per pivot.
 __device__ __forceinline__ double pivot_rroot(double piv) {
-  const int hi = __double2hiint(piv);
-  if (hi < 0x39C00000 || hi >= 0x46200000) {  // within a factor of 2 of 1e-30 and 1e30, or beyond
+  if (!rsqrt_seed_range(piv)) {  // within a factor of 2 of 1e-30 and 1e30, or beyond
     if (!(piv >= 1e-30 && piv <= 1e30)) return 1.0 / sqrt(piv);
   }
-  constexpr unsigned long long kBias = 896ull << 52;  // FP64 exponent bias minus FP32's
-  unsigned long long pb = (unsigned long long)__double_as_longlong(piv) - kBias;
-  pb += 0x0FFFFFFFull + ((pb >> 29) & 1ull);
-  const float seed = rsqrtf(__int_as_float((int)(pb >> 29)));
-  double y = __longlong_as_double((long long)(((unsigned long long)(unsigned)__float_as_int(seed) << 29) + kBias));
-  const double h = __hiloint2double((hi - 0x00100000) | 0x80000000, __double2loint(piv));
+  double y = rsqrt_seed(piv);
+  const double h = -times_pow2(piv, -1);
   y = y * fma(h, y * y, 1.5);
   return y * fma(h, y * y, 1.5);
 }
