@@ -255,11 +255,11 @@ __global__ void __launch_bounds__(MM_THREADS, 1) k_maxmin_grid(MaxminArgs a) {
   // the range of cells that can hold a changing point
   __shared__ int st_snext, st_clo[MAXD], st_chi[MAXD], st_rows;
   __shared__ double st_xn[MAXD];
-  // a round's: threshold, radius, sizes; number of steps, and whether there will be no more
+  // a round's: threshold, radius, sizes; number of steps (-1 while they are being taken)
   __shared__ long long rd_max, rd_tau;
   __shared__ float rd_radius;
-  __shared__ int rd_nodes, rd_cands, rd_taken, rd_count[32];
-  __shared__ volatile int rd_done;
+  __shared__ int rd_nodes, rd_cands, rd_count[32];
+  __shared__ volatile int rd_taken;
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5, nw = MM_THREADS / 32;
   const int d = a.d, n = a.n, gs = a.g1, per = gs / 32;
 
@@ -405,7 +405,7 @@ __global__ void __launch_bounds__(MM_THREADS, 1) k_maxmin_grid(MaxminArgs a) {
           rd_radius = __double2float_ru(sqrt(mx) * (1.0 + 1e-6));
           rd_nodes = 0;
           rd_cands = 0;
-          rd_done = 0;
+          rd_taken = -1;
         }
       }
       __syncthreads();
@@ -675,10 +675,11 @@ __global__ void __launch_bounds__(MM_THREADS, 1) k_maxmin_grid(MaxminArgs a) {
             __syncwarp();
           }
         }
+        // the lanes' entries of taken[] before their number: __syncwarp orders them before lane 0's fence
+        __syncwarp();
         if (lane == 0) {
-          rd_taken = s;
           __threadfence_block();
-          rd_done = 1;
+          rd_taken = s;
         }
       } else {
         // (c) meanwhile the other warps: the neighbourhoods of the points taken, one warp per point, its cells' slots
@@ -701,12 +702,11 @@ __global__ void __launch_bounds__(MM_THREADS, 1) k_maxmin_grid(MaxminArgs a) {
         for (int unit = w - 1; unit < nc * share; unit += nw - 1) {
           const int q = unit / share, part = unit % share;
           int c = -1;
-          for (;;) {  // until step q is there, or will not come: warp 0 ends after at most nc steps
+          for (;;) {  // until step q is there, or the number of steps says that it will not come
             if (lane == 0) {
-              const int done = rd_done;
+              const int steps = rd_taken;
               __threadfence_block();
-              c = *(volatile int*)(taken + q);
-              if (c < 0 && done) c = -2;
+              c = steps >= 0 && q >= steps ? -2 : *(volatile int*)(taken + q);
             }
             c = __shfl_sync(FULL, c, 0);
             if (c != -1) break;
