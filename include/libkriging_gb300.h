@@ -284,6 +284,9 @@ int lkg_set_graphs(int on);
 int lkg_oz7_mode_check(int mode, int M, int N, int K, const double* A, const double* B, int S, double* C,
                        int* where_out);
 
+/* No counterpart in the reference: the order of lkg_vecchia_sets with a limit (nanoseconds) on the waits inside its
+ * kernel.  0, or -1 when a wait gave up (the message says so) or the arguments are bad; the device stays usable. */
+int lkg_vecchia_sets_wait_check(int n, int d, const double* X, long long wait_ns, int* order_out);
 /* No counterpart in the reference: the square roots and their reciprocals that the Cholesky's diagonal blocks take of n
  * pivots x, beside CUDA's: out (4 n) = root, 1 / root, sqrt(x), 1 / sqrt(x) rounded to nearest.  0, or -1. */
 int lkg_pivot_roots_check(int n, const double* x, double* out);

@@ -114,6 +114,7 @@ _SIGS = {
     "lkg_kriging_is_vecchia_light": (_i, [_vp]),
     "lkg_kriging_get_vecchia_sets": (_i, [_vp, _ip, _ip, _ip, _ip]),
     "lkg_vecchia_sets": (_i, [_i, _i, _dp, _i, _ip, _ip]),
+    "lkg_vecchia_sets_wait_check": (_i, [_i, _i, _dp, ctypes.c_longlong, _ip]),
     "lkg_kriging_predict_vecchia": (_i, [_vp, _dp, _i, _i, _i, _i, _dp, _dp]),
     "lkg_set_tensor_path": (_i, [_i]),
     "lkg_get_tensor_path": (_i, []),

@@ -600,6 +600,14 @@ int lkg_vecchia_sets(int n, int d, const double* X, int m, int* order_out, int* 
   });
 }
 
+int lkg_vecchia_sets_wait_check(int n, int d, const double* X, long long wait_ns, int* order_out) {
+  return run_entry<int>(-1, [&]() -> int {
+    if (n < 1 || d < 1 || wait_ns < 0) throw std::invalid_argument("lkg_vecchia_sets_wait_check: bad arguments");
+    lkg::vecchia_sets_gpu(n, d, X, 0, order_out, nullptr, (unsigned long long)wait_ns);
+    return 0;
+  });
+}
+
 void* lkg_vecchia_shard_new(const char* kernel, int n, int d, int p, const double* X, const double* y,
                             const double* F, const int* order, const int* nbr, int m, int t0, int t1) {
   return run_entry<void*>(nullptr, [&]() -> void* {

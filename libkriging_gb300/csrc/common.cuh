@@ -56,6 +56,13 @@ struct Unchained {
   int on_;
 };
 
+// wall clock of the device in nanoseconds, for waits that give up
+__device__ __forceinline__ uint64_t global_ns() {
+  uint64_t t;
+  asm volatile("mov.u64 %0, %globaltimer;\n" : "=l"(t));
+  return t;
+}
+
 template <class... KA, class... A>
 void launch_chained(bool chained, void (*kernel)(KA...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A... args) {
   cudaLaunchAttribute attr{};

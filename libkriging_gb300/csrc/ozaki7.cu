@@ -117,12 +117,6 @@ __device__ __forceinline__ bool mbar_poll(uint32_t m, uint32_t parity) {
   return ok != 0;
 }
 
-__device__ __forceinline__ uint64_t global_ns() {
-  uint64_t t;
-  asm volatile("mov.u64 %0, %globaltimer;\n" : "=l"(t));
-  return t;
-}
-
 __device__ __forceinline__ bool mbar_wait(uint32_t m, uint32_t parity) {
   if (mbar_poll(m, parity)) return true;
   const uint64_t t0 = global_ns();

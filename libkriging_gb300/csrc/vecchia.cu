@@ -1063,17 +1063,28 @@ __global__ void k_gather_points(int n, int d, const double* __restrict__ X, cons
 
 }  // namespace
 
-void vecchia_sets_gpu(int n, int d, const double* X, int m, int32_t* order, int32_t* nbr) {
+void vecchia_sets_gpu(int n, int d, const double* X, int m, int32_t* order, int32_t* nbr, unsigned long long wait_ns) {
   if (d > 8) throw std::invalid_argument("Vecchia sets on the GPU support d <= 8");
   if (m > VECCHIA_MAX_M) throw std::invalid_argument("Vecchia sets on the GPU support m <= 32");
   const int mm = std::min(m, n - 1);
-  cudaStream_t st;
-  LKG_CUDA(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
-  double* dX;
-  int32_t *dorder, *dnbr;
-  valloc(&dX, (size_t)n * d);
-  valloc(&dorder, n);
-  valloc(&dnbr, (size_t)n * std::max(m, 1));
+  struct Owned {  // released whichever way the call ends
+    cudaStream_t st = nullptr;
+    double* dX = nullptr;
+    int32_t *dorder = nullptr, *dnbr = nullptr;
+    ~Owned() {
+      cudaFree(dX);
+      cudaFree(dorder);
+      cudaFree(dnbr);
+      if (st) cudaStreamDestroy(st);
+    }
+  } own;
+  LKG_CUDA(cudaStreamCreateWithFlags(&own.st, cudaStreamNonBlocking));
+  valloc(&own.dX, (size_t)n * d);
+  valloc(&own.dorder, n);
+  valloc(&own.dnbr, (size_t)n * std::max(m, 1));
+  const cudaStream_t st = own.st;
+  double* dX = own.dX;
+  int32_t *dorder = own.dorder, *dnbr = own.dnbr;
   LKG_CUDA(cudaMemcpyAsync(dX, X, sizeof(double) * n * d, cudaMemcpyHostToDevice, st));
   // first point: closest to the centroid (index_min: first minimum), computed on the host in FP64 with the
   // reference's sequential sums (the host code is built without floating-point contraction)
@@ -1096,7 +1107,7 @@ void vecchia_sets_gpu(int n, int d, const double* X, int m, int32_t* order, int3
       first = i;
     }
   }
-  vecchia_sets_grid(n, d, X, dX, first, m, dorder, dnbr, st);
+  vecchia_sets_grid(n, d, X, dX, first, m, dorder, dnbr, st, wait_ns);
   LKG_CUDA(cudaMemcpyAsync(order, dorder, sizeof(int32_t) * n, cudaMemcpyDeviceToHost, st));
   std::vector<int32_t> tmp((size_t)n * std::max(mm, 1));
   if (mm > 0)
@@ -1104,10 +1115,6 @@ void vecchia_sets_gpu(int n, int d, const double* X, int m, int32_t* order, int3
   LKG_CUDA(cudaStreamSynchronize(st));
   for (int t = 0; t < n; ++t)
     for (int a = 0; a < m; ++a) nbr[(size_t)t * m + a] = (a < mm) ? tmp[(size_t)t * mm + a] : -1;
-  cudaFree(dX);
-  cudaFree(dorder);
-  cudaFree(dnbr);
-  cudaStreamDestroy(st);
 }
 
 void vecchia_predict_gpu(int kernel, int n, int d, const double* X, const double* resid, const double* theta, int q,

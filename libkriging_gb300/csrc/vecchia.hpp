@@ -70,13 +70,16 @@ std::string vecchia_failure_message();
 // GPU construction of the Vecchia sets, same definition as make_vecchia_sets: maxmin ordering from the point closest
 // to the centroid (argmin / argmax ties -> lowest index), then the min(m, t) nearest earlier-ordered points by
 // (squared distance, index).  X n x d column-major on the host; outputs host arrays order[n], nbr[n * m].
-void vecchia_sets_gpu(int n, int d, const double* X, int m, int32_t* order, int32_t* nbr);
+// wait_ns: limit of the waits inside the order's kernel, after which the call throws.
+constexpr unsigned long long SETS_WAIT_NS = 1000000000ull;
+void vecchia_sets_gpu(int n, int d, const double* X, int m, int32_t* order, int32_t* nbr,
+                      unsigned long long wait_ns = SETS_WAIT_NS);
 
 // The same sets from X on the device (n x d column-major; hX its host copy, for the grids' bounding box) with the
 // maxmin order started at `first`, on uniform grids (vecchia_grid.cu): dorder[n], dnbr[n x min(m, n - 1)].
 // Synchronises `st` before returning (its temporary buffers are freed).
 void vecchia_sets_grid(int n, int d, const double* hX, const double* dX, int first, int m, int32_t* dorder,
-                       int32_t* dnbr, cudaStream_t st);
+                       int32_t* dnbr, cudaStream_t st, unsigned long long wait_ns = SETS_WAIT_NS);
 
 // predictVecchia's local kriging (Kriging.cpp:950-1022) on the GPU: for each of the q points of Xq (q x d
 // column-major, normalised), the m nearest of the n observations X (n x d column-major) by (squared distance,

@@ -191,6 +191,8 @@ struct MaxminArgs {
   const int* slot_of;
   double* dist;  // read past L1 (rounds update it with atomics)
   int* order;
+  int* err;                    // set when a wait gave up; the launches after it do nothing
+  unsigned long long wait_ns;  // limit of a wait for a round's next step
   float eps[MAXD];  // bound on the error of a difference of two Xf in dimension k
 };
 
@@ -260,6 +262,7 @@ __global__ void __launch_bounds__(MM_THREADS, 1) k_maxmin_grid(MaxminArgs a) {
   __shared__ float rd_radius;
   __shared__ int rd_nodes, rd_cands, rd_count[32];
   __shared__ volatile int rd_taken;
+  __shared__ int rd_expired;
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5, nw = MM_THREADS / 32;
   const int d = a.d, n = a.n, gs = a.g1, per = gs / 32;
 
@@ -329,6 +332,8 @@ __global__ void __launch_bounds__(MM_THREADS, 1) k_maxmin_grid(MaxminArgs a) {
     }
   };
 
+  if (*a.err != 0) return;  // uniform: written only by an earlier launch's kernel here
+
   // rebuild the tree from the distances of the previous launch
   for (int g0 = w; g0 < a.ng1; g0 += 4 * nw) {
     int gi[4];
@@ -341,6 +346,7 @@ __global__ void __launch_bounds__(MM_THREADS, 1) k_maxmin_grid(MaxminArgs a) {
   if (tid == 0) {
     nlist1 = 0;
     overflow = 0;
+    rd_expired = 0;
   }
   __syncthreads();
   for (int gidx = w; gidx < a.ng2; gidx += nw) reduce_l2(gidx);
@@ -702,11 +708,20 @@ __global__ void __launch_bounds__(MM_THREADS, 1) k_maxmin_grid(MaxminArgs a) {
         for (int unit = w - 1; unit < nc * share; unit += nw - 1) {
           const int q = unit / share, part = unit % share;
           int c = -1;
+          unsigned long long since = 0;
           for (;;) {  // until step q is there, or the number of steps says that it will not come
             if (lane == 0) {
               const int steps = rd_taken;
               __threadfence_block();
               c = steps >= 0 && q >= steps ? -2 : *(volatile int*)(taken + q);
+              if (c == -1) {
+                const unsigned long long now = global_ns();
+                if (since == 0) since = now;
+                if (now - since >= a.wait_ns) {
+                  rd_expired = 1;
+                  c = -3;
+                }
+              }
             }
             c = __shfl_sync(FULL, c, 0);
             if (c != -1) break;
@@ -788,6 +803,10 @@ __global__ void __launch_bounds__(MM_THREADS, 1) k_maxmin_grid(MaxminArgs a) {
         drain(qn);
       }
       __syncthreads();
+      if (rd_expired) {
+        if (tid == 0) *a.err = 1;
+        return;
+      }
       t += rd_taken;
       refresh_tree();
       continue;
@@ -1069,7 +1088,7 @@ void grid_sort(int np, const double* P, const GridDesc& g, int* cell, int* cell_
 }  // namespace
 
 void vecchia_sets_grid(int n, int d, const double* hX, const double* dX, int first, int m, int32_t* dorder,
-                       int32_t* dnbr, cudaStream_t st) {
+                       int32_t* dnbr, cudaStream_t st, unsigned long long wait_ns) {
   if (d < 1 || d > MAXD) throw std::invalid_argument("Vecchia sets on the GPU support 1 <= d <= 8");
   if (m > VECCHIA_MAX_M) throw std::invalid_argument("Vecchia sets on the GPU support m <= 32");
   // bounding box of the points (the grids' extent)
@@ -1081,7 +1100,8 @@ void vecchia_sets_grid(int n, int d, const double* hX, const double* dX, int fir
     }
   DevBuf<double> Xp((size_t)n * d), Xs((size_t)n * d), dist(n);
   DevBuf<float> Xf((size_t)n * d);
-  DevBuf<int> cell(n), perm(n), orig(n), slot_of(n);
+  DevBuf<int> cell(n), perm(n), orig(n), slot_of(n), err(1);
+  LKG_CUDA(cudaMemsetAsync(err.p, 0, sizeof(int), st));
   k_points_major<<<ceil_div(n, 256), 256, 0, st>>>(n, d, dX, nullptr, Xp.p, nullptr);
   LKG_LAUNCH("k_points_major");
 
@@ -1112,6 +1132,8 @@ void vecchia_sets_grid(int n, int d, const double* hX, const double* dX, int fir
     a.slot_of = slot_of.p;
     a.dist = dist.p;
     a.order = dorder;
+    a.err = err.p;
+    a.wait_ns = wait_ns;
     // FP32 squares of differences between 1e-18 and 1e18 stay in range; other boxes take every step alone
     a.singles = ROUND_FROM;
     for (int k = 0; k < d; ++k)
@@ -1127,7 +1149,11 @@ void vecchia_sets_grid(int n, int d, const double* hX, const double* dX, int fir
       kernel<<<1, MM_THREADS, smem, st>>>(a);
       LKG_LAUNCH("k_maxmin_grid");
     }
+    int expired = 0;
+    LKG_CUDA(cudaMemcpyAsync(&expired, err.p, sizeof(int), cudaMemcpyDeviceToHost, st));
     LKG_CUDA(cudaStreamSynchronize(st));  // cstart / cursor are freed at scope exit
+    // the order is incomplete then, and nothing may read it
+    if (expired) throw std::runtime_error("Vecchia sets: a round of the maxmin order did not complete (timed out)");
   }
   if (m <= 0 || n < 2) return;
   // ---- neighbour sets (rows of m = min(m, n - 1) entries): ordered coordinates, then one grid per prefix of
