@@ -533,13 +533,14 @@ __global__ void __launch_bounds__(MM_THREADS, 1) k_maxmin_grid(MaxminArgs a) {
         }
       }
       __syncthreads();
-      // FP32 bounds: with E the length of the error bounds of the differences and d2 the FP32 squared distance, the true
-      // one is at least (sqrt(d2) - E)^2 and at most (sqrt(d2) + E)^2, up to 2^-19 for the rounding of at most 8 terms
-      // and of the square roots
+      // FP32 bounds: with E no less than the length of the error bounds of the differences and d2 the FP32 squared distance,
+      // the true one is at least (sqrt(d2) - E)^2 and at most (sqrt(d2) + E)^2, up to 2^-19 for the rounding of at most 8
+      // terms and of the square roots.  E is the sum of the bounds: their squares would underflow to zero where all sides
+      // of the box are below 1e-16, and pairs would pass as clear that are not.
       float E = 0.0f;
 #pragma unroll
-      for (int k = 0; k < DM; ++k) E = k < d ? fmaf(a.eps[k], a.eps[k], E) : E;
-      E = sqrtf(E) * (1.0f + 0x1p-20f);
+      for (int k = 0; k < DM; ++k) E += k < d ? a.eps[k] : 0.0f;
+      E *= 1.0f + 0x1p-20f;
       if (tid < nc) {
         const int r = rank[tid], s = uslot[tid];
         skey[r] = ukey[tid];
