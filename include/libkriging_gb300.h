@@ -284,6 +284,10 @@ int lkg_set_graphs(int on);
 int lkg_oz7_mode_check(int mode, int M, int N, int K, const double* A, const double* B, int S, double* C,
                        int* where_out);
 
+/* No counterpart in the reference: leaves the engines of a Kriging model as a digit product does whose wait expired, so that
+ * the next evaluation or save of this model, and of no other, fails with that error, and the ones after it succeed.
+ * Returns 0, or -1 for a null handle. */
+int lkg_kriging_mark_digits_expired(void* ptr);
 /* No counterpart in the reference: the order of lkg_vecchia_sets with a limit (nanoseconds) on the waits inside its
  * kernel.  0, or -1 when a wait gave up (the message says so) or the arguments are bad; the device stays usable. */
 int lkg_vecchia_sets_wait_check(int n, int d, const double* X, long long wait_ns, int* order_out);

@@ -41,6 +41,7 @@ _SIGS = {
     "lkg_kriging_cov_mat": (_i, [_vp, _dp, _i, _i, _dp, _i, _i, _dp]),
     "lkg_kriging_get_F": (_i, [_vp, _dp, _ip, _ip]),
     "lkg_oz7_mode_check": (_i, [_i, _i, _i, _i, _dp, _dp, _i, _dp, _ip]),
+    "lkg_kriging_mark_digits_expired": (_i, [_vp]),
     "lkg_pivot_roots_check": (_i, [_i, _dp, _dp]),
     "lkg_kriging_log_likelihood_fun": (_i, [_vp, _dp, _i, _i, _i, _dp, _dp, _dp]),
     "lkg_kriging_log_likelihood": (_d, [_vp]),

@@ -510,6 +510,13 @@ int lkg_kriging_set_precision(void* ptr, int slices) {
   });
 }
 
+int lkg_kriging_mark_digits_expired(void* ptr) {
+  return run_entry<int>(-1, [&]() -> int {
+    K(ptr)->mark_digits_expired();
+    return 0;
+  });
+}
+
 int lkg_kriging_get_precision(void* ptr) {
   return run_entry<int>(-1, [&]() -> int {
     return K(ptr)->precision();

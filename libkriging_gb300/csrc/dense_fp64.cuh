@@ -54,6 +54,7 @@ struct MixedWorkspace {
   int digits = FP64_DIGITS;      // digits of the Cholesky's products (6 .. 8)
   int digits_inv = FP64_DIGITS;  // digits of the triangular inverse and W^T W, which feed only the gradient (5 .. 8)
   bool wide = true;              // 8-bit leading digits (ozaki7.cu)
+  int* err = nullptr;            // status words of the products (OZ7_ERR_WORDS)
   void* panel = nullptr;  // bf16 planes, oz7_plane_elems(n, 256, 8) per batch entry
   int* panel_exp = nullptr;
   void* rowblk = nullptr;  // bf16 planes, same size
@@ -80,10 +81,11 @@ void wtw_lower_mixed(const double* W, int64_t ldw, int64_t wstride, int n, doubl
 // C (n x n, ldc) = A B with A, B n x n column-major (lda, ldb), FP64_DIGITS digits, in chunks of ws.wk / 2 columns of A
 void gemm_square_digits(int n, const double* A, int64_t lda, const double* B, int64_t ldb, double* C, int64_t ldc,
                         const MixedWorkspace& ws, cudaStream_t st);
-// Bytes of scratch for trsm_lower_left_digits, and L X = B in place (B n x r column-major, ldb; one matrix)
+// Bytes of scratch for trsm_lower_left_digits, and L X = B in place (B n x r column-major, ldb; one matrix); err: status
+// words of the products (OZ7_ERR_WORDS)
 size_t trsm_digits_bytes(int n, int r);
 void trsm_lower_left_digits(const double* L, int64_t lda, int n, const double* Dinv, double* B, int64_t ldb, int r,
-                            void* scratch, cudaStream_t st);
+                            void* scratch, int* err, cudaStream_t st);
 // Whether the FP64 path runs its products over n x n factors as 8-digit products (else as DFMA tiles).
 bool digits_pay(int n);
 

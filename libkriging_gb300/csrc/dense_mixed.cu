@@ -47,9 +47,9 @@ void potrf_blocked_mixed7(double* A, int64_t lda, int64_t mstride, int n, double
                           const MixedWorkspace& ws, cudaStream_t st) {
   LKG_CUDA(cudaMemsetAsync(info, 0, sizeof(int) * batch, st));
   const int S = ws.digits;
-  Split7 P = oz7_buffer(ws.panel, ws.panel_exp, S, ws.n, OZ7_KB, OZ7_KB, ws.wide);
-  Split7 SA = oz7_buffer(ws.panel, ws.panel_exp, S, ws.n, NB, NB, ws.wide);
-  Split7 SD = oz7_buffer(ws.rowblk, ws.rowblk_exp, S, ws.n, NB, NB, ws.wide);
+  Split7 P = oz7_buffer(ws.panel, ws.panel_exp, S, ws.n, OZ7_KB, OZ7_KB, ws.err, ws.wide);
+  Split7 SA = oz7_buffer(ws.panel, ws.panel_exp, S, ws.n, NB, NB, ws.err, ws.wide);
+  Split7 SD = oz7_buffer(ws.rowblk, ws.rowblk_exp, S, ws.n, NB, NB, ws.err, ws.wide);
   const bool ahead = ws.side_stream && batch == 1;
   if (!ahead) {
     for (int K0 = 0; K0 < n; K0 += OZ7_KB) {
@@ -66,7 +66,7 @@ void potrf_blocked_mixed7(double* A, int64_t lda, int64_t mstride, int n, double
   }
   // the side stream's panel splits have their own buffer: the main stream's trailing update still reads P (the
   // Dinv splits in rowblk are used by one stream at a time)
-  Split7 SAs = oz7_buffer(ws.side, ws.side_exp, S, ws.n, NB, NB, ws.wide);
+  Split7 SAs = oz7_buffer(ws.side, ws.side_exp, S, ws.n, NB, NB, ws.err, ws.wide);
   const int rest_ctas = std::max(1, oz7_sm_count() - ws.side_ctas);
   factor_panel7(A, lda, mstride, n, 0, Dinv, info, batch, SA, SD, 0, st);
   for (int K0 = 0; K0 < n; K0 += OZ7_KB) {
@@ -126,10 +126,10 @@ void trtri_blocked_mixed7(const double* L, int64_t lda, int64_t mstride, int n, 
   const int64_t dstride = (int64_t)nblk * NB * NB;
   inverse_init(Dinv, n, W, ldw, wstride, batch, st);
   const int S = ws.digits_inv;
-  Split7 SL = oz7_buffer(ws.panel, ws.panel_exp, S, ws.n, OZ7_KB, OZ7_KB, ws.wide);
-  Split7 SR = oz7_buffer(ws.rowblk, ws.rowblk_exp, S, ws.n, OZ7_KB, OZ7_KB, ws.wide);
-  Split7 SA = oz7_buffer(ws.panel, ws.panel_exp, S, ws.n, NB, NB, ws.wide);
-  Split7 SB = oz7_buffer(ws.rowblk, ws.rowblk_exp, S, ws.n, NB, NB, ws.wide);
+  Split7 SL = oz7_buffer(ws.panel, ws.panel_exp, S, ws.n, OZ7_KB, OZ7_KB, ws.err, ws.wide);
+  Split7 SR = oz7_buffer(ws.rowblk, ws.rowblk_exp, S, ws.n, OZ7_KB, OZ7_KB, ws.err, ws.wide);
+  Split7 SA = oz7_buffer(ws.panel, ws.panel_exp, S, ws.n, NB, NB, ws.err, ws.wide);
+  Split7 SB = oz7_buffer(ws.rowblk, ws.rowblk_exp, S, ws.n, NB, NB, ws.err, ws.wide);
   for (int K0 = 0; K0 < n; K0 += OZ7_KB) {
     const int Wd = std::min(OZ7_KB, n - K0);
     trtri_block7(L, lda, mstride, n, K0, Wd, Dinv, dstride, W, ldw, wstride, batch, SA, SB, st);
@@ -148,7 +148,7 @@ void trtri_blocked_mixed7(const double* L, int64_t lda, int64_t mstride, int n, 
 // each, whatever the chunk, so the result does not depend on ws.wk.
 void wtw_lower_mixed7(const double* W, int64_t ldw, int64_t wstride, int n, double* C, int64_t ldc, int64_t cstride,
                       int batch, const MixedWorkspace& ws, cudaStream_t st) {
-  Split7 SW = oz7_buffer(ws.wchunk, ws.wchunk_exp, ws.digits_inv, ws.n, ws.wk, OZ7_KB, ws.wide);
+  Split7 SW = oz7_buffer(ws.wchunk, ws.wchunk_exp, ws.digits_inv, ws.n, ws.wk, OZ7_KB, ws.err, ws.wide);
   for (int c0 = 0; c0 < n; c0 += ws.wk) {
     const int kc = std::min(ws.wk, n - c0);
     oz7_split(c0 + kc, kc, W + c0, ldw, 1, wstride, batch, SW, st);  // rows of the split = columns of W
@@ -177,9 +177,9 @@ void gemm_square_digits(int n, const double* A, int64_t lda, const double* B, in
                         const MixedWorkspace& ws, cudaStream_t st) {
   const int S = FP64_DIGITS, kh = ws.wk / 2 / OZ7_KB * OZ7_KB;  // half of the chunk buffer for each operand
   __nv_bfloat16* planes = static_cast<__nv_bfloat16*>(ws.wchunk);
-  Split7 SA = oz7_buffer(planes, ws.wchunk_exp, S, ws.n, kh, OZ7_KB, true);
+  Split7 SA = oz7_buffer(planes, ws.wchunk_exp, S, ws.n, kh, OZ7_KB, ws.err, true);
   Split7 SB = oz7_buffer(planes + oz7_plane_elems(ws.n, kh, S), ws.wchunk_exp + oz7_exp_elems(ws.n, kh, OZ7_KB), S, ws.n,
-                         kh, OZ7_KB, true);
+                         kh, OZ7_KB, ws.err, true);
   for (int c0 = 0; c0 < n; c0 += kh) {
     const int kc = std::min(kh, n - c0);
     oz7_split2(n, kc, A + (int64_t)c0 * lda, 1, lda, 0, SA, n, kc, B + c0, ldb, 1, 0, SB, 1, st, c0 > 0);
@@ -200,7 +200,7 @@ size_t trsm_digits_bytes(int n, int r) {
 // below.  A column's result depends on that column alone (its own exponents), so predictions do not depend on how the
 // points are grouped.
 void trsm_lower_left_digits(const double* L, int64_t lda, int n, const double* Dinv, double* B, int64_t ldb, int r,
-                            void* scratch, cudaStream_t st) {
+                            void* scratch, int* err, cudaStream_t st) {
   const int S = FP64_DIGITS;
   char* at = static_cast<char*>(scratch);
   void* lp = at;
@@ -209,9 +209,9 @@ void trsm_lower_left_digits(const double* L, int64_t lda, int n, const double* D
   at += oz7_plane_elems(r, OZ7_KB, S) * sizeof(__nv_bfloat16);
   int* le = reinterpret_cast<int*>(at);
   int* xe = le + (oz7_exp_elems(n, OZ7_KB, NB) * sizeof(int) + 255) / 256 * 64;
-  Split7 SL = oz7_buffer(lp, le, S, n, OZ7_KB, OZ7_KB, true);
-  Split7 SX = oz7_buffer(xp, xe, S, r, OZ7_KB, OZ7_KB, true);
-  Split7 sl = oz7_buffer(lp, le, S, n, NB, NB, true), sx = oz7_buffer(xp, xe, S, r, NB, NB, true);
+  Split7 SL = oz7_buffer(lp, le, S, n, OZ7_KB, OZ7_KB, err, true);
+  Split7 SX = oz7_buffer(xp, xe, S, r, OZ7_KB, OZ7_KB, err, true);
+  Split7 sl = oz7_buffer(lp, le, S, n, NB, NB, err, true), sx = oz7_buffer(xp, xe, S, r, NB, NB, err, true);
   for (int K0 = 0; K0 < n; K0 += OZ7_KB) {
     const int Wd = std::min(OZ7_KB, n - K0);
     for (int k0 = K0; k0 < K0 + Wd; k0 += NB) {

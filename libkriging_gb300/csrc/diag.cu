@@ -164,10 +164,12 @@ extern "C" int lkg_ozaki_gemm_check(int M, int N, int K, const double* A, const 
   // C = A * B^T with A (M x K) and B (N x K) column-major, computed by the split-bf16 tensor-core path
   double *dA = nullptr, *dB = nullptr, *dC = nullptr;
   void *pa = nullptr, *pb = nullptr;
-  int *ea = nullptr, *eb = nullptr;
+  int *ea = nullptr, *eb = nullptr, *err = nullptr;
   int rc = -1;
   lkg::set_last_error("");
   try {
+    LKG_CUDA(cudaMalloc(&err, lkg::OZ7_ERR_WORDS * sizeof(int)));
+    LKG_CUDA(cudaMemset(err, 0, lkg::OZ7_ERR_WORDS * sizeof(int)));
     LKG_CUDA(cudaMalloc(&dA, sizeof(double) * M * K));
     LKG_CUDA(cudaMalloc(&dB, sizeof(double) * N * K));
     LKG_CUDA(cudaMalloc(&dC, sizeof(double) * M * N));
@@ -180,13 +182,16 @@ extern "C" int lkg_ozaki_gemm_check(int M, int N, int K, const double* A, const 
     LKG_CUDA(cudaMalloc(&pb, lkg::oz7_plane_elems(N, K, slices) * 2));
     LKG_CUDA(cudaMalloc(&ea, lkg::oz7_exp_elems(M, K, kb) * sizeof(int)));
     LKG_CUDA(cudaMalloc(&eb, lkg::oz7_exp_elems(N, K, kb) * sizeof(int)));
-    lkg::Split7 sa = lkg::oz7_buffer(pa, ea, slices, M, K, kb), sb = lkg::oz7_buffer(pb, eb, slices, N, K, kb);
+    lkg::Split7 sa = lkg::oz7_buffer(pa, ea, slices, M, K, kb, err),
+                sb = lkg::oz7_buffer(pb, eb, slices, N, K, kb, err);
     lkg::oz7_split(M, K, dA, 1, M, 0, 1, sa, 0);
     lkg::oz7_split(N, K, dB, 1, N, 0, 1, sb, 0);
     lkg::oz7_gemm(M, N, 0, sa.nblk, 1.0, sa, sb, 0.0, dC, M, 0, 1, false, 0);
     LKG_CUDA(cudaDeviceSynchronize());
     LKG_CUDA(cudaMemcpy(C, dC, sizeof(double) * M * N, cudaMemcpyDeviceToHost));
-    rc = lkg::oz7_error_and_reset() ? -1 : 0;
+    int expired = 0;
+    LKG_CUDA(cudaMemcpy(&expired, err, sizeof(int), cudaMemcpyDeviceToHost));
+    rc = expired ? -1 : 0;
   } catch (const std::exception& e) {
     lkg::set_last_error(e.what());
     rc = -1;
@@ -199,5 +204,6 @@ extern "C" int lkg_ozaki_gemm_check(int M, int N, int K, const double* A, const 
   cudaFree(pb);
   cudaFree(ea);
   cudaFree(eb);
+  cudaFree(err);
   return rc;
 }

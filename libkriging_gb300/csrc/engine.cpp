@@ -70,6 +70,8 @@ struct Timer {
   }
 };
 
+constexpr int kStatWords = (OZ7_ERR_WORDS + 15) / 16 * 16;
+
 template <typename P>
 void dalloc(P** p, size_t count) {
   LKG_CUDA(cudaMalloc((void**)p, sizeof(P) * std::max<size_t>(count, 1)));
@@ -142,8 +144,10 @@ Engine::Engine(int kernel, int n, int d, int p, int ndesign, const double* X, co
   dalloc(&drstar_, (size_t)std::max(p * p, 1) * cap_);
   dalloc(&dsse_, cap_);
   dalloc(&dadj_, (size_t)adjoint_nacc(d) * cap_);
-  dalloc(&dinfo_, cap_);
-  dalloc(&dgls_info_, cap_);
+  dalloc(&dstat_, (size_t)kStatWords + 2 * cap_);
+  dinfo_ = dstat_ + kStatWords;
+  dgls_info_ = dinfo_ + cap_;
+  LKG_CUDA(cudaMemsetAsync(dstat_, 0, sizeof(int) * kStatWords, st_));
   LKG_CUDA(cudaStreamSynchronize(st_));
 }
 
@@ -152,8 +156,7 @@ Engine::~Engine() {
   for (double* p : {dX_, dY_, dF_, dA_, dDinv_, dW_, dRinv_, dFY_, dEstar_, dxv_, dtheta_, dfactor_, ddiag_, dgram_,
                     dbeta_, drstar_, dsse_, dpart_, dadj_, dvec_, dcol_, dloo_m_, dloo_at_, dloo_vec_, dWp_})
     if (p) cudaFree(p);
-  if (dinfo_) cudaFree(dinfo_);
-  if (dgls_info_) cudaFree(dgls_info_);
+  if (dstat_) cudaFree(dstat_);
   if (dXe_) cudaFree(dXe_);
   if (dnv_) cudaFree(dnv_);
   for (void* p : {dpanel_, drowblk_, dwchunk_, dside_})
@@ -328,6 +331,7 @@ MixedWorkspace Engine::digit_workspace(int batch, bool long_products) {
     mw.digits_inv = std::min(8, std::max(5, std::max(4, slices_ - 2)));
     mw.wide = false;
   }
+  mw.err = dstat_;
   mw.n = n_;
   mw.panel = dpanel_;
   mw.panel_exp = dpanel_exp_;
@@ -345,6 +349,19 @@ MixedWorkspace Engine::digit_workspace(int batch, bool long_products) {
     mw.side_ctas = lookahead_ctas();
   }
   return mw;
+}
+
+void Engine::check_digits(int expired) {
+  if (!expired) return;
+  LKG_CUDA(cudaMemsetAsync(dstat_, 0, sizeof(int) * kStatWords, st_));
+  LKG_CUDA(cudaStreamSynchronize(st_));
+  throw std::runtime_error("a tensor-core digit product did not complete (timed out)");
+}
+
+void Engine::mark_digits_expired() {
+  const int one = 1;
+  LKG_CUDA(cudaMemcpyAsync(dstat_, &one, sizeof(int), cudaMemcpyHostToDevice, st_));
+  LKG_CUDA(cudaStreamSynchronize(st_));
 }
 
 void Engine::ensure_grad_buffers() {
@@ -390,9 +407,10 @@ const double* Engine::factor_inverse() {
 
 size_t Engine::solve_scratch_bytes(int r) const { return r > 16 && digits_pay(n_) ? trsm_digits_bytes(n_, r) : 0; }
 
-void Engine::solve_lower_inplace(int b, double* dB, int64_t ldb, int r, void* scratch) const {
+void Engine::solve_lower_inplace(int b, double* dB, int64_t ldb, int r, void* scratch, int* err) const {
   if (r > 16 && digits_pay(n_))
-    trsm_lower_left_digits(dA_ + (size_t)b * mstride_, lda_, n_, dDinv_ + (size_t)b * dstride_, dB, ldb, r, scratch, st_);
+    trsm_lower_left_digits(dA_ + (size_t)b * mstride_, lda_, n_, dDinv_ + (size_t)b * dstride_, dB, ldb, r, scratch, err,
+                           st_);
   else
     trsm_lower_left(dA_ + (size_t)b * mstride_, lda_, mstride_, n_, dDinv_ + (size_t)b * dstride_, dB, ldb, 0, r, 1,
                     st_);
@@ -564,7 +582,8 @@ void Engine::evaluate(int batch, const double* thetas, const double* factors, bo
   const bool rcond_check = cfg.chol_rcond_check && !plain_chol_;
   std::vector<int> inc(batch, 0);
   std::vector<char> dead(batch, 0);
-  std::vector<int> info(batch, 0);
+  std::vector<int> stat(kStatWords + batch, 0);  // the products' status, then info
+  int* const info = stat.data() + kStatWords;
   std::vector<double> rc2(batch, -1.0);
   bool digit = digit_path();  // digit products, else DFMA tiles
   MixedWorkspace mw;
@@ -643,8 +662,9 @@ void Engine::evaluate(int batch, const double* thetas, const double* factors, bo
         LKG_CUDA(cudaMemcpyAsync(cl.data(), dcol_, sizeof(double) * n * batch, cudaMemcpyDeviceToHost, st_));
         LKG_CUDA(cudaMemcpyAsync(cw.data(), dvec_, sizeof(double) * n * batch, cudaMemcpyDeviceToHost, st_));
       }
-      LKG_CUDA(cudaMemcpyAsync(info.data(), dinfo_, sizeof(int) * batch, cudaMemcpyDeviceToHost, st_));
+      LKG_CUDA(cudaMemcpyAsync(stat.data(), dstat_, sizeof(int) * stat.size(), cudaMemcpyDeviceToHost, st_));
       LKG_CUDA(cudaStreamSynchronize(st_));
+      check_digits(stat[0]);  // before the retry rules look at a factor that is not one
     };
     if (slices_ > 0 && !retreated) {
       factor_to_host(false);  // a failed factor is redone: its inverse is not worth starting
@@ -774,12 +794,13 @@ void Engine::evaluate(int batch, const double* thetas, const double* factors, bo
 
   // ---- results to host ----
   std::vector<double> gram((size_t)gram_stride_ * batch), sse(batch), beta((size_t)std::max(p, 1) * batch);
-  std::vector<int> gls(batch);
+  std::vector<int> stat_end(kStatWords + cap_ + batch);  // the products' status, info, the GLS's info
+  const int* const gls = stat_end.data() + kStatWords + cap_;
   std::vector<double> adj;
   LKG_CUDA(cudaMemcpyAsync(gram.data(), dgram_, sizeof(double) * gram.size(), cudaMemcpyDeviceToHost, st_));
   LKG_CUDA(cudaMemcpyAsync(sse.data(), dsse_, sizeof(double) * batch, cudaMemcpyDeviceToHost, st_));
   LKG_CUDA(cudaMemcpyAsync(beta.data(), dbeta_, sizeof(double) * beta.size(), cudaMemcpyDeviceToHost, st_));
-  LKG_CUDA(cudaMemcpyAsync(gls.data(), dgls_info_, sizeof(int) * batch, cudaMemcpyDeviceToHost, st_));
+  LKG_CUDA(cudaMemcpyAsync(stat_end.data(), dstat_, sizeof(int) * stat_end.size(), cudaMemcpyDeviceToHost, st_));
   std::vector<double> rstar((size_t)p * p * batch);
   if (p > 0)
     LKG_CUDA(cudaMemcpyAsync(rstar.data(), drstar_, sizeof(double) * rstar.size(), cudaMemcpyDeviceToHost, st_));
@@ -790,8 +811,7 @@ void Engine::evaluate(int batch, const double* thetas, const double* factors, bo
     LKG_CUDA(cudaMemcpyAsync(adj.data(), dadj_, sizeof(double) * adj.size(), cudaMemcpyDeviceToHost, st_));
   }
   LKG_CUDA(cudaStreamSynchronize(st_));
-  if ((digit || slices_ > 0) && oz7_error_and_reset())
-    throw std::runtime_error("a tensor-core digit product did not complete (timed out)");
+  check_digits(stat_end[0]);
   for (int b = 0; b < batch; ++b) {
     EvalOut& o = out[b];
     if (o.status == 0 && gls[b] != 0) {
@@ -897,10 +917,11 @@ void Engine::leave_one_out(int batch, const double* thetas, const double* factor
     }
     const int nvec = want_grad ? 2 * d + 2 : 2;
     std::vector<double> hv((size_t)n * nvec);
+    int expired = 0;
     LKG_CUDA(cudaMemcpyAsync(hv.data(), dloo_vec_, sizeof(double) * hv.size(), cudaMemcpyDeviceToHost, st_));
+    if (digit) LKG_CUDA(cudaMemcpyAsync(&expired, dstat_, sizeof(int), cudaMemcpyDeviceToHost, st_));
     LKG_CUDA(cudaStreamSynchronize(st_));
-    if (digit && oz7_error_and_reset())
-      throw std::runtime_error("leave-one-out: a tensor-core digit product did not complete (timed out)");
+    check_digits(expired);
     // host assembly (Kriging.cpp:411-465), n-vectors only
     const double* dg = hv.data();
     const double* by = hv.data() + n;
@@ -1091,9 +1112,12 @@ void Engine::model_matrices(const double* theta, double factor, std::vector<doub
       wtw_lower(dW_, lda_, mstride_, n, dRinv_, lda_, mstride_, 1, st_);
     }
     Rinv->assign((size_t)n * n, 0.0);
+    int expired = 0;
+    LKG_CUDA(cudaMemcpyAsync(&expired, dstat_, sizeof(int), cudaMemcpyDeviceToHost, st_));
     LKG_CUDA(cudaMemcpy2DAsync(Rinv->data(), sizeof(double) * n, dRinv_, sizeof(double) * lda_, sizeof(double) * n,
                                n, cudaMemcpyDeviceToHost, st_));
     LKG_CUDA(cudaStreamSynchronize(st_));
+    check_digits(expired);
     mirror(*Rinv);
   }
 }

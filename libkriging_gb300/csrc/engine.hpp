@@ -122,6 +122,8 @@ class Engine {
   void set_slices(int s);
   // several engines evaluate at the same time: their kernels fill the gaps of one another's, so an evaluation keeps to one
   // stream and chains no kernels (24 experts of 100 to 2500 rows: 19.5 ms, 21.4 chained)
+  // leaves the status words as a digit product does whose wait expired: the next evaluation reports it
+  void mark_digits_expired();
   void set_alone(bool alone) { alone_ = alone; }
   bool lookahead_enabled() const;
   int lookahead_ctas() const;
@@ -137,8 +139,9 @@ class Engine {
   int64_t mstride() const { return mstride_; }
   const double* dFY(int b = 0) const { return dFY_ + (size_t)b * fystride_; }
   const double* dEstar(int b = 0) const { return dEstar_ + (size_t)b * n_; }
-  // solve L Z = B in place for entry b (B device, n x r, ldb); scratch: solve_scratch_bytes(r) bytes
-  void solve_lower_inplace(int b, double* dB, int64_t ldb, int r, void* scratch) const;
+  // solve L Z = B in place for entry b (B device, n x r, ldb); scratch: solve_scratch_bytes(r) bytes; err: the
+  // caller's status words (OZ7_ERR_WORDS, ozaki7.cuh)
+  void solve_lower_inplace(int b, double* dB, int64_t ldb, int r, void* scratch, int* err) const;
   size_t solve_scratch_bytes(int r) const;
   // W = L^-1 of the (single-matrix) factor, formed once per factor on the FP64 path and kept for predictions whose
   // solves run as digit products (W R_on)
@@ -156,6 +159,8 @@ class Engine {
   // (re)allocates the digit buffers and describes them; long_products: also those of the inverse's W^T W and of
   // leave-one-out's square products
   MixedWorkspace digit_workspace(int batch, bool long_products);
+  // throws when a digit product of this engine expired (word 0 of its status words, on the host), and clears the words
+  void check_digits(int expired);
   // rcond(L)^2 per entry, dtrcon('1') style estimate on each entry's first nvb[b] rows / columns
   void rcond_batch(int batch, std::vector<double>& rc2, const std::vector<int>& nvb);
   // the same estimate for the n x n lower factors at A (lda, mstride) with diagonal-block inverses Dinv
@@ -204,7 +209,9 @@ class Engine {
   double *dtheta_ = nullptr, *dfactor_ = nullptr, *ddiag_ = nullptr;
   double *dgram_ = nullptr, *dbeta_ = nullptr, *drstar_ = nullptr, *dsse_ = nullptr;
   double *dpart_ = nullptr, *dadj_ = nullptr, *dvec_ = nullptr, *dcol_ = nullptr;
-  int *dinfo_ = nullptr, *dgls_info_ = nullptr;
+  // one block, so that one copy brings them down: status words of this engine's digit products (dstat_), then per entry the
+  // factorisation's info and the GLS's
+  int *dstat_ = nullptr, *dinfo_ = nullptr, *dgls_info_ = nullptr;
   size_t part_size_ = 0;
   int gram_stride_ = 0;
 };

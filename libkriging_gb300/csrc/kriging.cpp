@@ -213,6 +213,11 @@ void Kriging::ensure_engine(int batch_cap) {
   m_eval->set_slices(m_slices);
 }
 
+void Kriging::mark_digits_expired() {
+  for (Engine* e : {m_eval.get(), m_model.get()})
+    if (e) e->mark_digits_expired();
+}
+
 void Kriging::set_precision(int slices) {
   if (slices != 0 && (slices < 4 || slices > 8))
     throw std::invalid_argument("set_precision: slices must be 0 (FP64) or 4..8");

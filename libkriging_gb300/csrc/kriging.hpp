@@ -149,6 +149,8 @@ class Kriging {
 
   // per-stage timings of the last logLikelihoodFun(..., bench=true) call (Bench keys of the reference)
   const std::map<std::string, double>& last_bench() const { return m_bench; }
+  // diagnostic: the model's engines as after a digit product whose wait expired
+  void mark_digits_expired();
   // total evaluations performed by the engine since construction (objective calls, batched entries counted once each)
   long long evaluations() const { return m_evals; }
   // GPU evaluation launches since construction: a batched round of a multistart fit counts once

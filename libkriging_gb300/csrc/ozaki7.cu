@@ -38,7 +38,7 @@
 //                 folds the S diagonals exactly (int32 pairs, two exact doubles, one rounded FP64 addition) and
 //                 updates C, then releases its accumulator set to the next block (18 warps leave 96 registers a
 //                 thread: a sub-partition holds 5 warps of its 16K registers)
-// All mbarrier waits are bounded; on expiry the CTA records an error (oz7_error_and_reset), drains what it issued and
+// All mbarrier waits are bounded; on expiry the CTA records it in its operands' status words, drains what it issued and
 // returns.
 #include "ozaki7.cuh"
 
@@ -87,9 +87,6 @@ constexpr int ring_depth() {
 }
 constexpr int NTHREADS = 576;                  // 18 warps
 
-__device__ int g_oz7_error;
-__device__ int g_oz7_where[8];  // first expired wait: role, tile, k block, sub-chunk, digit, and the role's counters
-
 // instruction descriptor of tcgen05.mma kind::f16: D FP32, A and B bf16, both K-major, M = 128, N = TN k (k B
 // digits side by side, up to N = 256)
 __host__ __device__ constexpr uint32_t idesc_n(int n) {
@@ -126,17 +123,18 @@ __device__ __forceinline__ bool mbar_wait(uint32_t m, uint32_t parity) {
   }
 }
 
-__device__ __forceinline__ void record_expiry(int role, long long tile, int kb, int s, int i, uint32_t c0, uint32_t c1,
+// the first expired wait of the product's status words (OZ7_ERR_WORDS)
+__device__ __forceinline__ void record_expiry(int* err, int role, long long tile, int kb, int s, int i, uint32_t c0, uint32_t c1,
                                               uint32_t c2) {
-  if (atomicCAS(&g_oz7_error, 0, 1) == 0) {
-    g_oz7_where[0] = role;
-    g_oz7_where[1] = (int)tile;
-    g_oz7_where[2] = kb;
-    g_oz7_where[3] = s;
-    g_oz7_where[4] = i;
-    g_oz7_where[5] = (int)c0;
-    g_oz7_where[6] = (int)c1;
-    g_oz7_where[7] = (int)c2;
+  if (atomicCAS(err, 0, 1) == 0) {
+    err[1] = role;
+    err[2] = (int)tile;
+    err[3] = kb;
+    err[4] = s;
+    err[5] = i;
+    err[6] = (int)c0;
+    err[7] = (int)c1;
+    err[8] = (int)c2;
   }
 }
 
@@ -431,7 +429,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_oz7_gemm(Oz7Args g, long long n
           for (int s = kb * spb; s < s1 && ok; ++s) {
             const int bb = ub & 1;
             if (!mbar_wait(bar(bars.b_empty[bb]), ((ub >> 1) & 1) ^ 1)) {
-              record_expiry(1, ti, kb, s, -1, ua, ub, 0);
+              record_expiry(g.SA.err, 1, ti, kb, s, -1, ua, ub, 0);
               ok = false;
               break;
             }
@@ -446,7 +444,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_oz7_gemm(Oz7Args g, long long n
               const int st = ua % NA;
               const uint32_t us = ua / NA;
               if (!mbar_wait(bar(bars.a_empty[st]), (us & 1) ^ 1)) {
-                record_expiry(2, ti, kb, s, gi, ua, ub, 0);
+                record_expiry(g.SA.err, 2, ti, kb, s, gi, ua, ub, 0);
                 ok = false;
                 break;
               }
@@ -466,7 +464,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_oz7_gemm(Oz7Args g, long long n
         if (last_fill_a[i] >= 0) (void)mbar_wait(bar(bars.a_full[i]), last_fill_a[i] & 1);
       for (int i = 0; i < 2; ++i)
         if (last_fill_b[i] >= 0) (void)mbar_wait(bar(bars.b_full[i]), last_fill_b[i] & 1);
-      if (!ok) atomicExch(&g_oz7_error, 1);
+      if (!ok) atomicExch(g.SA.err, 1);
     }
   } else if (w == 1) {
     // ------------------------------- MMA issue -------------------------------
@@ -482,7 +480,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_oz7_gemm(Oz7Args g, long long n
           const int set = NSET == 2 ? (int)(uacc & 1) : 0;
           const uint32_t use = NSET == 2 ? (uacc >> 1) : uacc;  // uses of this set before this one
           if (!mbar_wait(bar(bars.acc_empty[set]), (use & 1) ^ 1)) {
-            record_expiry(3, ti, kb, -1, -1, ua, ub, uacc);
+            record_expiry(g.SA.err, 3, ti, kb, -1, -1, ua, ub, uacc);
             ok = false;
             break;
           }
@@ -493,7 +491,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_oz7_gemm(Oz7Args g, long long n
             const bool first_sub = (s == kb * spb);
             const int bb = ub & 1;
             if (!mbar_wait(bar(bars.b_full[bb]), (ub >> 1) & 1)) {
-              record_expiry(4, ti, kb, s, -1, ua, ub, uacc);
+              record_expiry(g.SA.err, 4, ti, kb, s, -1, ua, ub, uacc);
               ok = false;
               break;
             }
@@ -504,7 +502,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_oz7_gemm(Oz7Args g, long long n
             for (int gi = 0; gi < NG; ++gi) {
               const int st = ua % NA;
               if (!mbar_wait(bar(bars.a_full[st]), (ua / NA) & 1)) {
-                record_expiry(5, ti, kb, s, gi, ua, ub, uacc);
+                record_expiry(g.SA.err, 5, ti, kb, s, gi, ua, ub, uacc);
                 ok = false;
                 break;
               }
@@ -545,7 +543,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_oz7_gemm(Oz7Args g, long long n
         mma_commit(bar(bars.drain));
         (void)mbar_wait(bar(bars.drain), 0);
       }
-      if (!ok) atomicExch(&g_oz7_error, 1);
+      if (!ok) atomicExch(g.SA.err, 1);
     }
   } else {
     // ------------------------------- epilogue -------------------------------
@@ -591,7 +589,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_oz7_gemm(Oz7Args g, long long n
                                 : ((!first || g.beta == 1.0) ? (g.alpha == -1.0 ? 2 : (g.alpha == 1.0 ? 3 : 4)) : 5);
         const bool got = mbar_wait(bar(bars.acc_full[set]), use & 1);
         if (!__all_sync(0xffffffffu, got)) {
-          if (lane == 0) record_expiry(6 + 16 * w, ti, kb, -1, -1, 0, 0, uacc);
+          if (lane == 0) record_expiry(g.SA.err, 6 + 16 * w, ti, kb, -1, -1, 0, 0, uacc);
           ok = false;
           break;
         }
@@ -647,7 +645,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_oz7_gemm(Oz7Args g, long long n
         ++uacc;
       }
     }
-    if (!ok && lane == 0) atomicExch(&g_oz7_error, 1);
+    if (!ok && lane == 0) atomicExch(g.SA.err, 1);
   }
   asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
   __syncthreads();
@@ -712,8 +710,10 @@ size_t oz7_exp_elems(int rows, int K, int kb) {
   return (size_t)2 * ceil_div(K, kb) * (ceil_div(rows, TM) * TM);
 }
 
-Split7 oz7_buffer(void* planes, int* exps, int S, int rows_cap, int K_cap, int kb, bool wide) {
+Split7 oz7_buffer(void* planes, int* exps, int S, int rows_cap, int K_cap, int kb, int* err, bool wide) {
+  if (!err) throw std::logic_error("oz7_buffer: no status words");
   Split7 s;
+  s.err = err;
   s.planes = static_cast<__nv_bfloat16*>(planes);
   s.exps = exps;
   s.S = S;
@@ -831,24 +831,16 @@ void oz7_set_tile(int tn) {
 
 int oz7_tile() { return g_tile_n; }
 
-int oz7_error_and_reset(int* where) {
-  int e = 0, z = 0;
-  LKG_CUDA(cudaMemcpyFromSymbol(&e, g_oz7_error, sizeof(int)));
-  if (e) {
-    if (where) LKG_CUDA(cudaMemcpyFromSymbol(where, g_oz7_where, 8 * sizeof(int)));
-    LKG_CUDA(cudaMemcpyToSymbol(g_oz7_error, &z, sizeof(int)));
-  }
-  return e;
-}
-
 // Diagnostic entry: one product of each mode on host data (see the declaration in the C ABI header)
 extern "C" int lkg_oz7_mode_check(int mode, int M, int N, int K, const double* A, const double* B, int S, double* C,
                                   int* where_out) {
   double *dA = nullptr, *dB = nullptr, *dC = nullptr;
   void *pa = nullptr, *pb = nullptr;
-  int *ea = nullptr, *eb = nullptr;
+  int *ea = nullptr, *eb = nullptr, *err = nullptr;
   int rc = -1;
   try {
+    LKG_CUDA(cudaMalloc(&err, OZ7_ERR_WORDS * sizeof(int)));
+    LKG_CUDA(cudaMemset(err, 0, OZ7_ERR_WORDS * sizeof(int)));
     if (mode == 1 || mode == 2) N = M;
     const int ka = (mode == 2) ? M : K;  // W^T W: k runs over the rows of the n x n matrix W
     LKG_CUDA(cudaMalloc(&dA, sizeof(double) * (size_t)M * ka));
@@ -861,7 +853,7 @@ extern "C" int lkg_oz7_mode_check(int mode, int M, int N, int K, const double* A
     LKG_CUDA(cudaMemset(dC, 0, sizeof(double) * (size_t)M * N));
     LKG_CUDA(cudaMalloc(&pa, oz7_plane_elems(M, ka, S) * 2));
     LKG_CUDA(cudaMalloc(&ea, oz7_exp_elems(M, ka, OZ7_KB) * sizeof(int)));
-    Split7 sa = oz7_buffer(pa, ea, S, M, ka, OZ7_KB);
+    Split7 sa = oz7_buffer(pa, ea, S, M, ka, OZ7_KB, err);
     if (mode == 2) {
       oz7_split(M, M, dA, M, 1, 0, 1, sa, 0);  // rows of the split = columns of W
       oz7_wtw(M, 0, sa, dC, M, 0, 1, 0);
@@ -871,14 +863,17 @@ extern "C" int lkg_oz7_mode_check(int mode, int M, int N, int K, const double* A
       if (mode == 0) {
         LKG_CUDA(cudaMalloc(&pb, oz7_plane_elems(N, K, S) * 2));
         LKG_CUDA(cudaMalloc(&eb, oz7_exp_elems(N, K, OZ7_KB) * sizeof(int)));
-        sb = oz7_buffer(pb, eb, S, N, K, OZ7_KB);
+        sb = oz7_buffer(pb, eb, S, N, K, OZ7_KB, err);
         oz7_split(N, K, dB, 1, N, 0, 1, sb, 0);
       }
       oz7_gemm(M, N, 0, sa.nblk, 1.0, sa, sb, 0.0, dC, M, 0, 1, mode == 1, 0);
     }
     LKG_CUDA(cudaDeviceSynchronize());
     LKG_CUDA(cudaMemcpy(C, dC, sizeof(double) * (size_t)M * N, cudaMemcpyDeviceToHost));
-    rc = oz7_error_and_reset(where_out) ? -2 : 0;
+    int status[OZ7_ERR_WORDS];
+    LKG_CUDA(cudaMemcpy(status, err, sizeof(status), cudaMemcpyDeviceToHost));
+    rc = status[0] ? -2 : 0;
+    if (rc && where_out) std::copy(status + 1, status + OZ7_ERR_WORDS, where_out);
   } catch (const std::exception& e) {
     set_last_error(e.what());
     rc = -1;
@@ -890,6 +885,7 @@ extern "C" int lkg_oz7_mode_check(int mode, int M, int N, int K, const double* A
   cudaFree(pb);
   cudaFree(ea);
   cudaFree(eb);
+  cudaFree(err);
   return rc;
 }
 

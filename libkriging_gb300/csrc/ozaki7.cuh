@@ -16,6 +16,7 @@ constexpr int OZ7_KB = 256;      // the k block of the trailing updates and of W
 struct Split7 {
   __nv_bfloat16* planes = nullptr;
   int* exps = nullptr;
+  int* err = nullptr;  // OZ7_ERR_WORDS device words for the products that read this operand, see oz7_buffer
   int S = 0, sub_per_blk = 0, nsub = 0, nblk = 0, rows_pad = 0;
   int wide = 0;  // 1: 8-bit leading digits (one bit more per operand, see ozaki7.cu)
   int64_t plane_bstride = 0, exp_bstride = 0;
@@ -35,9 +36,14 @@ struct Oz7Args {
 
 size_t oz7_plane_elems(int rows, int K, int S);     // bf16 elements per batch entry
 size_t oz7_exp_elems(int rows, int K, int kb);      // ints per batch entry (exponents and squares)
-// a split descriptor over caller-owned buffers sized for rows_cap x K_cap, exponent block kb (64 .. 256)
-// (wide: see Split7)
-Split7 oz7_buffer(void* planes, int* exps, int S, int rows_cap, int K_cap, int kb, bool wide = false);
+// Status of the products of one engine or call: word 0 is set when a wait inside a kernel expired, the next 8 say where --
+// role (1, 2 producer B / A; 3, 4, 5 MMA TMEM / B / A; 6 + 16 warp epilogue), tile, k block, sub-chunk, digit group and the
+// role's counters.  The caller zeroes them, copies them down with its results, and discards those when word 0 is set; its
+// own words, so that of two that run at once each learns of its own failure.
+constexpr int OZ7_ERR_WORDS = 9;
+// a split descriptor over caller-owned buffers sized for rows_cap x K_cap, exponent block kb (64 .. 256), status words
+// err (wide: see Split7)
+Split7 oz7_buffer(void* planes, int* exps, int S, int rows_cap, int K_cap, int kb, int* err, bool wide = false);
 
 // rows x K operand, element (r, k) at p[b*bstride + r*s_r + k*s_k], into out.S digit planes
 void oz7_split(int rows, int K, const double* p, int64_t s_r, int64_t s_k, int64_t bstride, int batch, Split7& out,
@@ -62,9 +68,5 @@ void oz7_wtw(int n, int c0, const Split7& SW, double* C, int64_t ldc, int64_t cs
 // output tile width of the digit products: 32 (two TMEM accumulator sets, the default) or 64 (one set)
 void oz7_set_tile(int tn);
 int oz7_tile();
-// 1 if a CTA gave up waiting since the last call (then reset); synchronous.  where (8 ints, optional): the first
-// expired wait -- role (1, 2 producer B / A; 3, 4, 5 MMA TMEM / B / A; 6 + 16 warp epilogue), tile, k block,
-// sub-chunk, digit group and the role's counters
-int oz7_error_and_reset(int* where = nullptr);
 
 }  // namespace lkg

@@ -72,7 +72,9 @@ PredictOut predict_gpu(Engine& model, const double* Xn, int q, const double* the
   const bool whole = need_cov || need_deriv;
   const int qc = whole ? q : (int)std::max<int64_t>(1, std::min<int64_t>(q, ((int64_t)1 << 25) / n));
   DevBuf dXn((size_t)q * d, st), dth(d, st), dz(n, st), dRs((size_t)n * qc, st), drz(q, st), drr(q, st),
-      drm((size_t)q * std::max(p, 1), st);
+      drm((size_t)q * std::max(p, 1), st), dstat(OZ7_ERR_WORDS, st);
+  int* err = reinterpret_cast<int*>(dstat.p);  // status words of this call's digit products
+  LKG_CUDA(cudaMemsetAsync(err, 0, sizeof(int) * OZ7_ERR_WORDS, st));
   LKG_CUDA(cudaMemcpyAsync(dXn.p, Xn, sizeof(double) * q * d, cudaMemcpyHostToDevice, st));
   LKG_CUDA(cudaMemcpyAsync(dth.p, theta, sizeof(double) * d, cudaMemcpyHostToDevice, st));
   LKG_CUDA(cudaMemcpyAsync(dz.p, z, sizeof(double) * n, cudaMemcpyHostToDevice, st));
@@ -80,7 +82,7 @@ PredictOut predict_gpu(Engine& model, const double* Xn, int q, const double* the
     cov_cross(model.kernel(), n, q, d, model.dX(), dXn.p, dth.p, factor, dRs.p, st);
     {
       DevBuf dsc(model.solve_scratch_bytes(q) / sizeof(double) + 1, st);
-      model.solve_lower_inplace(0, dRs.p, n, q, dsc.p);
+      model.solve_lower_inplace(0, dRs.p, n, q, dsc.p, err);
     }
     predict_reduce(n, q, p, dRs.p, dz.p, dRs.p, 1, model.dFY(0), drz.p, drr.p, drm.p, st);
   } else {
@@ -95,8 +97,8 @@ PredictOut predict_gpu(Engine& model, const double* Xn, int q, const double* the
     Split7 SW, SR;
     DevBuf dsc(digits ? 1 : model.solve_scratch_bytes(qc) / sizeof(double) + 1, st);
     if (digits) {
-      SW = oz7_buffer(dWs.p, reinterpret_cast<int*>(dWe.p), S, n, n, OZ7_KB);
-      SR = oz7_buffer(dRsp.p, reinterpret_cast<int*>(dRse.p), S, qc, n, OZ7_KB);
+      SW = oz7_buffer(dWs.p, reinterpret_cast<int*>(dWe.p), S, n, n, OZ7_KB, err);
+      SR = oz7_buffer(dRsp.p, reinterpret_cast<int*>(dRse.p), S, qc, n, OZ7_KB, err);
       oz7_split(n, n, W, 1, model.lda(), 0, 1, SW, st);
     }
     for (int c0 = 0; c0 < q; c0 += qc) {
@@ -109,7 +111,7 @@ PredictOut predict_gpu(Engine& model, const double* Xn, int q, const double* the
         oz7_split(nc, n, dRs.p, n, 1, 0, 1, SR, st);
         oz7_gemm(n, nc, 0, SW.nblk, 1.0, SW, SR, 0.0, dRs.p, n, 0, 1, false, st);
       } else {
-        model.solve_lower_inplace(0, dRs.p, n, nc, dsc.p);
+        model.solve_lower_inplace(0, dRs.p, n, nc, dsc.p, err);
       }
       predict_reduce(n, nc, p, dRs.p, dz.p, dRs.p, 1, model.dFY(0), drz.p + c0, drr.p + c0,
                      drm.p + (size_t)c0 * p, st);
@@ -155,7 +157,7 @@ PredictOut predict_gpu(Engine& model, const double* Xn, int q, const double* the
       DevBuf dxc((size_t)nc * d, st);
       LKG_CUDA(cudaMemcpyAsync(dxc.p, xc.data(), sizeof(double) * nc * d, cudaMemcpyHostToDevice, st));
       dcov_cross(model.kernel(), n, nc, d, model.dX(), dxc.p, dth.p, factor, dW.p, st);
-      model.solve_lower_inplace(0, dW.p, n, ncol, dsc.p);
+      model.solve_lower_inplace(0, dW.p, n, ncol, dsc.p, err);
       predict_reduce(n, ncol, p, dW.p, dz.p, dRs.p + (size_t)c0 * n, d, model.dFY(0), dwz.p, dwr.p, dwm.p, st);
       LKG_CUDA(cudaMemcpyAsync(o.wz.data() + (size_t)c0 * d, dwz.p, sizeof(double) * ncol, cudaMemcpyDeviceToHost,
                                st));
@@ -167,8 +169,10 @@ PredictOut predict_gpu(Engine& model, const double* Xn, int q, const double* the
       LKG_CUDA(cudaStreamSynchronize(st));  // xc and dxc are released at the end of the iteration
     }
   }
+  int expired = 0;
+  LKG_CUDA(cudaMemcpyAsync(&expired, err, sizeof(int), cudaMemcpyDeviceToHost, st));
   LKG_CUDA(cudaStreamSynchronize(st));
-  if ((digits || digits_pay(n)) && oz7_error_and_reset())
+  if (expired)
     throw std::runtime_error("predict: a tensor-core digit product did not complete (timed out)");
   return o;
 }
