@@ -55,12 +55,13 @@ struct MixedWorkspace {
   int digits_inv = FP64_DIGITS;  // digits of the triangular inverse and W^T W, which feed only the gradient (5 .. 8)
   bool wide = true;              // 8-bit leading digits (ozaki7.cu)
   int* err = nullptr;            // status words of the products (OZ7_ERR_WORDS)
-  void* panel = nullptr;  // bf16 planes, oz7_plane_elems(n, 256, 8) per batch entry
+  void* panel = nullptr;  // bf16 planes, oz7_plane_elems(n, 256, 8) for each of panel_group entries
   int* panel_exp = nullptr;
   void* rowblk = nullptr;  // bf16 planes, same size
   int* rowblk_exp = nullptr;
-  void* wchunk = nullptr;  // bf16 planes, oz7_plane_elems(n, wk, 8) per batch entry
+  void* wchunk = nullptr;  // bf16 planes, oz7_plane_elems(n, wk, 8) for each of chunk_group entries
   int* wchunk_exp = nullptr;
+  int panel_group = 1, chunk_group = 1;  // a batch's entries share the buffers, this many at a time
   int wk = 0;  // columns of a chunk of the long products (W^T W, square products): a multiple of 256, at least 512
   int n = 0;
   // look-ahead of the blocked Cholesky (single matrix): the next panel is factored on side_stream, on side_ctas SMs

@@ -160,17 +160,25 @@ void wtw_lower_mixed7(const double* W, int64_t ldw, int64_t wstride, int n, doub
 
 void potrf_blocked_mixed(double* A, int64_t lda, int64_t mstride, int n, double* Dinv, int* info, int batch,
                          const MixedWorkspace& ws, cudaStream_t st) {
-  potrf_blocked_mixed7(A, lda, mstride, n, Dinv, info, batch, ws, st);
+  const int64_t dstride = (int64_t)ceil_div(n, NB) * NB * NB;
+  for (int b = 0; b < batch; b += ws.panel_group)
+    potrf_blocked_mixed7(A + b * mstride, lda, mstride, n, Dinv + b * dstride, info + b, std::min(ws.panel_group, batch - b),
+                         ws, st);
 }
 
 void trtri_blocked_mixed(const double* L, int64_t lda, int64_t mstride, int n, const double* Dinv, double* W,
                          int64_t ldw, int64_t wstride, int batch, const MixedWorkspace& ws, cudaStream_t st) {
-  trtri_blocked_mixed7(L, lda, mstride, n, Dinv, W, ldw, wstride, batch, ws, st);
+  const int64_t dstride = (int64_t)ceil_div(n, NB) * NB * NB;
+  for (int b = 0; b < batch; b += ws.panel_group)
+    trtri_blocked_mixed7(L + b * mstride, lda, mstride, n, Dinv + b * dstride, W + b * wstride, ldw, wstride,
+                         std::min(ws.panel_group, batch - b), ws, st);
 }
 
 void wtw_lower_mixed(const double* W, int64_t ldw, int64_t wstride, int n, double* C, int64_t ldc, int64_t cstride,
                      int batch, const MixedWorkspace& ws, cudaStream_t st) {
-  wtw_lower_mixed7(W, ldw, wstride, n, C, ldc, cstride, batch, ws, st);
+  for (int b = 0; b < batch; b += ws.chunk_group)
+    wtw_lower_mixed7(W + b * wstride, ldw, wstride, n, C + b * cstride, ldc, cstride, std::min(ws.chunk_group, batch - b),
+                     ws, st);
 }
 
 void gemm_square_digits(int n, const double* A, int64_t lda, const double* B, int64_t ldb, double* C, int64_t ldc,

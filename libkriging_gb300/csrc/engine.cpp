@@ -15,6 +15,7 @@
 #include <atomic>
 #include <cstdlib>
 #include <cstring>
+#include <initializer_list>
 #include <string>
 
 #include "common.cuh"
@@ -291,37 +292,89 @@ int Engine::lookahead_ctas() const { return lookahead_ctas_for(n_); }
 
 bool Engine::digit_path() const { return slices_ > 0 || digits_pay(n_); }
 
+// Digit scratch is shared by the entries of a batch in groups: a group's images fill a buffer of at most kDigitScratch (or
+// one entry's), and the groups go one after another.  An entry of 200 rows has 0.96 MB of matrices and would have 4.2 MB
+// of images of its own.  Where memory is short the groups are halved until they fit.
+namespace {
+constexpr size_t kDigitScratch = (size_t)512 << 20;  // bytes of each of the two panels and of the long products' chunk
+
+int entries_within(size_t bytes, int cap) { return (int)std::max<size_t>(1, std::min<size_t>(cap, kDigitScratch / bytes)); }
+
+// false when there is no memory
+bool fits(void** p, size_t bytes) {
+  const cudaError_t e = cudaMalloc(p, std::max<size_t>(bytes, 1));
+  if (e == cudaErrorMemoryAllocation) {
+    (void)cudaGetLastError();
+    *p = nullptr;
+    return false;
+  }
+  LKG_CUDA(e);
+  return true;
+}
+
+void release(std::initializer_list<void**> ps) {
+  for (void** p : ps)
+    if (*p) {
+      cudaFree(*p);
+      *p = nullptr;
+    }
+}
+}  // namespace
+
+void Engine::release_digit_scratch() {
+  buffers_changed();
+  release({&dpanel_, &drowblk_, &dwchunk_, (void**)&dpanel_exp_, (void**)&drowblk_exp_, (void**)&dwchunk_exp_});
+}
+
+size_t Engine::digit_scratch_bytes(int n, int entries) {
+  const size_t panel = oz7_plane_elems(n, OZ7_KB, FP64_DIGITS) * 2, chunk = 2 * panel;
+  const size_t g = entries_within(chunk, entries), whole = oz7_plane_elems(n, n, FP64_DIGITS) * 2;
+  return 2 * panel * entries_within(panel, entries) + std::max(chunk * g, std::min(whole * g, kDigitScratch));
+}
+
 MixedWorkspace Engine::digit_workspace(int batch, bool long_products) {
-  // up to 8 7-bit digits of a 256-wide panel per batch entry (ozaki7.cuh)
-  const size_t pe = oz7_plane_elems(n_, OZ7_KB, FP64_DIGITS) * cap_;
-  const size_t ee = oz7_exp_elems(n_, OZ7_KB, NB) * cap_;
+  // up to 8 7-bit digits of a 256-wide panel per entry (ozaki7.cuh)
+  const size_t pe = oz7_plane_elems(n_, OZ7_KB, FP64_DIGITS) * 2, ee = oz7_exp_elems(n_, OZ7_KB, NB) * sizeof(int);
   if (!dpanel_) {
     buffers_changed();
-    LKG_CUDA(cudaMalloc(&dpanel_, pe * 2));
-    LKG_CUDA(cudaMalloc(&drowblk_, pe * 2));
-    dalloc(&dpanel_exp_, ee);
-    dalloc(&drowblk_exp_, ee);
+    for (panel_group_ = entries_within(pe, cap_);; panel_group_ = (panel_group_ + 1) / 2) {
+      if (fits(&dpanel_, pe * panel_group_) && fits(&drowblk_, pe * panel_group_) &&
+          fits((void**)&dpanel_exp_, ee * panel_group_) && fits((void**)&drowblk_exp_, ee * panel_group_))
+        break;
+      release({&dpanel_, &drowblk_, (void**)&dpanel_exp_, (void**)&drowblk_exp_});
+      if (panel_group_ == 1) LKG_CUDA(cudaErrorMemoryAllocation);
+    }
   }
   // the look-ahead's own panel splits (single-matrix evaluations of a size where it pays)
   if (lookahead_enabled() && !dside_) {
     buffers_changed();
-    const size_t pe1 = oz7_plane_elems(n_, OZ7_KB, FP64_DIGITS), ee1 = oz7_exp_elems(n_, OZ7_KB, NB);
-    LKG_CUDA(cudaMalloc(&dside_, pe1 * 2));
-    dalloc(&dside_exp_, ee1);
     if (!side_st_) {
       LKG_CUDA(cudaStreamCreateWithFlags(&side_st_, cudaStreamNonBlocking));
       LKG_CUDA(cudaEventCreateWithFlags(&ev_strip_, cudaEventDisableTiming));
       LKG_CUDA(cudaEventCreateWithFlags(&ev_panel_, cudaEventDisableTiming));
     }
+    if (!fits(&dside_, pe) || !fits((void**)&dside_exp_, ee)) {
+      release({&dside_, (void**)&dside_exp_});
+      LKG_CUDA(cudaErrorMemoryAllocation);
+    }
   }
-  // the long products' operand in chunks of at most 512 MiB (a whole n x n split would take twice the matrix)
+  // the long products' operand in chunks of columns (a whole n x n split would take twice the matrix), two 256-wide blocks at
+  // least
   if (long_products && !dwchunk_) {
     buffers_changed();
-    const size_t per_k = oz7_plane_elems(n_, OZ7_KB, FP64_DIGITS) / OZ7_KB * 2 * cap_;  // bytes per column
-    const int64_t fit = (int64_t)(((size_t)512 << 20) / per_k) / OZ7_KB * OZ7_KB;
-    wchunk_k_ = (int)std::max<int64_t>(2 * OZ7_KB, std::min<int64_t>(fit, ceil_div(n_, OZ7_KB) * (int64_t)OZ7_KB));
-    LKG_CUDA(cudaMalloc(&dwchunk_, oz7_plane_elems(n_, wchunk_k_, FP64_DIGITS) * cap_ * 2));
-    dalloc(&dwchunk_exp_, oz7_exp_elems(n_, wchunk_k_, OZ7_KB) * cap_);
+    const size_t per_k = oz7_plane_elems(n_, OZ7_KB, FP64_DIGITS) / OZ7_KB * 2;  // bytes per column and entry
+    for (chunk_group_ = entries_within(per_k * 2 * OZ7_KB, cap_);; chunk_group_ = (chunk_group_ + 1) / 2) {
+      const int64_t fit = (int64_t)(kDigitScratch / (per_k * chunk_group_)) / OZ7_KB * OZ7_KB;
+      wchunk_k_ = (int)std::max<int64_t>(2 * OZ7_KB, std::min<int64_t>(fit, ceil_div(n_, OZ7_KB) * (int64_t)OZ7_KB));
+      for (; wchunk_k_ >= 2 * OZ7_KB; wchunk_k_ -= OZ7_KB) {
+        if (fits(&dwchunk_, per_k * wchunk_k_ * chunk_group_) &&
+            fits((void**)&dwchunk_exp_, oz7_exp_elems(n_, wchunk_k_, OZ7_KB) * sizeof(int) * chunk_group_))
+          break;
+        release({&dwchunk_, (void**)&dwchunk_exp_});
+      }
+      if (dwchunk_) break;
+      if (chunk_group_ == 1) LKG_CUDA(cudaErrorMemoryAllocation);
+    }
   }
   MixedWorkspace mw;
   if (slices_ > 0) {
@@ -340,6 +393,8 @@ MixedWorkspace Engine::digit_workspace(int batch, bool long_products) {
   mw.wchunk = dwchunk_;
   mw.wchunk_exp = dwchunk_exp_;
   mw.wk = wchunk_k_;
+  mw.panel_group = panel_group_;
+  mw.chunk_group = chunk_group_;
   if (batch == 1 && dside_ && lookahead_enabled()) {
     mw.side_stream = side_st_;
     mw.ev_strip = ev_strip_;
@@ -364,8 +419,9 @@ void Engine::mark_digits_expired() {
   LKG_CUDA(cudaStreamSynchronize(st_));
 }
 
-void Engine::ensure_grad_buffers() {
-  if (dW_) return;
+bool Engine::ensure_grad_buffers() {
+  if (dpart_) return false;
+  bool released = false;
   buffers_changed();
   if (!solve_st_) {
     int least = 0, greatest = 0;
@@ -374,10 +430,15 @@ void Engine::ensure_grad_buffers() {
     LKG_CUDA(cudaEventCreateWithFlags(&ev_fork_, cudaEventDisableTiming));
     LKG_CUDA(cudaEventCreateWithFlags(&ev_join_, cudaEventDisableTiming));
   }
-  dalloc(&dW_, (size_t)mstride_ * cap_);
-  dalloc(&dRinv_, (size_t)mstride_ * cap_);
+  for (double** m : {&dW_, &dRinv_})
+    if (!*m && !fits((void**)m, sizeof(double) * mstride_ * cap_)) {
+      release_digit_scratch();  // it takes what the matrices leave
+      released = true;
+      dalloc(m, (size_t)mstride_ * cap_);
+    }
   part_size_ = adjoint_partials_size(n_, d_, cap_);
   dalloc(&dpart_, part_size_);
+  return released;
 }
 
 void Engine::solve_phase(int batch, cudaStream_t st) {
@@ -588,6 +649,15 @@ void Engine::evaluate(int batch, const double* thetas, const double* factors, bo
   bool digit = digit_path();  // digit products, else DFMA tiles
   MixedWorkspace mw;
   if (digit) mw = digit_workspace(batch, with_grad);
+  // (while the factorisation runs: allocating them takes the host as long as that)
+  auto grad_buffers = [&] {
+    if (!ensure_grad_buffers() || !digit) return;
+    const MixedWorkspace was = mw;
+    mw = digit_workspace(batch, with_grad);
+    mw.digits = was.digits;
+    mw.digits_inv = was.digits_inv;
+    mw.wide = was.wide;
+  };
   bool retreated = false;
   bool w_valid = false;  // W = L^-1 of the accepted factor is already in dW_
   // the covariance build and the factorisation as one launch sequence (a CUDA graph after its first run): its
@@ -624,7 +694,7 @@ void Engine::evaluate(int batch, const double* thetas, const double* factors, bo
   const bool beside = early_inverse && bench == nullptr && alone_;
   bool solved = false;
   auto inverse_phase = [&] {
-    ensure_grad_buffers();
+    grad_buffers();
     const std::string key = "inverse:b=" + std::to_string(batch) + ":m=" +
                             std::to_string(digit ? mw.digits_inv + 100 * mw.wide : 0) + ":t=" +
                             std::to_string(oz7_tile()) + ":g=" + std::to_string(buf_gen_);
@@ -741,7 +811,7 @@ void Engine::evaluate(int batch, const double* thetas, const double* factors, bo
 
   // ---- [F* y*] = L \ [F y], GLS, E*, SSE, and the gradient's R^-1 and adjoint sums: one launch sequence (a CUDA
   // graph after its first run) ----
-  if (with_grad) ensure_grad_buffers();
+  if (with_grad) grad_buffers();
   const std::string post_key = "post:b=" + std::to_string(batch) + ":m=" + std::to_string(digit ? mw.digits_inv + 100 * mw.wide : 0) +
                                ":gr=" + std::to_string(with_grad) + ":w=" + std::to_string(w_valid) +
                                std::to_string(solved) + ":sa=" +

@@ -124,6 +124,8 @@ class Engine {
   // stream and chains no kernels (24 experts of 100 to 2500 rows: 19.5 ms, 21.4 chained)
   // leaves the status words as a digit product does whose wait expired: the next evaluation reports it
   void mark_digits_expired();
+  // bytes of digit scratch of an engine of this many entries, with gradients
+  static size_t digit_scratch_bytes(int n, int entries);
   void set_alone(bool alone) { alone_ = alone; }
   bool lookahead_enabled() const;
   int lookahead_ctas() const;
@@ -148,7 +150,8 @@ class Engine {
   const double* factor_inverse();
 
  private:
-  void ensure_grad_buffers();
+  // true when the digit scratch had to make room and is gone: digit_workspace again
+  bool ensure_grad_buffers();
   // [F* y*] = L \ [F y], the GLS solve, E* and SSE of all entries, on st
   void solve_phase(int batch, cudaStream_t st);
   void ensure_loo_buffers(bool with_product);
@@ -159,6 +162,7 @@ class Engine {
   // (re)allocates the digit buffers and describes them; long_products: also those of the inverse's W^T W and of
   // leave-one-out's square products
   MixedWorkspace digit_workspace(int batch, bool long_products);
+  void release_digit_scratch();
   // throws when a digit product of this engine expired (word 0 of its status words, on the host), and clears the words
   void check_digits(int expired);
   // rcond(L)^2 per entry, dtrcon('1') style estimate on each entry's first nvb[b] rows / columns
@@ -196,7 +200,8 @@ class Engine {
   int slices_ = 0;
   void *dpanel_ = nullptr, *drowblk_ = nullptr, *dwchunk_ = nullptr, *dside_ = nullptr;
   int *dpanel_exp_ = nullptr, *drowblk_exp_ = nullptr, *dwchunk_exp_ = nullptr, *dside_exp_ = nullptr;
-  int wchunk_k_ = 0;  // columns that dwchunk_ holds
+  int wchunk_k_ = 0;                        // columns that dwchunk_ holds
+  int panel_group_ = 0, chunk_group_ = 0;  // entries that the panels and dwchunk_ hold
   cudaStream_t side_st_ = nullptr;  // look-ahead stream of the mixed Cholesky (single-matrix evaluations)
   cudaEvent_t ev_strip_ = nullptr, ev_panel_ = nullptr;
   cudaStream_t solve_st_ = nullptr;  // the solves of an evaluation with gradient, beside the inverse

@@ -121,11 +121,13 @@ class NestedService : public DenseService {
     // batch capacity per class: every design x starts entries, scaled down to ~70% of the free device memory
     size_t free_b = 0, total_b = 0;
     LKG_CUDA(cudaMemGetInfo(&free_b, &total_b));
-    // bytes per entry: A, W, R^-1, and the digit images of two 256-column panels and a 512-column chunk
+    // A, W and R^-1 of every entry, and each engine's digit scratch
     double need = 0.0;
     for (auto& c : classes_) {
-      const double n = c.n_pad, digits = slices > 0 || digits_pay(c.n_pad) ? 16384.0 * ceil_div(c.n_pad, 128) * 128 : 0.0;
-      need += (25.0 * n * n + digits) * c.designs.size() * starts;
+      const double n = c.n_pad;
+      const int entries = (int)c.designs.size() * starts;
+      need += 25.0 * n * n * entries;
+      if (slices > 0 || digits_pay(c.n_pad)) need += (double)Engine::digit_scratch_bytes(c.n_pad, entries);
     }
     const double scale = std::min(1.0, 0.7 * (double)free_b / std::max(need, 1.0));
     for (auto& c : classes_) {
