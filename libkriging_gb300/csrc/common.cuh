@@ -106,11 +106,15 @@ __device__ __forceinline__ double rsqrt_seed(double x) {
 //   exp       exp(-sum t_k)
 //   matern3_2 prod (1 + t_k) exp(-sum t_k)              = exp(-sum (t_k - log1p t_k))
 //   matern5_2 prod (1 + t_k + t_k^2 / 3) exp(-sum t_k)  = exp(-sum (t_k - log1p(t_k + t_k^2 / 3)))
-// Every covariance build uses them: within a few ulps of the true value, as the log1p form is (whose exponent carries
-// one rounding of each t_k), and an eighth of its FP64 instructions, which bound these kernels (GB300 issues one
-// FP64 warp instruction per 19 clocks and SM).  Measured, n = 4096, d = 8, matern5_2: the build of R takes 1.29 ms
-// against 9.81 ms with the division and log1p per dimension; R_on of 5003 points against 4001, d = 6: 2.52 against
-// 17.7 ms.
+// They take an eighth of the FP64 instructions of the log1p form, and these bound the covariance kernels (GB300 issues one
+// FP64 warp instruction per 19 clocks and SM).
+//
+// In plain FP64 (cov_fast_*: gradient sums, Vecchia blocks, pairs of submodels) the value carries the rounding of sum t_k,
+// which is several times the exponent that it nearly cancels with the product, and one rounding per factor: 2.5 units of
+// 2^-53 (rms) at d = 8 and theta of three times the distances, where the log1p form has 0.6.  The matrices and
+// cross-covariances that go into factors and solves take CovSum instead, whose values are as accurate as the log1p
+// form's: log-likelihoods of 24 designs of n = 4096, d = 8 were 2.5 times further from extended precision with the plain
+// form.
 template <int K>
 __device__ __forceinline__ double cov_scale() {
   if constexpr (K == KMATERN32) return sqrt(3.0);
@@ -150,6 +154,113 @@ __device__ __forceinline__ double cov_fast_finish(double sum_state, double prod_
     return prod_state * exp(-sum_state);
   }
 }
+
+// The scale of one dimension for CovSum: c = cov_scale / |theta| in FP64 and what c lacks of it, relative to c, with the
+// rounding of the square root: true scale = c (1 + rest)
+struct CovScale {
+  double c;
+  float rest;
+};
+template <int K>
+__device__ __forceinline__ CovScale cov_scale_of(double theta) {
+  constexpr double kRoot = K == KMATERN32 ? 5.7937e-17 : K == KMATERN52 ? -4.8586e-17 : 0.0;  // of sqrt(3), sqrt(5) in FP64
+  const double s = cov_scale<K>(), th = fabs(theta), c = s / th;
+  const double rest = fma(-c, th, s) / s + kRoot;
+  return {c, fabs(rest) < 1.0 ? (float)rest : 0.0f};
+}
+
+// The same value with sum t_k (sum t_k^2) in fixed point (64 fraction bits, by integer operations, exact but for 2^-64 a term: integer
+// instructions are cheap beside an FP64 one) and, for the Materns, the rounding errors of the product, which fma gives
+// exactly, summed in FP32 relative to it, with the effect of the scale's rounding; all go into the value at the end.  As many
+// FP64 operations per dimension as the plain form: the fused update p + p a replaces 1 + a and the product, and pays for
+// the error; four more per pair.  Measured, n = 4096, d = 8, matern5_2: the build of R 1.27 ms, 1.29 in the plain form, 9.81
+// with the division and log1p per dimension; R_on of 5003 points against 4001, d = 6: 2.67 ms, 2.52, 17.7.
+template <int K>
+struct CovSum {
+  static constexpr unsigned kHuge = 2048u, kInf = 1u << 20, kNan = 1u << 26;  // of 32 terms at most: no overflow
+  double p = 1.0;                  // Materns: the product
+  unsigned long long frac = 0ull;  // sum t, gauss: sum t^2: ip + frac 2^-64
+  unsigned ip = 0u;
+  float r = 0.0f;  // relative correction of the value
+
+  __device__ __forceinline__ void add(double dx, const CovScale& k) {
+    const double t = fabs(dx) * k.c;
+    const float tf = fminf(narrowed(t), 2048.0f);  // the value is zero beyond
+    if constexpr (K == KGAUSS) {
+      add_fixed(t * t);
+      r = fmaf(-k.rest * tf, tf, r);
+    } else {
+      add_fixed(t);
+      if constexpr (K == KEXP) r = fmaf(-k.rest, tf, r);
+      // - t dlnC/dt = t^2 / (1 + t), t^2 (1 + t) / (3 + 3 t + t^2)
+      if constexpr (K == KMATERN32) r = fmaf(-k.rest, __fdividef(tf * tf, 1.0f + tf), r);
+      if constexpr (K == KMATERN52) r = fmaf(-k.rest, __fdividef(tf * tf * (1.0f + tf), fmaf(tf, tf + 3.0f, 3.0f)), r);
+      if constexpr (K != KEXP) {
+        double a = t;  // the factor minus one
+        if constexpr (K == KMATERN52) a = fma(t, t * (1.0 / 3.0), t);
+        const double pn = fma(p, a, p);
+        const double e = fma(p, a, p - pn);
+        // e / pn in FP32: e with pn's exponent taken off, over pn's significand
+        const int he = __double2hiint(e), hp = __double2hiint(pn), fe = ((he >> 20) & 0x7FF) - (hp >> 20) + 127;
+        const int eb = (he & 0x80000000) | (fe << 23) | ((he & 0xFFFFF) << 3) | (int)((unsigned)__double2loint(e) >> 29);
+        r += __fdividef(fe > 0 ? __int_as_float(eb) : 0.0f, __int_as_float(0x3F800000 | ((hp & 0xFFFFF) << 3)));
+        p = pn;
+      }
+    }
+  }
+
+  __device__ __forceinline__ double value() const {
+    if (ip >= kNan) return __longlong_as_double(0x7FF8000000000000ll);
+    const double hi = __longlong_as_double((long long)(0x40B0000000000000ull | ((unsigned long long)(ip & 4095u) << 40) |
+                                                       (frac >> 24))) -
+                      4096.0;  // ip and the 40 leading fraction bits: exact
+    const float lo = (float)(unsigned)(frac & 0xFFFFFFull) * 0x1p-64f;
+    if constexpr (K == KGAUSS || K == KEXP) {
+      constexpr float h = K == KGAUSS ? 0.5f : 1.0f;
+      if (ip >= kHuge) return 0.0;
+      const double e = exp(-(double)h * hi);
+      return fma(widened(r - h * lo), e, e);
+    } else {
+      if (ip >= 700u) {  // the exponential alone leaves the FP64 range
+        if (ip >= kInf) return __longlong_as_double(0x7FF8000000000000ll);  // infinity times 0, as in the log1p form
+        // past 1500 the value is below the smallest double for any d <= 32 (p <= (1 + 1500 / 32 + (1500 / 32)^2 / 3)^32 <
+        // e^214)
+        if (ip >= 1500u) return 0.0;
+        const double h = exp(-0.5 * hi);
+        return fma(p * h, widened(r - lo), p * h) * h;
+      }
+      const double e = exp(-hi), y = p * e;
+      return y + fma(y, widened(r - lo), fma(p, e, -y));
+    }
+  }
+
+ private:
+  __device__ __forceinline__ void add_fixed(double t) {
+    const int hi = __double2hiint(t), e = hi >> 20, q = e - 1022;  // t = m 2^(q - 64) with m's leading bit 63
+    const unsigned long long m = ((unsigned long long)__double_as_longlong(t) << 11) | 0x8000000000000000ull;
+    unsigned long long f, up, i;  // the shifts give zero past 63
+    asm("shr.u64 %0, %1, %2;" : "=l"(f) : "l"(m), "r"(-q));
+    asm("shl.b64 %0, %1, %2;" : "=l"(up) : "l"(m), "r"(q));
+    asm("shr.u64 %0, %1, %2;" : "=l"(i) : "l"(m), "r"(64 - q));
+    if (q > 0) f = up;
+    unsigned w = (unsigned)i;
+    if (q > 11) w = e < 2047 ? kHuge : (hi & 0xFFFFF) | __double2loint(t) ? kNan : kInf;
+    frac += f;
+    ip += w + (frac < f ? 1u : 0u);
+  }
+  // t >= 0 cut to FP32 by integer operations
+  static __device__ __forceinline__ float narrowed(double t) {
+    const int hi = __double2hiint(t), e = hi >> 20;
+    if (e <= 896) return 0.0f;
+    if (e >= 1151) return 2048.0f;
+    return __int_as_float(((e - 896) << 23) | ((hi & 0xFFFFF) << 3) | (int)((unsigned)__double2loint(t) >> 29));
+  }
+  // an FP32 number below 1 as FP64 by integer operations (zero becomes 2^-127)
+  static __device__ __forceinline__ double widened(float x) {
+    const unsigned b = __float_as_uint(x);
+    return __hiloint2double((int)((b & 0x80000000u) | (((b & 0x7FFFFFFFu) >> 3) + (896u << 20))), (int)(b << 29));
+  }
+};
 
 // dlnC/dtheta_k with inv = 1 / theta_k and ck = s / theta_k
 template <int K>

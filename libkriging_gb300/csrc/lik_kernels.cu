@@ -60,7 +60,8 @@ __global__ void __launch_bounds__(256) k_cov_lower(int n, int d, const double* _
   int I, J;
   lower_tile_of(blockIdx.x, I, J);
   const int64_t b = blockIdx.z;
-  __shared__ double xi[DM][T], xj[DM][T], th[DM];
+  __shared__ double xi[DM][T], xj[DM][T];
+  __shared__ CovScale cks[DM];
   const int r0 = I * T, c0 = J * T, t = threadIdx.x;
   const double* Xb = X + b * xb;
   for (int idx = t; idx < DM * T; idx += 256) {
@@ -68,18 +69,19 @@ __global__ void __launch_bounds__(256) k_cov_lower(int n, int d, const double* _
     xi[k][q] = (k < d && r0 + q < n) ? Xb[(r0 + q) + (int64_t)k * n] : 0.0;
     xj[k][q] = (k < d && c0 + q < n) ? Xb[(c0 + q) + (int64_t)k * n] : 0.0;
   }
-  if (t < DM) th[t] = (t < d) ? theta[b * d + t] : 1.0;
+  if (t < DM) cks[t] = cov_scale_of<K>((t < d) ? theta[b * d + t] : 1.0);
   __syncthreads();
   const double f = factor[b], dv = diag[b];
   const int nv = nvalid ? nvalid[b] : n;  // rows/columns >= nv are padding: identity
   const int ri = t & 63, i = r0 + ri;
   if (i >= n) return;
   double* Ab = A + b * mstride;
-  double xr[DM], ck[DM];
+  double xr[DM];
+  CovScale ck[DM];
 #pragma unroll
   for (int k = 0; k < DM; ++k) {
     xr[k] = xi[k][ri];
-    ck[k] = cov_scale<K>() / fabs(th[k]);
+    ck[k] = cks[k];
   }
   for (int s = blockIdx.y; s < 16; s += gridDim.y) {
     const int cj = (t >> 6) + 4 * s, j = c0 + cj;
@@ -90,11 +92,11 @@ __global__ void __launch_bounds__(256) k_cov_lower(int n, int d, const double* _
     } else if (j == i) {
       v = dv;
     } else {
-      double sum = 0.0, prod = 1.0;
+      CovSum<K> c;
 #pragma unroll
       for (int k = 0; k < DM; ++k)
-        if (k < d) cov_fast_term<K>(xj[k][cj] - xr[k], ck[k], sum, prod);
-      v = cov_fast_finish<K>(sum, prod) * f;
+        if (k < d) c.add(xj[k][cj] - xr[k], ck[k]);
+      v = c.value() * f;
     }
     Ab[i + (int64_t)j * lda] = v;
   }
@@ -104,31 +106,32 @@ template <int K, int DM>
 __global__ void __launch_bounds__(256) k_cov_cross(int n_o, int q, int d, const double* __restrict__ Xo,
                                                    const double* __restrict__ Xn, const double* __restrict__ theta,
                                                    double factor, double* __restrict__ R, bool snap) {
-  __shared__ double xo[DM][T], xn[DM][T], cks[DM];
+  __shared__ double xo[DM][T], xn[DM][T];
+  __shared__ CovScale cks[DM];
   const int r0 = blockIdx.x * T, c0 = blockIdx.y * T, t = threadIdx.x;
   for (int idx = t; idx < DM * T; idx += 256) {
     const int k = idx / T, qq = idx % T;
     xo[k][qq] = (k < d && r0 + qq < n_o) ? Xo[(r0 + qq) + (int64_t)k * n_o] : 0.0;
     xn[k][qq] = (k < d && c0 + qq < q) ? Xn[(c0 + qq) + (int64_t)k * q] : 0.0;
   }
-  if (t < DM) cks[t] = (t < d) ? cov_scale<K>() / fabs(theta[t]) : 1.0;
+  if (t < DM) cks[t] = cov_scale_of<K>((t < d) ? theta[t] : 1.0);
   __syncthreads();
   const int ri = t & 63, i = r0 + ri;
   if (i >= n_o) return;
   for (int s = blockIdx.z; s < 16; s += gridDim.z) {
     const int cj = (t >> 6) + 4 * s, j = c0 + cj;
     if (j >= q) continue;
-    double sum = 0.0, prod = 1.0;
+    CovSum<K> c;
     bool coincident = true;
 #pragma unroll
     for (int k = 0; k < DM; ++k) {
       if (k < d) {
         const double dx = xo[k][ri] - xn[k][cj];
         coincident = coincident && (fabs(dx) <= 2.220446049250313e-16);
-        cov_fast_term<K>(dx, cks[k], sum, prod);
+        c.add(dx, cks[k]);
       }
     }
-    R[i + (int64_t)j * n_o] = (snap && coincident) ? 1.0 : cov_fast_finish<K>(sum, prod) * factor;
+    R[i + (int64_t)j * n_o] = (snap && coincident) ? 1.0 : c.value() * factor;
   }
 }
 
@@ -158,7 +161,8 @@ template <int K, int DM>
 __global__ void __launch_bounds__(256) k_dcov_cross(int n_o, int q, int d, const double* __restrict__ Xo,
                                                     const double* __restrict__ Xn, const double* __restrict__ theta,
                                                     double factor, double* __restrict__ DR) {
-  __shared__ double xo[DM][T], xn[DM][T], th[DM], cks[DM];
+  __shared__ double xo[DM][T], xn[DM][T], th[DM];
+  __shared__ CovScale cks[DM];
   const int r0 = blockIdx.x * T, c0 = blockIdx.y * T, t = threadIdx.x;
   for (int idx = t; idx < DM * T; idx += 256) {
     const int k = idx / T, qq = idx % T;
@@ -167,7 +171,7 @@ __global__ void __launch_bounds__(256) k_dcov_cross(int n_o, int q, int d, const
   }
   if (t < DM) {
     th[t] = (t < d) ? theta[t] : 1.0;
-    cks[t] = cov_scale<K>() / fabs(th[t]);
+    cks[t] = cov_scale_of<K>(th[t]);
   }
   __syncthreads();
   const int ri = t & 63, i = r0 + ri;
@@ -175,17 +179,17 @@ __global__ void __launch_bounds__(256) k_dcov_cross(int n_o, int q, int d, const
   for (int s = blockIdx.z; s < 16; s += gridDim.z) {
     const int cj = (t >> 6) + 4 * s, j = c0 + cj;
     if (j >= q) continue;
-    double sum = 0.0, prod = 1.0;
+    CovSum<K> c;
     bool coincident = true;
 #pragma unroll
     for (int k = 0; k < DM; ++k) {
       if (k < d) {
         const double dx = xo[k][ri] - xn[k][cj];
         coincident = coincident && (fabs(dx) <= 2.220446049250313e-16);
-        cov_fast_term<K>(dx, cks[k], sum, prod);
+        c.add(dx, cks[k]);
       }
     }
-    const double r = coincident ? 1.0 : cov_fast_finish<K>(sum, prod) * factor;
+    const double r = coincident ? 1.0 : c.value() * factor;
     double* out = DR + i + (int64_t)j * d * n_o;
 #pragma unroll
     for (int k = 0; k < DM; ++k)
@@ -481,14 +485,15 @@ template <int K, int DM>
 __global__ void __launch_bounds__(256) k_loo_gradR(int n, int d, const double* __restrict__ X,
                                                    const double* __restrict__ theta, double factor, int kdim,
                                                    double* __restrict__ G, int64_t ldg) {
-  __shared__ double xi[DM][T], xj[DM][T], cks[DM];
+  __shared__ double xi[DM][T], xj[DM][T];
+  __shared__ CovScale cks[DM];
   const int r0 = blockIdx.x * T, c0 = blockIdx.y * T, t = threadIdx.x;
   for (int idx = t; idx < DM * T; idx += 256) {
     const int k = idx / T, q = idx % T;
     xi[k][q] = (k < d && r0 + q < n) ? X[(r0 + q) + (int64_t)k * n] : 0.0;
     xj[k][q] = (k < d && c0 + q < n) ? X[(c0 + q) + (int64_t)k * n] : 0.0;
   }
-  if (t < DM) cks[t] = (t < d) ? cov_scale<K>() / fabs(theta[t]) : 1.0;
+  if (t < DM) cks[t] = cov_scale_of<K>((t < d) ? theta[t] : 1.0);
   __syncthreads();
   const int ri = t & 63, i = r0 + ri;
   if (i >= n) return;
@@ -498,16 +503,17 @@ __global__ void __launch_bounds__(256) k_loo_gradR(int n, int d, const double* _
     if (j >= n) continue;
     double v = 0.0;
     if (j != i) {
-      double sum = 0.0, prod = 1.0, dk = 0.0;
+      CovSum<K> c;
+      double dk = 0.0;
 #pragma unroll
       for (int k = 0; k < DM; ++k) {
         if (k < d) {
           const double dx = xj[k][cj] - xi[k][ri];
-          cov_fast_term<K>(dx, cks[k], sum, prod);
-          if (k == kdim) dk = dlncov_fast<K>(dx, inv, cks[k]);
+          c.add(dx, cks[k]);
+          if (k == kdim) dk = dlncov_fast<K>(dx, inv, cks[k].c);
         }
       }
-      v = (cov_fast_finish<K>(sum, prod) * factor) * dk;
+      v = (c.value() * factor) * dk;
     }
     G[i + (int64_t)j * ldg] = v;
   }

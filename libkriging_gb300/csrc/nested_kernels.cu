@@ -52,12 +52,11 @@ __global__ void __launch_bounds__(128) k_nk_corr(int n, int d, const double* __r
   double v = 0.0;
   if (a < nvalid[e]) {
     const double* Xe = X + (int64_t)e * xs;
-    double s = 0.0, pr = 1.0;
+    CovSum<K> c;
 #pragma unroll
     for (int q = 0; q < DM; ++q)
-      if (q < d)
-        cov_fast_term<K>(Xe[a + (int64_t)q * n] - Xc[t + (int64_t)q * qc], cov_scale<K>() / fabs(theta[q]), s, pr);
-    v = cov_fast_finish<K>(s, pr);
+      if (q < d) c.add(Xe[a + (int64_t)q * n] - Xc[t + (int64_t)q * qc], cov_scale_of<K>(theta[q]));
+    v = c.value();
   }
   out[(int64_t)e * os + a + (int64_t)t * n] = v;
 }
