@@ -466,15 +466,24 @@ const double* Engine::factor_inverse() {
   return dWp_;
 }
 
-size_t Engine::solve_scratch_bytes(int r) const { return r > 16 && digits_pay(n_) ? trsm_digits_bytes(n_, r) : 0; }
+// Right-hand sides that one digit solve takes at a time: their images (4 KB a column) stay within 128 MiB beside the factor's.
+// A column's result depends on that column alone, so the split does not show in the results.
+// 150000 points on 200: 9.33 ms against 9.13 at once with 0.6 GB of images; 9.73 at half of it.
+namespace {
+constexpr int kSolveColumns = 32768;
+}
+
+size_t Engine::solve_scratch_bytes(int r) const {
+  return r > 16 && digits_pay(n_) ? trsm_digits_bytes(n_, std::min(r, kSolveColumns)) : 0;
+}
 
 void Engine::solve_lower_inplace(int b, double* dB, int64_t ldb, int r, void* scratch, int* err) const {
+  const double *L = dA_ + (size_t)b * mstride_, *Dinv = dDinv_ + (size_t)b * dstride_;
   if (r > 16 && digits_pay(n_))
-    trsm_lower_left_digits(dA_ + (size_t)b * mstride_, lda_, n_, dDinv_ + (size_t)b * dstride_, dB, ldb, r, scratch, err,
-                           st_);
+    for (int c = 0; c < r; c += kSolveColumns)
+      trsm_lower_left_digits(L, lda_, n_, Dinv, dB + (int64_t)c * ldb, ldb, std::min(kSolveColumns, r - c), scratch, err, st_);
   else
-    trsm_lower_left(dA_ + (size_t)b * mstride_, lda_, mstride_, n_, dDinv_ + (size_t)b * dstride_, dB, ldb, 0, r, 1,
-                    st_);
+    trsm_lower_left(L, lda_, mstride_, n_, Dinv, dB, ldb, 0, r, 1, st_);
 }
 
 // dtrcon('1', 'L', 'N') style estimate (LAPACK dlacn2 iteration of Hager / Higham) of rcond(L)^2 for every entry,

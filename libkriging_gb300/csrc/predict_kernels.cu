@@ -68,7 +68,8 @@ PredictOut predict_gpu(Engine& model, const double* Xn, int q, const double* the
   PredictOut o;
   if (q <= 0) return o;
   // the covariance and the derivatives need Rstar_on for all points at once; otherwise the points go in chunks of
-  // at most 2^25 / n (Rstar_on of a chunk below 256 MB)
+  // at most 2^25 / n (Rstar_on of a chunk below 256 MB; the solves' digit images are another 128 MiB and 4 KB for each row of
+  // the factor, solve_scratch_bytes)
   const bool whole = need_cov || need_deriv;
   const int qc = whole ? q : (int)std::max<int64_t>(1, std::min<int64_t>(q, ((int64_t)1 << 25) / n));
   DevBuf dXn((size_t)q * d, st), dth(d, st), dz(n, st), dRs((size_t)n * qc, st), drz(q, st), drr(q, st),
