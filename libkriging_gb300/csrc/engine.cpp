@@ -914,9 +914,9 @@ void Engine::ensure_loo_buffers(bool with_product) {
     buffers_changed();
     dalloc(&dloo_at_, (size_t)cap_ * n_ * std::max(p_, 1));
   }
-  if (with_product && !dloo_m_) {
+  if (with_product && !dloo_vec_) {  // the last of the two: an allocation that failed is tried again
     buffers_changed();
-    dalloc(&dloo_m_, (size_t)mstride_);
+    if (!dloo_m_) dalloc(&dloo_m_, (size_t)mstride_);
     dalloc(&dloo_vec_, (size_t)n_ * (2 * d_ + 2));
   }
 }
