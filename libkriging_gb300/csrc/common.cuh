@@ -43,8 +43,9 @@ inline void check_cuda(cudaError_t e, const char* what, const char* file, int li
 __device__ __forceinline__ void chain_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
-// No chains in launches of this thread while one lives: for evaluations that run beside others, whose SMs waiting kernels
-// would hold.
+// No chains in launches of this thread while one lives: for batched evaluations that run beside others, whose SMs waiting
+// kernels would hold.  (Predictions of submodels beside one another keep theirs: 200 points on 24 submodels of 150 to 2500
+// rows take 3.5 ms chained, 4.0 unchained, 5000 points 22.0 and 22.2.)
 inline thread_local int t_unchained = 0;
 struct Unchained {
   explicit Unchained(bool on) : on_(on) { t_unchained += on_; }

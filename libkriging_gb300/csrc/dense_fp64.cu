@@ -8,6 +8,7 @@
 
 #include <stdexcept>
 
+#include "ozaki7.cuh"
 #include "stats.hpp"
 
 namespace lkg {
@@ -689,7 +690,7 @@ void zero_upper(double* A, int64_t lda, int64_t mstride, int n, int batch, cudaS
 namespace {
 
 // Up to two waves of large tiles take the small ones: the FP64 pipes need as long for the same terms, but all SMs have some.
-bool few_tiles(int64_t tiles) { return tiles <= 2 * 152; }
+bool few_tiles(int64_t tiles) { return tiles <= 2 * oz7_sm_count(); }
 
 template <int TM, int TN>
 void gemm_small_launch(int M, int N, int K, double alpha, MatView A, MatView B, double beta, double* C, int64_t ldc,
