@@ -113,9 +113,8 @@ __device__ __forceinline__ double rsqrt_seed(double x) {
 // In plain FP64 (cov_fast_*: gradient sums, Vecchia blocks, pairs of submodels) the value carries the rounding of sum t_k,
 // which is several times the exponent that it nearly cancels with the product, and one rounding per factor: 2.5 units of
 // 2^-53 (rms) at d = 8 and theta of three times the distances, where the log1p form has 0.6.  The matrices and
-// cross-covariances that go into factors and solves take CovSum instead, whose values are as accurate as the log1p
-// form's: log-likelihoods of 24 designs of n = 4096, d = 8 were 2.5 times further from extended precision with the plain
-// form.
+// cross-covariances that go into factors and solves take CovValue: from d = 5 on (the kernels' template for eight and more
+// dimensions) CovSum, whose values are as accurate as the log1p form's.
 template <int K>
 __device__ __forceinline__ double cov_scale() {
   if constexpr (K == KMATERN32) return sqrt(3.0);
@@ -262,6 +261,21 @@ struct CovSum {
     return __hiloint2double((int)((b & 0x80000000u) | (((b & 0x7FFFFFFFu) >> 3) + (896u << 20))), (int)(b << 29));
   }
 };
+
+template <int K>
+struct CovPlain {
+  double s = 0.0, p = 1.0;
+  __device__ __forceinline__ void add(double dx, const CovScale& k) { cov_fast_term<K>(dx, k.c, s, p); }
+  __device__ __forceinline__ double value() const { return cov_fast_finish<K>(s, p); }
+};
+
+// The line lies where the plain form's error shows: with it, and the digit products, results are 0.4 (d = 2) to 0.9 (d = 4)
+// times as far from 80-bit arithmetic as with DFMA products on log1p-form matrices, and 1.1 to 1.9 times from d = 6 on; CovSum
+// brings those to 0.3 .. 0.7 (geometric means of LL, gradient, leave-one-out and predictions, 382 outputs of Matern designs).
+// Below it smooth designs without noise are so ill-conditioned that results show every rounding of R (gradients in two
+// dimensions move by 2e-9), so they keep theirs.
+template <int K, int DM>
+using CovValue = std::conditional_t<(DM <= 4), CovPlain<K>, CovSum<K>>;
 
 // dlnC/dtheta_k with inv = 1 / theta_k and ck = s / theta_k
 template <int K>

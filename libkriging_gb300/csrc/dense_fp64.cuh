@@ -47,7 +47,7 @@ void wtw_lower(const double* W, int64_t ldw, int64_t wstride, int n, double* C, 
 void inverse_init(const double* Dinv, int n, double* W, int64_t ldw, int64_t wstride, int batch, cudaStream_t st);
 
 // Digit-product variants: the O(n^3) products on the bf16 tensor cores by error-free splitting into 7-bit digits
-// (ozaki7.cuh); the diagonal blocks stay FP64.  With 8 digits (56-bit operands, one rounding per 256 columns) they
+// (ozaki7.cuh); the diagonal blocks stay FP64.  With 8 digits (57-bit operands with wide leading digits, 56-bit without, one rounding per 256 columns) they
 // serve the FP64 path too: see digits_pay().
 constexpr int FP64_DIGITS = 8;
 struct MixedWorkspace {

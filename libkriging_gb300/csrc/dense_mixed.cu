@@ -243,9 +243,9 @@ void trsm_lower_left_digits(const double* L, int64_t lda, int n, const double* D
 
 // The FP64 path's products as digit products: GB300 issues one FP64 warp instruction per 19 clocks and SM (1.25 TFLOP/s
 // over the chip), so 36 exact bf16 products of 7-bit digits are 10 to 30 times faster than one DFMA.  Their error is no
-// larger: one rounding per 256 columns instead of one per column, on operands of 57 bits (relative errors of LL, gradient
-// and leave-one-out against extended precision, 12 designs x 6 seeds, n = 300 and 520, geometric mean: 2.4e-13 here,
-// 4.5e-13 with DFMA; n = 2048 at cond(R) near 1e10: gradient 2.8e-11 here, 1.2e-10 with DFMA).  Measured, LL + gradient, d =
+// larger: one rounding per 256 columns instead of one per column, on operands of 57 bits.  On the same matrices, 24 designs
+// of n = 4096, d = 8 against 80-bit arithmetic (geometric means): LL 1.2e-11 here, 1.4e-11 with DFMA (absolute), gradient
+// 1.1e-13 here, 1.7e-13 with DFMA (relative).  Measured, LL + gradient, d =
 // 4, matern5_2 (us, DFMA / digits), one matrix: n = 192 434 / 475, 256 550 / 588, 448 906 / 946; 64 at once: n = 192
 // 2756 / 1985, 256 4414 / 2792, 448 12184 / 5222; one matrix of 1024 8313 / 3394 (large DFMA tiles).  The rule looks at n
 // alone, so that a matrix gives the same bits alone and in a batch: from 192 on a batch gains more than one matrix loses.

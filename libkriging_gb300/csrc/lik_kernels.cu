@@ -92,7 +92,7 @@ __global__ void __launch_bounds__(256) k_cov_lower(int n, int d, const double* _
     } else if (j == i) {
       v = dv;
     } else {
-      CovSum<K> c;
+      CovValue<K, DM> c;
 #pragma unroll
       for (int k = 0; k < DM; ++k)
         if (k < d) c.add(xj[k][cj] - xr[k], ck[k]);
@@ -121,7 +121,7 @@ __global__ void __launch_bounds__(256) k_cov_cross(int n_o, int q, int d, const 
   for (int s = blockIdx.z; s < 16; s += gridDim.z) {
     const int cj = (t >> 6) + 4 * s, j = c0 + cj;
     if (j >= q) continue;
-    CovSum<K> c;
+    CovValue<K, DM> c;
     bool coincident = true;
 #pragma unroll
     for (int k = 0; k < DM; ++k) {
@@ -179,7 +179,7 @@ __global__ void __launch_bounds__(256) k_dcov_cross(int n_o, int q, int d, const
   for (int s = blockIdx.z; s < 16; s += gridDim.z) {
     const int cj = (t >> 6) + 4 * s, j = c0 + cj;
     if (j >= q) continue;
-    CovSum<K> c;
+    CovValue<K, DM> c;
     bool coincident = true;
 #pragma unroll
     for (int k = 0; k < DM; ++k) {
@@ -503,7 +503,7 @@ __global__ void __launch_bounds__(256) k_loo_gradR(int n, int d, const double* _
     if (j >= n) continue;
     double v = 0.0;
     if (j != i) {
-      CovSum<K> c;
+      CovValue<K, DM> c;
       double dk = 0.0;
 #pragma unroll
       for (int k = 0; k < DM; ++k) {

@@ -52,7 +52,7 @@ __global__ void __launch_bounds__(128) k_nk_corr(int n, int d, const double* __r
   double v = 0.0;
   if (a < nvalid[e]) {
     const double* Xe = X + (int64_t)e * xs;
-    CovSum<K> c;
+    CovValue<K, DM> c;
 #pragma unroll
     for (int q = 0; q < DM; ++q)
       if (q < d) c.add(Xe[a + (int64_t)q * n] - Xc[t + (int64_t)q * qc], cov_scale_of<K>(theta[q]));

@@ -1,5 +1,5 @@
-"""Rounding of the covariance values: root mean square of the relative errors against extended precision, beside what the
-log1p form has in FP64 arithmetic on the same pairs."""
+"""Rounding of the covariance values from five dimensions on, where the plain product form loses digits: root mean square of
+the relative errors against extended precision, beside what the log1p form has in FP64 arithmetic on the same pairs."""
 import numpy as np
 import pytest
 
@@ -25,7 +25,7 @@ def _forms(kernel, B, theta):
 
 
 @pytest.mark.parametrize("kernel", ["gauss", "exp", "matern3_2", "matern5_2"])
-@pytest.mark.parametrize("d", [1, 2, 3, 5, 8, 16])
+@pytest.mark.parametrize("d", [5, 8, 9, 16])
 @pytest.mark.parametrize("theta", [0.05, 0.3, 1.0, 3.0, 10.0])
 def test_no_larger_than_the_log1p_forms(gpu_lib, kernel, d, theta):
     import libkriging_gb300 as lk
