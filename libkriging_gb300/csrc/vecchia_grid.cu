@@ -193,6 +193,7 @@ struct MaxminArgs {
   int* order;
   int* err;                    // set when a wait gave up; the launches after it do nothing
   unsigned long long wait_ns;  // limit of a wait for a round's next step
+  float eps_length;  // no less than the length of eps, from FP64: in FP32 its squares are zero for sides below 1e-16
   float eps[MAXD];  // bound on the error of a difference of two Xf in dimension k
 };
 
@@ -533,14 +534,10 @@ __global__ void __launch_bounds__(MM_THREADS, 1) k_maxmin_grid(MaxminArgs a) {
         }
       }
       __syncthreads();
-      // FP32 bounds: with E no less than the length of the error bounds of the differences and d2 the FP32 squared distance,
-      // the true one is at least (sqrt(d2) - E)^2 and at most (sqrt(d2) + E)^2, up to 2^-19 for the rounding of at most 8
-      // terms and of the square roots.  E is the sum of the bounds: their squares would underflow to zero where all sides
-      // of the box are below 1e-16, and pairs would pass as clear that are not.
-      float E = 0.0f;
-#pragma unroll
-      for (int k = 0; k < DM; ++k) E += k < d ? a.eps[k] : 0.0f;
-      E *= 1.0f + 0x1p-20f;
+      // FP32 bounds: with E the length of the error bounds of the differences and d2 the FP32 squared distance, the true one
+      // is at least (sqrt(d2) - E)^2 and at most (sqrt(d2) + E)^2, up to 2^-19 for the rounding of at most 8 terms and of the
+      // square roots
+      const float E = a.eps_length;
       if (tid < nc) {
         const int r = rank[tid], s = uslot[tid];
         skey[r] = ukey[tid];
@@ -1101,8 +1098,9 @@ void vecchia_sets_grid(int n, int d, const double* hX, const double* dX, int fir
     }
   DevBuf<double> Xp((size_t)n * d), Xs((size_t)n * d), dist(n);
   DevBuf<float> Xf((size_t)n * d);
-  DevBuf<int> cell(n), perm(n), orig(n), slot_of(n), err(1);
-  LKG_CUDA(cudaMemsetAsync(err.p, 0, sizeof(int), st));
+  DevBuf<int> cell(n), perm(n), orig(n), slot_of((size_t)n + 1);
+  int* const err = slot_of.p + n;  // the error word of the order's kernel
+  LKG_CUDA(cudaMemsetAsync(err, 0, sizeof(int), st));
   k_points_major<<<ceil_div(n, 256), 256, 0, st>>>(n, d, dX, nullptr, Xp.p, nullptr);
   LKG_LAUNCH("k_points_major");
 
@@ -1128,12 +1126,17 @@ void vecchia_sets_grid(int n, int d, const double* hX, const double* dX, int fir
     a.Xs = Xs.p;
     a.Xf = Xf.p;
     // |x - lo| <= ext: two roundings to FP32 and the subtraction's own
-    for (int k = 0; k < d; ++k) a.eps[k] = std::nextafter((float)((hi[k] - lo[k]) * 0x1p-22), INFINITY);
+    double length2 = 0.0;
+    for (int k = 0; k < d; ++k) {
+      a.eps[k] = std::nextafter((float)((hi[k] - lo[k]) * 0x1p-22), INFINITY);
+      length2 += (double)a.eps[k] * a.eps[k];
+    }
+    a.eps_length = (float)(std::sqrt(length2) * (1.0 + 0x1p-20));
     a.orig = orig.p;
     a.slot_of = slot_of.p;
     a.dist = dist.p;
     a.order = dorder;
-    a.err = err.p;
+    a.err = err;
     a.wait_ns = wait_ns;
     // FP32 squares of differences between 1e-18 and 1e18 stay in range; other boxes take every step alone
     a.singles = ROUND_FROM;
@@ -1151,7 +1154,7 @@ void vecchia_sets_grid(int n, int d, const double* hX, const double* dX, int fir
       LKG_LAUNCH("k_maxmin_grid");
     }
     int expired = 0;
-    LKG_CUDA(cudaMemcpyAsync(&expired, err.p, sizeof(int), cudaMemcpyDeviceToHost, st));
+    LKG_CUDA(cudaMemcpyAsync(&expired, err, sizeof(int), cudaMemcpyDeviceToHost, st));
     LKG_CUDA(cudaStreamSynchronize(st));  // cstart / cursor are freed at scope exit
     // the order is incomplete then, and nothing may read it
     if (expired) throw std::runtime_error("Vecchia sets: a round of the maxmin order did not complete (timed out)");
