@@ -182,7 +182,7 @@ void Engine::set_slices(int s) {
 // (LKG_LOOKAHEAD_CTAS, lkg_set_lookahead) applies to every size; otherwise (-1) the autotuner's choice for the matrix
 // size is used ("lookahead:n=<n>", see Kriging::autotune_lookahead), else lookahead_default: the smaller the matrix, the
 // less its trailing updates have to do, and the more SMs the panel's products get.  Measured (ms, LL + gradient at 16 / 24 /
-// 32 / 48 / 64 SMs): n = 2048 5.02 / 4.91 / 4.87 / 4.84 / 4.83, 4096 13.51 / 13.00 / 12.76 / 12.54 / 12.42, 8192 (mixed) 42.1 /
+// 32 / 48 / 64 SMs, one evaluation at a time): n = 2048 5.02 / 4.91 / 4.87 / 4.84 / 4.83, 4096 13.51 / 13.00 / 12.76 / 12.54 / 12.42, 8192 (mixed) 42.1 /
 // 39.8 / 38.8 / 37.7 / 37.6, 12000 88.8 / 83.9 / 82.3 / 82.5 / 84.7, 16384 171.1 / 165.8 / 165.8 / 169.8 / 177.2.
 namespace {
 int lookahead_default(int n) { return std::min(64, std::max(16, 64 * 8192 / n)); }
